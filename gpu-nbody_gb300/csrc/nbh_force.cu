@@ -27,9 +27,9 @@ constexpr size_t force_smem_bytes(int threads, int cap) {
 }
 
 // The list walk (64-wide groups): per group, the records of accepted nodes awaiting
-// evaluation (at most 31 wait after an evaluation and one round adds at most 32) with each
-// record's full cell width^2 (for the error bound; 0 for a body), the undecided cells of a
-// round (at most 32), and a stack of `cap` cells whose children are still to be tested,
+// evaluation (at most 31 wait after an evaluation and one round adds at most 32; separate
+// arrays of x, y, z, m) with each record's full cell width^2 (for the error bound; 0 for a
+// body), the undecided cells of a round (at most 32, likewise as arrays), and a stack of `cap` cells whose children are still to be tested,
 // with their levels (a 64-entry stack also holds the per-level walk's 2 * kMaxDepth ints).
 constexpr int kListCap = 64;
 constexpr size_t list_group_bytes(int cap) {
@@ -79,47 +79,54 @@ __device__ __forceinline__ float dist2(const float dx, const float dy, const flo
         return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, eps2)));
 }
 
-// The first 32 records: unrolled completely for two or more bodies per lane (the 64-wide
-// walk's force 2.6 % faster than unrolled by 8), by 8 for one (the 32-wide walk on a 16K
-// ball measured the same either way).
-template <int BPL, bool FEAT>
-__device__ __forceinline__ void eval_list32(const float4* lst, const float* lw, const float4 (&pb)[BPL],
-                                            const float eps2, float (&ax)[BPL], float (&ay)[BPL], float (&az)[BPL],
-                                            float (&eb)[BPL]) {
-#pragma unroll(BPL >= 2 ? 32 : 8)
-    for (int i = 0; i < 32; ++i) {
-        const float4 q = lst[i];
-        const float s2 = FEAT ? lw[i] : 0.0f;
-#pragma unroll
-        for (int k = 0; k < BPL; ++k) {
-            const float dx = __fsub_rn(q.x, pb[k].x);
-            const float dy = __fsub_rn(q.y, pb[k].y);
-            const float dz = __fsub_rn(q.z, pb[k].z);
-            const float d2 = dist2<false>(dx, dy, dz, eps2);
-            interact<false, FEAT>(q, dx, dy, dz, d2, ax[k], ay[k], az[k], eb[k], s2);
-        }
-    }
+// The list walk's arithmetic is packed: one FP32x2 instruction works on two consecutive records
+// of the list.  FP32x2 has the multiply-add rate of scalar FP32 (measured 2.03-2.1 cycles per
+// warp and scheduler against 2 x 1.11) but takes half the issue slots, and a list kept as
+// separate arrays of x, y, z and m hands its operand pairs over straight from 16-byte shared
+// loads, four records each, without a move.  A body's negated coordinates are held twice
+// over, and its sums as one partial sum over the even and one over the odd records.  A 32-record
+// batch for two bodies per lane, alone on an SM: 30.5 cycles per record and warp, 33.5 with
+// scalar arithmetic and 16-byte records, and 15 issue slots per record instead of 27, which
+// is what the walk's other instructions need.
+struct ListBody {
+    float2 nx, ny, nz;
+};
+struct ListSum {
+    float2 x, y, z, e;
+};
+
+template <bool FEAT>
+__device__ __forceinline__ void interact2(const float2 X, const float2 Y, const float2 Z, const float2 M,
+                                          const float2 S, const ListBody& b, const float2 eps2, ListSum& a) {
+    const float2 dx = __fadd2_rn(X, b.nx), dy = __fadd2_rn(Y, b.ny), dz = __fadd2_rn(Z, b.nz);
+    const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps2)));
+    const float2 rd = make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y));
+    const float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(M, rd), rd), rd);
+    a.x = __ffma2_rn(dx, f, a.x);
+    a.y = __ffma2_rn(dy, f, a.y);
+    a.z = __ffma2_rn(dz, f, a.z);
+    if constexpr (FEAT) a.e = __ffma2_rn(__fmul2_rn(f, rd), S, a.e);
 }
 
-// Evaluate the first cnt records of a group's list for the lane's bodies, in list order
-// (with FEAT also their error bounds, from the widths in lw).
+// Four records of the list (lst: arrays x, y, z, m and, with FEAT, width^2, kListCap apart;
+// `at` a multiple of 4) for the lane's bodies.
 template <int BPL, bool FEAT>
-__device__ __forceinline__ void eval_list(const float4* lst, const float* lw, const int cnt, const float4 (&pb)[BPL],
-                                          const float eps2, float (&ax)[BPL], float (&ay)[BPL], float (&az)[BPL],
-                                          float (&eb)[BPL]) {
-#pragma unroll 4
-    for (int i = 0; i < cnt; ++i) {
-        const float4 q = lst[i];
-        const float s2 = FEAT ? lw[i] : 0.0f;
+__device__ __forceinline__ void eval4(const float* lst, const int at, const ListBody (&b)[BPL], const float2 eps2,
+                                      ListSum (&a)[BPL]) {
+    const float4 X = *reinterpret_cast<const float4*>(lst + at);
+    const float4 Y = *reinterpret_cast<const float4*>(lst + kListCap + at);
+    const float4 Z = *reinterpret_cast<const float4*>(lst + 2 * kListCap + at);
+    const float4 M = *reinterpret_cast<const float4*>(lst + 3 * kListCap + at);
+    float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (FEAT) S = *reinterpret_cast<const float4*>(lst + 4 * kListCap + at);
 #pragma unroll
-        for (int k = 0; k < BPL; ++k) {
-            const float dx = __fsub_rn(q.x, pb[k].x);
-            const float dy = __fsub_rn(q.y, pb[k].y);
-            const float dz = __fsub_rn(q.z, pb[k].z);
-            const float d2 = dist2<false>(dx, dy, dz, eps2);
-            interact<false, FEAT>(q, dx, dy, dz, d2, ax[k], ay[k], az[k], eb[k], s2);
-        }
-    }
+    for (int k = 0; k < BPL; ++k)
+        interact2<FEAT>(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), make_float2(M.x, M.y),
+                        make_float2(S.x, S.y), b[k], eps2, a[k]);
+#pragma unroll
+    for (int k = 0; k < BPL; ++k)
+        interact2<FEAT>(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), make_float2(M.z, M.w),
+                        make_float2(S.z, S.w), b[k], eps2, a[k]);
 }
 
 // -------------------------------------------------------------------------------------
@@ -188,10 +195,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
     float4* const sq = sq_all + grp * cap;           // node record of each pending child
     int2* const se = se_all + grp * cap;             // (node index, bits of threshold or level factor)
     // list walk: the group's list of accepted records and its stack of (cell, level)
-    float4* const lst = reinterpret_cast<float4*>(smem_raw + (size_t)grp * list_group_bytes(cap));
-    float* const lw = reinterpret_cast<float*>(lst + kListCap);
-    float4* const ud = reinterpret_cast<float4*>(lw + kListCap);   // undecided cells of a round
-    int2* const cst = reinterpret_cast<int2*>(ud + 32);
+    float* const lst = reinterpret_cast<float*>(smem_raw + (size_t)grp * list_group_bytes(cap));
+    float* const ud = lst + 5 * kListCap;            // undecided cells of a round: x, y, z, threshold
+    int2* const cst = reinterpret_cast<int2*>(ud + 4 * 32);
     // deep-tree walk: (cell, next) per level
     int* const snode = LIST ? reinterpret_cast<int*>(cst) : reinterpret_cast<int*>(se);
     int* const snext = snode + kMaxDepth;
@@ -351,18 +357,34 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     rp2.z = __shfl_sync(0xffffffffu, mine2.z, r2src);
                 }
                 const unsigned lt = (1u << lane) - 1u;
-                if (lane == 0) cst[0] = make_int2(root, 0);
-                int ctop = 1, lcnt = 0, opened = 0;    // every tested child is accepted or opened
+                // from here on the bodies are held as ListBody (the empty asm keeps the compiler
+                // from holding their plain coordinates beside it)
+                ListBody lb[BPL];
+                ListSum ls[BPL];
+#pragma unroll
+                for (int k = 0; k < BPL; ++k) {
+                    float nx = -pb[k].x, ny = -pb[k].y, nz = -pb[k].z;
+                    asm volatile("" : "+f"(nx), "+f"(ny), "+f"(nz));
+                    lb[k].nx = make_float2(nx, nx), lb[k].ny = make_float2(ny, ny), lb[k].nz = make_float2(nz, nz);
+                    ls[k].x = ls[k].y = ls[k].z = ls[k].e = make_float2(0.f, 0.f);
+                }
+                const float2 eps22 = make_float2(eps2, eps2);
+                if (lane == 0) cst[0] = make_int2(root, __float_as_int(1.0f));
+                int ctop = 1, opened = 0;              // every tested child is accepted or opened
+                // the list is a ring of kListCap records; the first of the lcnt waiting ones is at
+                // lbase, 0 or 32
+                int lcnt = 0, lbase = 0;
                 long long accepted = 0;
                 __syncwarp();
                 while (ctop > 0) {
                     const int k4 = min(4, ctop);
                     const int ci = lane >> 3;
-                    int chk = kNull, lv = 0;
+                    int chk = kNull;
+                    float sl = 1.0f;                    // 4^-level of the cell whose child this is
                     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (ci < k4) {
                         const int2 e = cst[ctop - 1 - ci];
-                        lv = e.y;
+                        sl = __int_as_float(e.y);
                         const size_t o8 = ((size_t)(e.x - nbody) << 3) + (lane & 7);
                         chk = __ldg(child + o8);
                         q = __ldg(kids4 + o8);
@@ -370,15 +392,15 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     ctop -= k4;
                     __syncwarp();          // the popped entries are read before pushes reuse them
                     // children of a level-lv cell: t0 * 4^-lv + eps^2 (4^-lv exact)
-                    const float sl = __int_as_float((127 - 2 * lv) << 23);
                     bool acc = chk >= 0 && chk < nbody;
                     bool opn = false, inc = false;
+                    float qlb = 0.0f;
                     if (chk >= nbody) {
                         const float gx = fmaxf(fmaxf(__fsub_rn(q.x, hix), __fsub_rn(lox, q.x)), 0.0f);
                         const float gy = fmaxf(fmaxf(__fsub_rn(q.y, hiy), __fsub_rn(loy, q.y)), 0.0f);
                         const float gz = fmaxf(fmaxf(__fsub_rn(q.z, hiz), __fsub_rn(loz, q.z)), 0.0f);
                         const float dlb = dist2<false>(gx, gy, gz, eps2);
-                        const float qlb = PB ? __fmaf_rn(tlb, sl, eps2) : __fadd_rn(__fmul_rn(tlb, sl), eps2);
+                        qlb = PB ? __fmaf_rn(tlb, sl, eps2) : __fadd_rn(__fmul_rn(tlb, sl), eps2);
                         if (dlb >= qlb) {
                             acc = true;
                         } else {
@@ -397,29 +419,40 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                             }
                         }
                     }
-                    // undecided cells: the vote of every body, one cell after another
+                    // undecided cells: the vote of every body, two cells after two
                     const unsigned im = __ballot_sync(0xffffffffu, inc);
                     if (im) {
-                        // their records go to shared memory and every lane reads them back in turn
+                        // their records go to shared memory and every lane reads them back in turn,
+                        // with the finished threshold (fixed angle) or the level factor; the second
+                        // cell of an odd last pair is whatever lies there, its vote is not used
                         const int nud = __popc(im);
                         const int mine = __popc(im & lt);
-                        if (inc) ud[mine] = make_float4(q.x, q.y, q.z, sl);
+                        if (inc) {
+                            ud[mine] = q.x;
+                            ud[32 + mine] = q.y;
+                            ud[64 + mine] = q.z;
+                            ud[96 + mine] = PB ? sl : qlb;
+                        }
                         __syncwarp();
                         unsigned res = 0;
-#pragma unroll 2
-                        for (int j = 0; j < nud; ++j) {
-                            const float4 uq = ud[j];
-                            bool pass = true;
+                        for (int j = 0; j < nud; j += 2) {
+                            const float2 ux = *reinterpret_cast<const float2*>(ud + j);
+                            const float2 uy = *reinterpret_cast<const float2*>(ud + 32 + j);
+                            const float2 uz = *reinterpret_cast<const float2*>(ud + 64 + j);
+                            const float2 uq = *reinterpret_cast<const float2*>(ud + 96 + j);
+                            bool pass0 = true, pass1 = true;
 #pragma unroll
                             for (int k = 0; k < BPL; ++k) {
-                                const float dx = __fsub_rn(uq.x, pb[k].x);
-                                const float dy = __fsub_rn(uq.y, pb[k].y);
-                                const float dz = __fsub_rn(uq.z, pb[k].z);
-                                const float dq =
-                                    PB ? __fmaf_rn(t0[k], uq.w, eps2) : __fadd_rn(__fmul_rn(t0[k], uq.w), eps2);
-                                pass = pass && dist2<false>(dx, dy, dz, eps2) >= dq;
+                                const float2 dx = __fadd2_rn(ux, lb[k].nx);
+                                const float2 dy = __fadd2_rn(uy, lb[k].ny);
+                                const float2 dz = __fadd2_rn(uz, lb[k].nz);
+                                const float2 d2 =
+                                    __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, eps22)));
+                                pass0 = pass0 && d2.x >= (PB ? __fmaf_rn(t0[k], uq.x, eps2) : uq.x);
+                                pass1 = pass1 && d2.y >= (PB ? __fmaf_rn(t0[k], uq.y, eps2) : uq.y);
                             }
-                            res |= (__all_sync(0xffffffffu, pass) ? 1u : 0u) << j;
+                            res |= (__all_sync(0xffffffffu, pass0) ? 1u : 0u) << j;
+                            res |= (__all_sync(0xffffffffu, pass1) ? 2u : 0u) << j;
                         }
                         if (inc) {
                             acc = (res >> mine) & 1u;
@@ -435,30 +468,37 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         break;
                     }
                     if (acc) {
-                        const int at = lcnt + __popc(am & lt);
-                        lst[at] = q;
+                        const int at = (lbase + lcnt + __popc(am & lt)) & (kListCap - 1);
+                        lst[at] = q.x;
+                        lst[kListCap + at] = q.y;
+                        lst[2 * kListCap + at] = q.z;
+                        lst[3 * kListCap + at] = q.w;
                         // full width^2 of an accepted cell, r^2 * 4^-level (0 for a body)
-                        if constexpr (FEAT) lw[at] = chk >= nbody ? __fmul_rn(rr, sl) : 0.0f;
+                        if constexpr (FEAT) lst[4 * kListCap + at] = chk >= nbody ? __fmul_rn(rr, sl) : 0.0f;
                     }
-                    if (opn) cst[ctop + __popc(om & lt)] = make_int2(chk, min(lv + 1, kMaxDepth - 1));
+                    // children of a cell at level 63 are bodies: the factor stays a normal number
+                    if (opn) cst[ctop + __popc(om & lt)] = make_int2(chk, __float_as_int(__fmul_rn(sl, 0.25f)));
                     lcnt += __popc(am);
                     ctop += on;
                     __syncwarp();          // list and stack written before they are read
                     if (lcnt >= 32) {
-                        // 32 records at a time; the rest (at most 31) move to the front
-                        eval_list32<BPL, FEAT>(lst, lw, pb, eps2, ax, ay, az, eb);
+                        // 32 records at a time (unrolled completely: 2.6 % of the force at two bodies
+                        // per lane against unrolled by 8); at most 31 wait behind them
+#pragma unroll(BPL >= 2 ? 8 : 2)
+                        for (int i = 0; i < 32; i += 4) eval4<BPL, FEAT>(lst + lbase, i, lb, eps22, ls);
                         accepted += 32;
-                        __syncwarp();
-                        const int rest = lcnt - 32;
-                        if (lane < rest) {
-                            lst[lane] = lst[32 + lane];
-                            if constexpr (FEAT) lw[lane] = lw[32 + lane];
-                        }
-                        lcnt = rest;
-                        __syncwarp();
+                        lcnt -= 32;
+                        lbase ^= 32;
                     }
                     if (ctop == 0 && lcnt > 0) {
-                        eval_list<BPL, FEAT>(lst, lw, lcnt, pb, eps2, ax, ay, az, eb);
+                        // the last records, filled up to a multiple of four with massless ones
+                        if (lane < (-lcnt & 3)) {
+                            const int at = lbase + lcnt + lane;
+#pragma unroll
+                            for (int f = 0; f < (FEAT ? 5 : 4); ++f) lst[f * kListCap + at] = 0.0f;
+                        }
+                        __syncwarp();
+                        for (int i = 0; i < lcnt; i += 4) eval4<BPL, FEAT>(lst + lbase, i, lb, eps22, ls);
                         accepted += lcnt;
                         lcnt = 0;
                         __syncwarp();
@@ -467,9 +507,16 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                 if (walked) {
                     ninter = accepted;
                     visits = (int)accepted + opened;
+#pragma unroll
+                    for (int k = 0; k < BPL; ++k) {
+                        ax[k] = __fadd_rn(ls[k].x.x, ls[k].x.y);
+                        ay[k] = __fadd_rn(ls[k].y.x, ls[k].y.y);
+                        az[k] = __fadd_rn(ls[k].z.x, ls[k].z.y);
+                        if constexpr (FEAT) eb[k] = __fadd_rn(ls[k].e.x, ls[k].e.y);
+                    }
                 } else {
 #pragma unroll
-                    for (int k = 0; k < BPL; ++k) ax[k] = ay[k] = az[k] = eb[k] = 0.f;
+                    for (int k = 0; k < BPL; ++k) pb[k].x = -lb[k].nx.x, pb[k].y = -lb[k].ny.x, pb[k].z = -lb[k].nz.x;
                     __syncwarp();
                 }
             } else if (fast) {
