@@ -33,7 +33,8 @@ constexpr size_t force_smem_bytes(int threads, int cap) {
 // with their levels (a 64-entry stack also holds the per-level walk's 2 * kMaxDepth ints).
 constexpr int kListCap = 64;
 constexpr size_t list_group_bytes(int cap) {
-    return kListCap * (sizeof(float4) + sizeof(float)) + 32 * sizeof(float4) + (size_t)cap * sizeof(int2);
+    return kListCap * (sizeof(float4) + sizeof(float)) + 32 * sizeof(float4) + 4 * sizeof(float4) +
+           (size_t)cap * sizeof(int2);
 }
 constexpr size_t force_list_smem_bytes(int threads, int cap) { return (size_t)(threads / 32) * list_group_bytes(cap); }
 static_assert(kStackCapMin * sizeof(int2) >= 2 * kMaxDepth * sizeof(int), "the per-level walk fits the cell stack");
@@ -197,7 +198,8 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
     // list walk: the group's list of accepted records and its stack of (cell, level)
     float* const lst = reinterpret_cast<float*>(smem_raw + (size_t)grp * list_group_bytes(cap));
     float* const ud = lst + 5 * kListCap;            // undecided cells of a round: x, y, z, threshold
-    int2* const cst = reinterpret_cast<int2*>(ud + 4 * 32);
+    float4* const gc = reinterpret_cast<float4*>(ud + 4 * 32);     // the group's box and representatives
+    int2* const cst = reinterpret_cast<int2*>(gc + 4);
     // deep-tree walk: (cell, next) per level
     int* const snode = LIST ? reinterpret_cast<int*>(cst) : reinterpret_cast<int*>(se);
     int* const snext = snode + kMaxDepth;
@@ -226,20 +228,17 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
         const bool gvalid = gfirst < uend;       // the group has any body at all
         const float r = p.uradius[u];
         const float rr = __fmul_rn(r, r);
-        bool valid[BPL];
-        int b[BPL];
         float4 pb[BPL];
         float t0[BPL];
         float ax[BPL], ay[BPL], az[BPL], eb[BPL];
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
             const int sk = wi.x + 32 * k + lane;
-            valid[k] = sk < uend;
-            b[k] = gvalid ? p.sorted[valid[k] ? sk : gfirst] : 0;
-            pb[k] = node4[b[k]];
+            const int bk = gvalid ? p.sorted[sk < uend ? sk : gfirst] : 0;
+            pb[k] = node4[bk];
             float th2 = p.theta2;
             if constexpr (PB) {
-                const float th = p.theta_body[b[k]];
+                const float th = p.theta_body[bk];
                 th2 = __fmul_rn(th, th);
             }
             t0[k] = th2 > 0.0f ? __fdiv_rn(rr, th2) : rr;
@@ -369,12 +368,18 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     ls[k].x = ls[k].y = ls[k].z = ls[k].e = make_float2(0.f, 0.f);
                 }
                 const float2 eps22 = make_float2(eps2, eps2);
-                if (lane == 0) cst[0] = make_int2(root, __float_as_int(1.0f));
+                if (lane == 0) {
+                    cst[0] = make_int2(root, __float_as_int(1.0f));
+                    gc[0] = make_float4(lox, loy, loz, tlb);
+                    gc[1] = make_float4(hix, hiy, hiz, trep);
+                    gc[2] = rp;
+                    if constexpr (PB) gc[3] = rp2;
+                }
                 int ctop = 1, opened = 0;              // every tested child is accepted or opened
                 // the list is a ring of kListCap records; the first of the lcnt waiting ones is at
                 // lbase, 0 or 32
                 int lcnt = 0, lbase = 0;
-                long long accepted = 0;
+                int accepted = 0;                      // one body's: below the body count
                 __syncwarp();
                 while (ctop > 0) {
                     const int k4 = min(4, ctop);
@@ -396,22 +401,25 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     bool opn = false, inc = false;
                     float qlb = 0.0f;
                     if (chk >= nbody) {
-                        const float gx = fmaxf(fmaxf(__fsub_rn(q.x, hix), __fsub_rn(lox, q.x)), 0.0f);
-                        const float gy = fmaxf(fmaxf(__fsub_rn(q.y, hiy), __fsub_rn(loy, q.y)), 0.0f);
-                        const float gz = fmaxf(fmaxf(__fsub_rn(q.z, hiz), __fsub_rn(loz, q.z)), 0.0f);
+                        const float4 lo = gc[0], hi = gc[1];
+                        const float gx = fmaxf(fmaxf(__fsub_rn(q.x, hi.x), __fsub_rn(lo.x, q.x)), 0.0f);
+                        const float gy = fmaxf(fmaxf(__fsub_rn(q.y, hi.y), __fsub_rn(lo.y, q.y)), 0.0f);
+                        const float gz = fmaxf(fmaxf(__fsub_rn(q.z, hi.z), __fsub_rn(lo.z, q.z)), 0.0f);
                         const float dlb = dist2<false>(gx, gy, gz, eps2);
-                        qlb = PB ? __fmaf_rn(tlb, sl, eps2) : __fadd_rn(__fmul_rn(tlb, sl), eps2);
+                        qlb = PB ? __fmaf_rn(lo.w, sl, eps2) : __fadd_rn(__fmul_rn(lo.w, sl), eps2);
                         if (dlb >= qlb) {
                             acc = true;
                         } else {
-                            const float rx = __fsub_rn(q.x, rp.x), ry = __fsub_rn(q.y, rp.y), rz = __fsub_rn(q.z, rp.z);
-                            const float qr = PB ? __fmaf_rn(trep, sl, eps2) : qlb;
+                            const float4 r1 = gc[2];
+                            const float rx = __fsub_rn(q.x, r1.x), ry = __fsub_rn(q.y, r1.y), rz = __fsub_rn(q.z, r1.z);
+                            const float qr = PB ? __fmaf_rn(hi.w, sl, eps2) : qlb;
                             if (dist2<false>(rx, ry, rz, eps2) < qr) {
                                 opn = true;
                             } else if constexpr (PB) {
                                 // the smallest-angle body's own test (its threshold is the box's)
-                                const float sx = __fsub_rn(q.x, rp2.x), sy = __fsub_rn(q.y, rp2.y),
-                                            sz = __fsub_rn(q.z, rp2.z);
+                                const float4 r2 = gc[3];
+                                const float sx = __fsub_rn(q.x, r2.x), sy = __fsub_rn(q.y, r2.y),
+                                            sz = __fsub_rn(q.z, r2.z);
                                 if (dist2<false>(sx, sy, sz, eps2) < qlb) opn = true;
                                 else inc = true;
                             } else {
@@ -506,7 +514,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                 }
                 if (walked) {
                     ninter = accepted;
-                    visits = (int)accepted + opened;
+                    visits = accepted + opened;
 #pragma unroll
                     for (int k = 0; k < BPL; ++k) {
                         ax[k] = __fadd_rn(ls[k].x.x, ls[k].x.y);
@@ -653,7 +661,10 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
 
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
-            if (!valid[k]) continue;
+            // looked up again rather than held in registers through the walk
+            const int sk = wi.x + 32 * k + lane;
+            if (sk >= p.ubody[u + 1]) continue;
+            const int bk = p.sorted[sk];
             if (p.G != 1.0f) {
                 ax[k] = __fmul_rn(ax[k], p.G);
                 ay[k] = __fmul_rn(ay[k], p.G);
@@ -662,30 +673,30 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
             }
             my_inter += (unsigned long long)ninter;
             if (p.probe) {
-                p.probe[b[k]] = make_float4(ax[k], ay[k], az[k], eb[k]);
+                p.probe[bk] = make_float4(ax[k], ay[k], az[k], eb[k]);
                 continue;
             }
-            float4 v = p.vel[b[k]];
-            const float4 ao = p.acc[b[k]];
+            float4 v = p.vel[bk];
+            const float4 ao = p.acc[bk];
             if (step > 0) {
                 const float tx = __fmul_rn(__fsub_rn(ax[k], ao.x), p.dt);
                 const float ty = __fmul_rn(__fsub_rn(ay[k], ao.y), p.dt);
                 const float tz = __fmul_rn(__fsub_rn(az[k], ao.z), p.dt);
                 if (p.precise) {
-                    float4 kv = p.kvel[b[k]];
+                    float4 kv = p.kvel[bk];
                     float y1, t1;
                     y1 = __fsub_rn(__fmul_rn(tx, 0.5f), kv.x); t1 = __fadd_rn(v.x, y1); kv.x = __fsub_rn(__fsub_rn(t1, v.x), y1); v.x = t1;
                     y1 = __fsub_rn(__fmul_rn(ty, 0.5f), kv.y); t1 = __fadd_rn(v.y, y1); kv.y = __fsub_rn(__fsub_rn(t1, v.y), y1); v.y = t1;
                     y1 = __fsub_rn(__fmul_rn(tz, 0.5f), kv.z); t1 = __fadd_rn(v.z, y1); kv.z = __fsub_rn(__fsub_rn(t1, v.z), y1); v.z = t1;
-                    p.kvel[b[k]] = kv;
+                    p.kvel[bk] = kv;
                 } else {
                     v.x = madd<REF>(tx, 0.5f, v.x);
                     v.y = madd<REF>(ty, 0.5f, v.y);
                     v.z = madd<REF>(tz, 0.5f, v.z);
                 }
-                p.vel[b[k]] = v;
+                p.vel[bk] = v;
             }
-            p.acc[b[k]] = make_float4(ax[k], ay[k], az[k], eb[k]);
+            p.acc[bk] = make_float4(ax[k], ay[k], az[k], eb[k]);
         }
         if (p.item_cost) {
             // the item's cost: its group's visits (the deep walk counts accepted children);
@@ -701,18 +712,19 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
     if (lane == 0 && my_inter) atomicAdd(&p.st->interactions, my_inter);
 }
 
-// The kernels.  The 64-wide walks ask for at least 3 resident blocks of the largest
-// geometry: the compiler then keeps up to 85 registers per thread and compiles them to
-// 63-64 registers without spills (left to itself it compiles the per-body-angle walk to 48,
-// with less overlap in the visit loop: 1.6 % slower, the fixed-angle walk 0.7 % slower).
-// The other widths keep the compiler's own choice (with the same hint the 32-wide walk ran
-// 5-10 % slower).
+// The kernels.  The 64-wide walks ask for resident blocks of the largest geometry, which
+// bounds their registers: 3 (up to 80 registers) for all but the plain list walk, which fits in
+// 64 without spills and takes 4 (measured, us per step with 4 against 3: 256-universe ensemble
+// 6407 against 6488, 1M sphere 2618 against 2600; the list walk with per-body angles spills at
+// 64: 8 learned steps 18143 against 17435).  The per-visit walks end up with 64 registers (left
+// to itself the compiler takes 48, with less overlap in the visit loop: 0.7-1.6 % slower).
+// The other widths keep the compiler's own choice.
 template <int W, bool REF, bool PB, bool FEAT, bool LIST = false>
 __global__ void __launch_bounds__(kForceThreadsMax) force_kernel(StepParams p) {
     force_walk<W, REF, PB, FEAT, LIST>(p);
 }
 template <bool PB, bool FEAT, bool LIST>
-__global__ void __launch_bounds__(kForceThreadsMax, 3) force_kernel64(StepParams p) {
+__global__ void __launch_bounds__(kForceThreadsMax, LIST && !PB && !FEAT ? 4 : 3) force_kernel64(StepParams p) {
     force_walk<64, false, PB, FEAT, LIST>(p);
 }
 
