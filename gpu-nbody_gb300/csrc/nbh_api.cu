@@ -1121,8 +1121,12 @@ int nbh_diagnostics(nbh_sim* sim, int32_t flags, nbh_diag* out, int32_t nout) {
     double* d_part = nullptr;
     double* d_out = nullptr;
     cudaError_t e;
-    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&d_part), sizeof(double) * kDiagFields * sim->nchunks, s)) !=
-            cudaSuccess ||
+    int max_chunks = 1;
+    for (int u = 0; u < sim->nuniv; ++u)
+        max_chunks = std::max(max_chunks, (sim->h_ubody[u + 1] - sim->h_ubody[u] + 255) / 256);
+    const int slices = potential ? diag_slices(sim->nchunks, max_chunks, sim->sms) : 0;
+    if ((e = cudaMallocAsync(reinterpret_cast<void**>(&d_part),
+                             sizeof(double) * (kDiagMoments + 2 * (size_t)slices) * sim->nchunks, s)) != cudaSuccess ||
         (e = cudaMallocAsync(reinterpret_cast<void**>(&d_out), sizeof(double) * kDiagFields * sim->nuniv, s)) !=
             cudaSuccess) {
         if (d_part) cudaFreeAsync(d_part, s);
@@ -1130,7 +1134,7 @@ int nbh_diagnostics(nbh_sim* sim, int32_t flags, nbh_diag* out, int32_t nout) {
     }
     const nbh_config& c = sim->cfg;
     const float eps2f = c.eps2 > 0.0f ? c.eps2 : c.eps * c.eps;
-    launch_diagnostics(sim->node4, sim->vel, sim->chunks, sim->nchunks, sim->ubody, sim->nuniv, potential, eps2f,
+    launch_diagnostics(sim->node4, sim->vel, sim->chunks, sim->nchunks, sim->ubody, sim->nuniv, slices, eps2f,
                        d_part, d_out, s);
     std::vector<double> h((size_t)kDiagFields * sim->nuniv);
     cudaMemcpyAsync(h.data(), d_out, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, s);

@@ -50,8 +50,11 @@ void launch_direct_f64(const float4* node4, int nidx, const int* idx, const int2
 // energy, 11 / 12 sum_i m_i phi_i softened / unsoftened (each pair twice).
 constexpr int kDiagMoments = 11;
 constexpr int kDiagFields = 13;
+// slices: blocks per chunk of the pair potential (diag_slices; 0: no potential).  part: per
+// chunk kDiagMoments doubles, then two per chunk and slice.
+int diag_slices(int nchunks, int max_chunks, int sms);
 void launch_diagnostics(const float4* node4, const float4* vel, const int4* chunks, int nchunks, const int* ubody,
-                        int nuniv, bool potential, float eps2, double* part, double* out, cudaStream_t s);
+                        int nuniv, int slices, float eps2, double* part, double* out, cudaStream_t s);
 
 struct DevState;
 void launch_wait_selftest(const int* flag, unsigned long long limit_ns, DevState* st, cudaStream_t s);

@@ -87,3 +87,32 @@ def test_energy_and_momentum_conserved_over_a_run():
     assert de < 1e-4
     assert dp < 1e-4
     assert dl < 1e-4
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 512, 513, 768, 1023, 1025, 4097])
+def test_pair_potential_counts_every_pair_once(n):
+    """One chunk, even and odd rings of chunks, ragged last chunks.  A pair term carries at most
+    about 4e-7 (FP32 differences and inverse square root) and a tile's FP32 sum less than 2e-6
+    in the mean over its targets: the bound of the other tests."""
+    arrs = plummer(n, seed=33)
+    g = gpu_sim(theta=0.5, eps=0.05, dt=0.01)
+    g.load(*arrs)
+    (d,) = g.diagnostics(potential=True)
+    r = O.diagnostics_f64(*arrs, eps=0.05)
+    assert abs(d["potential"] - r["potential"]) <= 2e-6 * abs(r["potential"])
+    assert abs(d["potential_unsoftened"] - r["potential_unsoftened"]) <= 2e-6 * abs(r["potential_unsoftened"])
+
+
+def test_pair_potential_of_a_subnormal_squared_distance():
+    """Two bodies of different chunks 3.2e-20 apart: their squared distance, 1e-39, is a
+    subnormal float (relative spacing 1.4e-6, so 7e-7 in the inverse distance)."""
+    n = 600
+    arrs = [a.copy() for a in plummer(n, seed=34)]
+    for k in range(3):
+        arrs[k][10] = arrs[k][500] = 0.0
+    arrs[0][500] = 3.2e-20
+    g = gpu_sim(theta=0.5, eps=0.05, dt=0.01)
+    g.load(*arrs)
+    (d,) = g.diagnostics(potential=True)
+    want = -np.float64(arrs[6][10]) * arrs[6][500] / np.float64(arrs[0][500])
+    assert abs(d["potential_unsoftened"] - want) <= 2e-6 * abs(want)
