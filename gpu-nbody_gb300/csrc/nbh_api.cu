@@ -7,6 +7,7 @@
 // (:276-290).  Here a step is one graph launch of the six kernels on a stream, and the
 // status word is read once per nbh_step call.
 #include "nbh_common.cuh"
+#include "nbh_direct.cuh"
 #include "nbh_kernels.h"
 #include "nbh_theta.h"
 
@@ -437,11 +438,11 @@ static cudaError_t direct_scratch_for(int device, StaticDirectScratch** out) {
 
 // Same sum as direct_f64_kernel; each target finds its universe's body range from the
 // universe offsets itself, and the partial sums land in the scratch's SoA columns.
-__global__ void __launch_bounds__(256) direct_f64_static_kernel(const float4* __restrict__ node4,
+__global__ void __launch_bounds__(kDirectTile) direct_f64_static_kernel(const float4* __restrict__ node4,
                                                                 const int* __restrict__ ubody, int nuniv,
                                                                 StaticDirectScratch* sc, int nidx, double eps2,
                                                                 double G) {
-    __shared__ double tile[256][4];
+    __shared__ Src64 tile[kDirectTile];
     __shared__ int blo, bhi;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = t < nidx;
@@ -470,35 +471,21 @@ __global__ void __launch_bounds__(256) direct_f64_static_kernel(const float4* __
         const float4 q = node4[i];
         xi = q.x; yi = q.y; zi = q.z;
     }
-    double sx = 0, sy = 0, sz = 0;
-    for (int base = s0; base < s1; base += 256) {
+    double a[3] = {0.0, 0.0, 0.0};
+    for (int base = s0; base < s1; base += kDirectTile) {
         const int j = base + threadIdx.x;
         __syncthreads();
         if (j < s1) {
             const float4 q = node4[j];
-            tile[threadIdx.x][0] = q.x; tile[threadIdx.x][1] = q.y;
-            tile[threadIdx.x][2] = q.z; tile[threadIdx.x][3] = q.w;
+            tile[threadIdx.x] = Src64{q.x, q.y, q.z, q.w};
         }
         __syncthreads();
-        const int cnt = min(256, s1 - base);
-        if (valid) {
-            for (int k = 0; k < cnt; ++k) {
-                const int jj = base + k;
-                if (jj < lo || jj >= hi) continue;
-                const double dx = tile[k][0] - xi, dy = tile[k][1] - yi, dz = tile[k][2] - zi;
-                const double d2 = dx * dx + dy * dy + dz * dz + eps2;
-                const double inv = 1.0 / sqrt(d2);
-                const double f = tile[k][3] * inv * inv * inv;
-                sx += dx * f;
-                sy += dy * f;
-                sz += dz * f;
-            }
-        }
+        direct_tile(tile, max(0, lo - base), min(min(kDirectTile, s1 - base), hi - base), xi, yi, zi, eps2, a);
     }
     if (valid) {
-        atomicAdd(&sc->ax[t], G * sx);
-        atomicAdd(&sc->ay[t], G * sy);
-        atomicAdd(&sc->az[t], G * sz);
+        atomicAdd(&sc->ax[t], G * a[0]);
+        atomicAdd(&sc->ay[t], G * a[1]);
+        atomicAdd(&sc->az[t], G * a[2]);
     }
 }
 
@@ -1093,7 +1080,7 @@ int nbh_direct_f64(nbh_sim* sim, int32_t nidx, const int32_t* idx, double* ax, d
     const nbh_config& c = sim->cfg;
     const float eps2f = c.eps2 > 0.0f ? c.eps2 : c.eps * c.eps;
     const int bx = (nidx + 255) / 256;
-    const int ysplit = std::max(1, std::min(256, (8 * sim->sms + bx - 1) / bx));
+    const int ysplit = direct_slices(bx, sim->sms);
     launch_direct_f64(sim->node4, nidx, d_idx, d_range, (double)eps2f, (double)c.G, d_out, ysplit, s);
     std::vector<double> out(3 * (size_t)nidx);
     cudaMemcpyAsync(out.data(), d_out, sizeof(double) * 3 * nidx, cudaMemcpyDeviceToHost, s);
@@ -1498,7 +1485,7 @@ int nbh_direct_f64_static(nbh_sim* sim, int32_t nidx, const int32_t* idx, double
     const nbh_config& c = sim->cfg;
     const float eps2f = c.eps2 > 0.0f ? c.eps2 : c.eps * c.eps;
     const int bx = (nidx + 255) / 256;
-    const int ysplit = std::max(1, std::min(256, (8 * sim->sms + bx - 1) / bx));
+    const int ysplit = direct_slices(bx, sim->sms);
     direct_f64_static_kernel<<<dim3(bx, ysplit), 256, 0, s>>>(sim->node4, sim->ubody, sim->nuniv, sc, nidx,
                                                               (double)eps2f, (double)c.G);
     CK(cudaGetLastError());

@@ -1,6 +1,7 @@
 // nbh_aux.cu — leapfrog integration, host<->device packing, the float4 export, the FP64
 // direct sum used to measure force error, and the FP32 throughput probe.
 #include "nbh_common.cuh"
+#include "nbh_direct.cuh"
 #include "nbh_kernels.h"
 
 #include <cstdint>
@@ -191,10 +192,6 @@ __global__ void export4_kernel(int n, const float4* node4, const float4* vel, fl
 // FP64 direct sum a_i = G sum_j m_j (x_j - x_i) / (|x_j - x_i|^2 + eps^2)^(3/2) for a list
 // of bodies, each over the bodies [lo, hi) of its own universe.  Sources are split across
 // blockIdx.y and the partial sums added atomically (outputs zeroed by the caller).
-constexpr int kDirectTile = 256;
-struct Src64 {
-    double x, y, z, m;
-};
 __global__ void __launch_bounds__(kDirectTile) direct_f64_kernel(const float4* __restrict__ node4, int nidx,
                                                                  const int* __restrict__ idx,
                                                                  const int2* __restrict__ range, double eps2,
@@ -225,7 +222,7 @@ __global__ void __launch_bounds__(kDirectTile) direct_f64_kernel(const float4* _
         const float4 q = node4[i];
         xi = q.x; yi = q.y; zi = q.z;
     }
-    double sx = 0, sy = 0, sz = 0;
+    double a[3] = {0.0, 0.0, 0.0};
     for (int base = s0; base < s1; base += kDirectTile) {
         const int j = base + threadIdx.x;
         __syncthreads();
@@ -234,26 +231,13 @@ __global__ void __launch_bounds__(kDirectTile) direct_f64_kernel(const float4* _
             tile[threadIdx.x] = Src64{q.x, q.y, q.z, q.w};
         }
         __syncthreads();
-        const int cnt = min(kDirectTile, s1 - base);
-        if (valid) {
-            for (int k = 0; k < cnt; ++k) {
-                const int jj = base + k;
-                if (jj < rg.x || jj >= rg.y) continue;
-                const Src64 q = tile[k];
-                const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-                const double d2 = dx * dx + dy * dy + dz * dz + eps2;
-                const double inv = 1.0 / sqrt(d2);
-                const double f = q.m * inv * inv * inv;
-                sx += dx * f;
-                sy += dy * f;
-                sz += dz * f;
-            }
-        }
+        // the target's own universe within the tile (none for threads without a target)
+        direct_tile(tile, max(0, rg.x - base), min(min(kDirectTile, s1 - base), rg.y - base), xi, yi, zi, eps2, a);
     }
     if (valid) {
-        atomicAdd(out + 3 * t + 0, G * sx);
-        atomicAdd(out + 3 * t + 1, G * sy);
-        atomicAdd(out + 3 * t + 2, G * sz);
+        atomicAdd(out + 3 * t + 0, G * a[0]);
+        atomicAdd(out + 3 * t + 1, G * a[1]);
+        atomicAdd(out + 3 * t + 2, G * a[2]);
     }
 }
 

@@ -116,3 +116,28 @@ def test_pair_potential_of_a_subnormal_squared_distance():
     (d,) = g.diagnostics(potential=True)
     want = -np.float64(arrs[6][10]) * arrs[6][500] / np.float64(arrs[0][500])
     assert abs(d["potential_unsoftened"] - want) <= 2e-6 * abs(want)
+
+
+@pytest.mark.parametrize("scale,eps", [(1.0, 0.05), (1.0, 1e-3), (3e18, 0.05), (1e19, 0.05), (1e-6, 1e-16)])
+def test_direct_f64_over_the_range_of_distances(scale, eps):
+    """Squared distances inside, across and above the range of normal floats, and a softening
+    below 2^-100: both entry points against extended precision.  A term is at most 8e-16 off and
+    the sum of n of them n 2^-53 of the sum of their magnitudes."""
+    n = 300
+    arrs = plummer(n, seed=35)
+    pos = [(a * np.float32(scale)).astype(np.float32) for a in arrs[:3]]
+    g = gpu_sim(theta=0.5, eps=eps, dt=0.01)
+    g.load(*pos, *arrs[3:])
+    idx = np.arange(n, dtype=np.int32)
+    p = np.stack(pos).astype(np.longdouble)
+    eps2 = np.longdouble(np.float32(eps) * np.float32(eps))
+    d = p[:, None, :] - p[:, :, None]
+    d2 = (d * d).sum(0) + eps2
+    f = arrs[6].astype(np.longdouble)[None] / (d2 * np.sqrt(d2))
+    want = (d * f[None]).sum(2)
+    size = np.abs(d * f[None]).sum(2)
+    static = [np.empty(n, np.float64) for _ in range(3)]
+    assert g._L.nbh_direct_f64_static(g._h, n, idx.ctypes.data, *[a.ctypes.data for a in static]) == 0
+    for got in (g.direct_f64(idx), static):
+        for k in range(3):
+            assert (np.abs(got[k] - want[k]) <= (8e-16 + n * 2.0 ** -53) * size[k]).all()
