@@ -1664,33 +1664,37 @@ int nbh_theta_features(nbh_sim* sim, float* feat, int32_t use_probe) {
 // ---- training of the model (FP32, on the device) ---------------------------------------
 
 namespace {
+// One device allocation for a call: samples, targets, outputs, parameters, gradient, Adam
+// moments, loss and (with targets) the training passes' work space.
 struct TrainBufs {
-    float *X = nullptr, *T = nullptr, *prm = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr, *loss = nullptr;
-    MlpWork w{};
+    float* all = nullptr;
+    float *X = nullptr, *T = nullptr, *Y = nullptr, *prm = nullptr, *grad = nullptr, *m1 = nullptr, *m2 = nullptr,
+          *loss = nullptr;
+    TrainWork w{};
+    int sms = 0;
     ~TrainBufs() {
-        void* ptrs[] = {X, T, prm, grad, m1, m2, loss, w.H1, w.H2, w.Y, w.dH1, w.dH2, w.dY};
-        for (void* q : ptrs)
-            if (q) cudaFree(q);
+        if (all) cudaFree(all);
     }
 };
 
-int train_setup(TrainBufs& b, const float* params, const float* X, const float* T, int n) {
+int train_setup(TrainBufs& b, int device, const float* params, const float* X, const float* T, int n) {
     nbh_sim* sim = nullptr;
-    std::vector<float> xt((size_t)kMlpIn * n);   // feature-major for the kernels
-    for (int s = 0; s < n; ++s)
-        for (int k = 0; k < kMlpIn; ++k) xt[(size_t)k * n + s] = X[(size_t)s * kMlpIn + k];
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.X), sizeof(float) * xt.size()));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.T), sizeof(float) * n));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.prm), sizeof(float) * kMlpParams));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.grad), sizeof(float) * kMlpParams));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.m1), sizeof(float) * kMlpParams));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.m2), sizeof(float) * kMlpParams));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.loss), sizeof(float)));
-    float** acts[] = {&b.w.H1, &b.w.H2, &b.w.dH1, &b.w.dH2};
-    for (float** a : acts) CK(cudaMalloc(reinterpret_cast<void**>(a), sizeof(float) * kMlpHid * n));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.w.Y), sizeof(float) * n));
-    CK(cudaMalloc(reinterpret_cast<void**>(&b.w.dY), sizeof(float) * n));
-    CK(cudaMemcpy(b.X, xt.data(), sizeof(float) * xt.size(), cudaMemcpyHostToDevice));
+    CK(cudaDeviceGetAttribute(&b.sms, cudaDevAttrMultiProcessorCount, device));
+    CK(prepare_train_kernels());
+    const size_t sizes[] = {(size_t)kMlpIn * n, (size_t)n, (size_t)n, (size_t)kMlpParams, (size_t)kMlpParams,
+                            (size_t)kMlpParams, (size_t)kMlpParams, 1};
+    float** ptrs[] = {&b.X, &b.T, &b.Y, &b.prm, &b.grad, &b.m1, &b.m2, &b.loss};
+    size_t total = 0;
+    for (size_t c : sizes) total += (c + 63) / 64 * 64;
+    const size_t work = T ? train_work_bytes(n, b.sms, nullptr, nullptr) : 0;
+    CK(cudaMalloc(reinterpret_cast<void**>(&b.all), sizeof(float) * total + work));
+    float* at = b.all;
+    for (int k = 0; k < 8; ++k) {
+        *ptrs[k] = at;
+        at += (sizes[k] + 63) / 64 * 64;
+    }
+    if (T) train_work_bytes(n, b.sms, &b.w, at);
+    CK(cudaMemcpy(b.X, X, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice));
     if (T) CK(cudaMemcpy(b.T, T, sizeof(float) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.prm, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
     CK(cudaMemset(b.m1, 0, sizeof(float) * kMlpParams));
@@ -1705,10 +1709,10 @@ int nbh_mlp_forward(int32_t device, const float* params, const float* X, int32_t
     CK(cudaSetDevice(device));
     TrainBufs b;
     int e;
-    if ((e = train_setup(b, params, X, nullptr, n))) return e;
-    mlp_forward(b.prm, b.X, n, b.w, nullptr);
+    if ((e = train_setup(b, device, params, X, nullptr, n))) return e;
+    mlp_forward(b.prm, b.X, n, b.Y, b.sms, nullptr);
     CK(cudaGetLastError());
-    CK(cudaMemcpy(y, b.w.Y, sizeof(float) * n, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(y, b.Y, sizeof(float) * n, cudaMemcpyDeviceToHost));
     return NBH_OK;
 }
 
@@ -1720,8 +1724,8 @@ int nbh_mlp_grad(int32_t device, const float* params, const float* X, const floa
     CK(cudaSetDevice(device));
     TrainBufs b;
     int e;
-    if ((e = train_setup(b, params, X, T, n))) return e;
-    mlp_grad(b.prm, b.X, b.T, n, quantile, b.w, b.grad, b.loss, nullptr);
+    if ((e = train_setup(b, device, params, X, T, n))) return e;
+    mlp_grad(b.prm, b.X, b.T, n, quantile, b.w, b.grad, b.loss, b.sms, nullptr);
     CK(cudaGetLastError());
     CK(cudaMemcpy(grad, b.grad, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
     if (loss) CK(cudaMemcpy(loss, b.loss, sizeof(float), cudaMemcpyDeviceToHost));
@@ -1736,7 +1740,7 @@ int nbh_mlp_train(int32_t device, float* params, const float* X, const float* T,
     CK(cudaSetDevice(device));
     TrainBufs b;
     int e;
-    if ((e = train_setup(b, params, X, T, n))) return e;
+    if ((e = train_setup(b, device, params, X, T, n))) return e;
     cudaStream_t s = nullptr;
     // The rate falls linearly to zero over the last 30 % of the steps.  The pinball loss's
     // gradient does not shrink near its minimum, so at a constant rate the fitted quantile
@@ -1745,12 +1749,11 @@ int nbh_mlp_train(int32_t device, float* params, const float* X, const float* T,
     // next; with the decay it ends at 0.198-0.202.
     const int t_decay = iters - (3 * iters) / 10;
     for (int it = 1; it <= iters; ++it) {
-        mlp_grad(b.prm, b.X, b.T, n, quantile, b.w, b.grad, b.loss, s);
         const float lr_t = it <= t_decay ? lr : lr * (float)(iters - it + 1) / (float)(iters - t_decay + 1);
-        adam_step(b.prm, b.grad, b.m1, b.m2, lr_t, it, s);
+        mlp_train_step(b.prm, b.X, b.T, n, quantile, b.w, b.loss, b.m1, b.m2, lr_t, it, b.sms, s);
     }
     // loss of the final parameters
-    mlp_grad(b.prm, b.X, b.T, n, quantile, b.w, b.grad, b.loss, s);
+    mlp_grad(b.prm, b.X, b.T, n, quantile, b.w, b.grad, b.loss, b.sms, s);
     CK(cudaGetLastError());
     CK(cudaMemcpy(params, b.prm, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
     if (loss) CK(cudaMemcpy(loss, b.loss, sizeof(float), cudaMemcpyDeviceToHost));

@@ -25,19 +25,24 @@ struct ThetaDev {
     float theta_min, theta_max;
 };
 
-// Work buffers of the training kernels for a batch of n samples.
-struct MlpWork {
-    float *H1, *H2, *Y, *dH1, *dH2, *dY;
-};
-
 void launch_theta(const StepParams& p, const ThetaDev* mdl, float* theta_out, int grid, cudaStream_t s);
 void launch_features(const StepParams& p, const ThetaDev* mdl, const float4* src, const float* theta_prev,
                      float* feat, int grid, cudaStream_t s);
 void launch_model_convert(const float* prm, ThetaDev* mdl, cudaStream_t s);
 
-void mlp_grad(const float* prm, const float* X, const float* T, int n, float q, MlpWork& w, float* grad, float* loss,
-              cudaStream_t s);
-void mlp_forward(const float* prm, const float* X, int n, MlpWork& w, cudaStream_t s);
-void adam_step(float* prm, const float* g, float* m1, float* m2, float lr, int t, cudaStream_t s);
+// Training (FP32).  X: n samples of kMlpIn features, row-major.  Work space: one allocation of
+// train_work_bytes() bytes, laid out by the same call with its base (16-byte aligned).
+// prepare_train_kernels() once per call on the device in use.
+struct TrainWork {
+    void* tiles;
+    float *part, *lossp;
+};
+size_t train_work_bytes(int n, int sms, TrainWork* w, void* base);
+cudaError_t prepare_train_kernels();
+void mlp_forward(const float* prm, const float* X, int n, float* Y, int sms, cudaStream_t s);
+void mlp_grad(const float* prm, const float* X, const float* T, int n, float q, TrainWork w, float* grad, float* loss,
+              int sms, cudaStream_t s);
+void mlp_train_step(float* prm, const float* X, const float* T, int n, float q, TrainWork w, float* loss, float* m1,
+                    float* m2, float lr, int t, int sms, cudaStream_t s);
 
 }  // namespace nbh

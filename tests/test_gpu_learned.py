@@ -195,3 +195,26 @@ def test_trained_model_gains_over_fixed_theta():
     assert gain > 1.05
     assert r["learned"]["p99"] <= r["plain"]["p99"]
     assert r["learned"]["p99_max"] <= r["plain"]["p99_max"]
+
+
+@pytest.mark.parametrize("n", [1, 5, 63, 64, 65, 3001, 40000])
+def test_mlp_passes_at_tile_edges(n):
+    """Partial tiles, one tile, a ragged last tile, and more tiles than blocks.  FP32 sums against
+    FP64, relative to the gradient's scale; at most 4 of the samples may fall on the other side
+    of a kink (a residual or a unit within rounding of zero), each worth at most 12 / n here."""
+    import mlp_ref
+    L, lib = _lib()
+    rng = np.random.default_rng(100 + n)
+    p = (rng.standard_normal(mlp_ref.NPARAMS) * 0.2).astype(np.float32)
+    X = rng.standard_normal((n, 12)).astype(np.float32)
+    T = rng.standard_normal(n).astype(np.float32)
+    g = np.empty(mlp_ref.NPARAMS, np.float32)
+    y = np.empty(n, np.float32)
+    loss = C.c_float()
+    L.check(lib.nbh_mlp_grad(0, p.ctypes.data, X.ctypes.data, T.ctypes.data, n, 0.2, g.ctypes.data, C.byref(loss)))
+    L.check(lib.nbh_mlp_forward(0, p.ctypes.data, X.ctypes.data, n, y.ctypes.data))
+    rl, rg = mlp_ref.grad(p, X, T, 0.2)
+    kinks = 0 if n <= 3001 else 4
+    assert abs(loss.value - rl) <= 1e-5 * max(1.0, abs(rl))
+    assert np.abs(g - rg).max() <= 2e-5 * np.abs(rg).max() + kinks * 12.0 / n
+    np.testing.assert_allclose(y, mlp_ref.forward(p, X), rtol=1e-4, atol=1e-4)
