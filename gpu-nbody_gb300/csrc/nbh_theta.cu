@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kWeightThreads) mlp_weights_kernel(const Train
     }
 }
 
-// Adds the chunks, in order, into grad, or (lr > 0) into one Adam step of prm; the last block
+// Adds the chunks, in order (many of them in FP64), into grad, or (lr > 0) into one Adam step of prm; the last block
 // adds the loss.
 struct AdamStep {
     float *prm, *m1, *m2;
@@ -648,8 +648,15 @@ __global__ void __launch_bounds__(kReduceThreads)
     const int i = blockIdx.x * kReduceThreads + threadIdx.x;
     if (i >= kMlpParams) return;
     float gi = 0.f;
+    if (chunks <= 16) {
+#pragma unroll 8
+        for (int c = 0; c < chunks; ++c) gi += part[(size_t)c * kMlpParams + i];
+    } else {
+        double sum = 0.0;                             // one rounding instead of up to 63
 #pragma unroll 16
-    for (int c = 0; c < chunks; ++c) gi += part[(size_t)c * kMlpParams + i];
+        for (int c = 0; c < chunks; ++c) sum += (double)part[(size_t)c * kMlpParams + i];
+        gi = (float)sum;
+    }
     if (ad.lr > 0.f) {
         const float a = ad.b1 * ad.m1[i] + (1.f - ad.b1) * gi;
         const float v = ad.b2 * ad.m2[i] + (1.f - ad.b2) * gi * gi;
