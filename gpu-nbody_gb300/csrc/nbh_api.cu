@@ -175,6 +175,7 @@ StepParams step_params(const nbh_sim* sim) {
     p.theta_group = sim->theta_group;
     p.stack_cap = sim->stack_cap;
     p.force_list = sim->force_list ? 1 : 0;
+    p.sms = sim->sms;
     p.buckets = sim->buckets;
     p.bwork = sim->bwork;
     p.bstack = sim->bstack;

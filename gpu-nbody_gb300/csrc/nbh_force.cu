@@ -37,6 +37,27 @@ constexpr size_t list_group_bytes(int cap) {
            (size_t)cap * sizeof(int2);
 }
 constexpr size_t force_list_smem_bytes(int threads, int cap) { return (size_t)(threads / 32) * list_group_bytes(cap); }
+
+// Groups shared among the warps of a block: cells waiting per warp when they are dealt out, the
+// room for the breadth-first queue, and what the warps tell each other.
+constexpr int kSplitFront = 8;
+constexpr int kSplitQueue = 256;
+constexpr int kSplitMax = 8;
+constexpr int kSplitKeep = kSplitQueue / (2 * 32);   // entries per lane of a warp's share, at two warps
+struct SplitTeam {
+    int item, status;
+    int accepted[kSplitMax], opened[kSplitMax];
+};
+// Warps per group for `groups` groups: doubled, up to 8, while there are fewer than 24 warps per
+// SM (the walk's residency).  Force stage of Plummer spheres in groups of 64, us, shared / one
+// warp each: 1,000 bodies 51 / 84, 16,384 145 / 449, 65,536 262 / 674, 100,003 367 / 702,
+// 200,000 (two warps) 549 / 743; at 300,000 two warps lose, 881 / 786.  With kSplitFront 4 and
+// 12 in place of 8: 172 and 149 at 16,384, 262 and 306 at 65,536.
+static int force_split(int groups, int sms) {
+    int s = 1;
+    while (s < kSplitMax && groups * s < 24 * sms) s *= 2;
+    return s;
+}
 static_assert(kStackCapMin * sizeof(int2) >= 2 * kMaxDepth * sizeof(int), "the per-level walk fits the cell stack");
 
 // Opening threshold of tree level L (root = 0): r^2/theta^2 * 4^-L + eps^2
@@ -174,10 +195,30 @@ __device__ __forceinline__ void eval4(const float* lst, const int at, const List
 // list order (rounding may differ from it in the last bits).  A cell stack that would
 // overflow restarts the group on the per-level walk (stack_cap entries: 256 by default,
 // enough for every 64-body group of the benchmarked spheres, which needed at most 99).
-template <int W, bool REF, bool PB, bool FEAT, bool LIST = false>
+//
+// SPLIT (with LIST): a block of S = 2, 4 or 8 warps shares one group.  A group's walk is one
+// chain of rounds, and a universe with fewer groups than the GPU has room for warps leaves
+// most of it idle (16,384 bodies in groups of 32: 512 warps on 608 schedulers).  Every warp
+// expands the tree from the root breadth first, all of them the same way, until kSplitFront
+// cells per warp wait; then warp w keeps every S-th of them and walks on alone, and the sums are
+// added in the order of the warps at the end.  The records accepted on the way are dealt out
+// the same way.  S depends on the number of groups only (force_split), so that the launch
+// geometry does not change the order of the sums.
+template <int W, bool REF, bool PB, bool FEAT, bool LIST = false, bool SPLIT = false>
 __device__ __forceinline__ void force_walk(const StepParams& p) {
     static_assert(!LIST || (W >= 32 && !REF), "the list walk takes whole-warp groups and FMA arithmetic");
-    if (load_status(p.st)) return;
+    static_assert(!SPLIT || LIST, "only the list walk shares a group among warps");
+    __shared__ SplitTeam team;
+    const int wt = SPLIT ? (int)(threadIdx.x >> 5) : 0;   // this warp of the S that share a group
+    const int S = SPLIT ? (int)(blockDim.x >> 5) : 1;
+    if constexpr (SPLIT) {
+        // one read of the status word for the whole block, which meets at barriers
+        if (threadIdx.x == 0) team.status = load_status(p.st);
+        __syncthreads();
+        if (team.status) return;
+    } else {
+        if (load_status(p.st)) return;
+    }
     if (p.feat_gate && theta_bound_step(p.st, p.st->step) != (p.feat_gate == 1)) return;
     constexpr int GL = group_lanes<W>();            // lanes per group
     constexpr int BPL = W / GL;                     // bodies per lane
@@ -196,7 +237,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
     float4* const sq = sq_all + grp * cap;           // node record of each pending child
     int2* const se = se_all + grp * cap;             // (node index, bits of threshold or level factor)
     // list walk: the group's list of accepted records and its stack of (cell, level)
-    float* const lst = reinterpret_cast<float*>(smem_raw + (size_t)grp * list_group_bytes(cap));
+    float* const lst = reinterpret_cast<float*>(smem_raw + (size_t)grp * list_group_bytes(SPLIT ? max(cap, kSplitQueue) : cap));
     float* const ud = lst + 5 * kListCap;            // undecided cells of a round: x, y, z, threshold
     float4* const gc = reinterpret_cast<float4*>(ud + 4 * 32);     // the group's box and representatives
     int2* const cst = reinterpret_cast<int2*>(gc + 4);
@@ -216,8 +257,15 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
 
     for (;;) {
         int item = 0;
-        if (lane == 0) item = atomicAdd(&p.st->force_next, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
+        if constexpr (SPLIT) {
+            __syncthreads();                 // the last group's sums have been read
+            if (threadIdx.x == 0) team.item = atomicAdd(&p.st->force_next, 1);
+            __syncthreads();
+            item = team.item;
+        } else {
+            if (lane == 0) item = atomicAdd(&p.st->force_next, 1);
+            item = __shfl_sync(0xffffffffu, item, 0);
+        }
         if (item >= nitems) break;
         if (p.item_order) item = p.item_order[item];   // costly items first (see item_order_kernel)
         const int2 wi = items[item];
@@ -376,25 +424,49 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     if constexpr (PB) gc[3] = rp2;
                 }
                 int ctop = 1, opened = 0;              // every tested child is accepted or opened
+                // breadth first (SPLIT) until there are enough cells to share: the cells from
+                // `head` on wait in order; dealt: accepted records so far
+                bool spread = SPLIT;
+                int head = 0, dealt = 0;
                 // the list is a ring of kListCap records; the first of the lcnt waiting ones is at
                 // lbase, 0 or 32
                 int lcnt = 0, lbase = 0;
                 int accepted = 0;                      // one body's: below the body count
                 __syncwarp();
-                while (ctop > 0) {
-                    const int k4 = min(4, ctop);
+                for (;;) {
+                    if (SPLIT && spread &&
+                        (ctop == head || ctop - head >= kSplitFront * S || ctop + 32 > kSplitQueue)) {
+                        // this warp's share, moved to the bottom
+                        int2 keep[kSplitKeep];
+#pragma unroll
+                        for (int k = 0; k < kSplitKeep; ++k) {
+                            const int at = head + wt + S * (lane + 32 * k);
+                            keep[k] = at < ctop ? cst[at] : make_int2(kNull, 0);
+                        }
+                        __syncwarp();
+                        const int mine = (ctop - head - wt + S - 1) / S;
+#pragma unroll
+                        for (int k = 0; k < kSplitKeep; ++k)
+                            if (keep[k].x != kNull) cst[lane + 32 * k] = keep[k];
+                        ctop = max(mine, 0);
+                        spread = false;
+                        __syncwarp();
+                    }
+                    if (ctop == 0) break;
+                    const int k4 = min(4, spread ? ctop - head : ctop);
                     const int ci = lane >> 3;
                     int chk = kNull;
                     float sl = 1.0f;                    // 4^-level of the cell whose child this is
                     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (ci < k4) {
-                        const int2 e = cst[ctop - 1 - ci];
+                        const int2 e = cst[spread ? head + ci : ctop - 1 - ci];
                         sl = __int_as_float(e.y);
                         const size_t o8 = ((size_t)(e.x - nbody) << 3) + (lane & 7);
                         chk = __ldg(child + o8);
                         q = __ldg(kids4 + o8);
                     }
-                    ctop -= k4;
+                    if (spread) head += k4;
+                    else ctop -= k4;
                     __syncwarp();          // the popped entries are read before pushes reuse them
                     // children of a level-lv cell: t0 * 4^-lv + eps^2 (4^-lv exact)
                     bool acc = chk >= 0 && chk < nbody;
@@ -467,14 +539,21 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                             opn = !acc;
                         }
                     }
-                    const unsigned am = __ballot_sync(0xffffffffu, acc);
                     const unsigned om = __ballot_sync(0xffffffffu, opn);
                     const int on = __popc(om);
-                    opened += on;
-                    if (ctop + on > cap) {               // group-uniform
-                        walked = false;
-                        break;
+                    if (SPLIT && spread) {
+                        const unsigned every = __ballot_sync(0xffffffffu, acc);
+                        acc = acc && ((dealt + __popc(every & lt)) & (S - 1)) == wt;
+                        dealt += __popc(every);
+                        if (wt == 0) opened += on;
+                    } else {
+                        opened += on;
+                        if (ctop + on > cap) {           // group-uniform
+                            walked = false;
+                            break;
+                        }
                     }
+                    const unsigned am = __ballot_sync(0xffffffffu, acc);
                     if (acc) {
                         const int at = (lbase + lcnt + __popc(am & lt)) & (kListCap - 1);
                         lst[at] = q.x;
@@ -498,7 +577,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         lcnt -= 32;
                         lbase ^= 32;
                     }
-                    if (ctop == 0 && lcnt > 0) {
+                }
+                if (walked) {
+                    if (lcnt > 0) {
                         // the last records, filled up to a multiple of four with massless ones
                         if (lane < (-lcnt & 3)) {
                             const int at = lbase + lcnt + lane;
@@ -508,13 +589,8 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         __syncwarp();
                         for (int i = 0; i < lcnt; i += 4) eval4<BPL, FEAT>(lst + lbase, i, lb, eps22, ls);
                         accepted += lcnt;
-                        lcnt = 0;
                         __syncwarp();
                     }
-                }
-                if (walked) {
-                    ninter = accepted;
-                    visits = accepted + opened;
 #pragma unroll
                     for (int k = 0; k < BPL; ++k) {
                         ax[k] = __fadd_rn(ls[k].x.x, ls[k].x.y);
@@ -522,9 +598,40 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         az[k] = __fadd_rn(ls[k].z.x, ls[k].z.y);
                         if constexpr (FEAT) eb[k] = __fadd_rn(ls[k].e.x, ls[k].e.y);
                     }
+                }
+                if constexpr (SPLIT) {
+                    // the warps' sums through shared memory (each in its own list's place)
+                    float4* const out = reinterpret_cast<float4*>(lst);
+#pragma unroll
+                    for (int k = 0; k < BPL; ++k) out[32 * k + lane] = make_float4(ax[k], ay[k], az[k], eb[k]);
+                    if (lane == 0) team.accepted[wt] = walked ? accepted : -1, team.opened[wt] = opened;
+                    __syncthreads();
+                    if (wt != 0) continue;               // the first warp finishes the group
+                    for (int w = 1; w < S; ++w) {
+                        const float4* const from = reinterpret_cast<const float4*>(
+                            smem_raw + (size_t)w * list_group_bytes(max(cap, kSplitQueue)));
+                        if (team.accepted[w] < 0) walked = false;
+                        accepted += team.accepted[w];
+                        opened += team.opened[w];
+#pragma unroll
+                        for (int k = 0; k < BPL; ++k) {
+                            const float4 f = from[32 * k + lane];
+                            ax[k] = __fadd_rn(ax[k], f.x);
+                            ay[k] = __fadd_rn(ay[k], f.y);
+                            az[k] = __fadd_rn(az[k], f.z);
+                            if constexpr (FEAT) eb[k] = __fadd_rn(eb[k], f.w);
+                        }
+                    }
+                }
+                if (walked) {
+                    ninter = accepted;
+                    visits = accepted + opened;
                 } else {
 #pragma unroll
-                    for (int k = 0; k < BPL; ++k) pb[k].x = -lb[k].nx.x, pb[k].y = -lb[k].ny.x, pb[k].z = -lb[k].nz.x;
+                    for (int k = 0; k < BPL; ++k) {
+                        ax[k] = ay[k] = az[k] = eb[k] = 0.0f;
+                        pb[k].x = -lb[k].nx.x, pb[k].y = -lb[k].ny.x, pb[k].z = -lb[k].nz.x;
+                    }
                     __syncwarp();
                 }
             } else if (fast) {
@@ -728,6 +835,11 @@ __global__ void __launch_bounds__(kForceThreadsMax, LIST && !PB && !FEAT ? 4 : 3
     force_walk<64, false, PB, FEAT, LIST>(p);
 }
 
+template <int W, bool PB, bool FEAT>
+__global__ void __launch_bounds__(32 * kSplitMax) force_split_kernel(StepParams p) {
+    force_walk<W, false, PB, FEAT, true, true>(p);
+}
+
 template <int W, bool REF, bool PB, bool FEAT, bool LIST = false>
 static auto force_entry() {
     if constexpr (W == 64 && !REF) return force_kernel64<PB, FEAT, LIST>;
@@ -739,6 +851,15 @@ template <int W, bool REF, bool PB>
 static void launch_force_pf(const StepParams& p, bool feat, int grid, int threads, cudaStream_t s) {
     if constexpr (W >= 32 && !REF) {
         if (p.force_list) {
+            const int groups = W == 128 ? p.nitems128 : (W == 64 ? p.nitems64 : p.nwarps);
+            const int split = force_split(groups, p.sms);
+            if (split > 1) {
+                const int cap = p.stack_cap > kSplitQueue ? p.stack_cap : kSplitQueue;
+                const size_t sm = force_list_smem_bytes(32 * split, cap);
+                if (feat) force_split_kernel<W, PB, true><<<groups, 32 * split, sm, s>>>(p);
+                else force_split_kernel<W, PB, false><<<groups, 32 * split, sm, s>>>(p);
+                return;
+            }
             const size_t sm = force_list_smem_bytes(threads, p.stack_cap);
             if (feat) force_entry<W, false, PB, true, true>()<<<grid, threads, sm, s>>>(p);
             else force_entry<W, false, PB, false, true>()<<<grid, threads, sm, s>>>(p);
@@ -777,6 +898,11 @@ template <int W>
 static cudaError_t prep_list_w() {
     cudaError_t e = cudaSuccess, t;
     const int sm = (int)force_list_smem_bytes(kForceThreadsMax, kStackCapMax);
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if ((t = cudaFuncSetAttribute(force_split_kernel<W, false, false>, attr, sm)) != cudaSuccess) e = t;
+    if ((t = cudaFuncSetAttribute(force_split_kernel<W, false, true>, attr, sm)) != cudaSuccess) e = t;
+    if ((t = cudaFuncSetAttribute(force_split_kernel<W, true, false>, attr, sm)) != cudaSuccess) e = t;
+    if ((t = cudaFuncSetAttribute(force_split_kernel<W, true, true>, attr, sm)) != cudaSuccess) e = t;
     if ((t = cudaFuncSetAttribute(force_entry<W, false, false, false, true>(),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, sm)) != cudaSuccess)
         e = t;

@@ -737,3 +737,25 @@ def test_write_resumes_from_checkpoint():
     ra, rb = a.read(), b.read()
     for k in KEYS:
         np.testing.assert_array_equal(ra[k], rb[k])
+
+
+@pytest.mark.parametrize("vote,n,kw", [
+    (64, 1, {}), (64, 65, {}), (64, 1000, {}), (64, 60000, {}), (64, 110000, {}), (64, 190000, {}), (32, 33, {}),
+    (32, 40000, {}), (128, 300, {}), (128, 50000, {}), (64, 3000, {"stack_cap": 64, "theta": 0.15}),
+    (64, 3000, {"force_threads": 64})])
+def test_groups_shared_among_warps_match_the_oracle(vote, n, kw):
+    """Universes with fewer groups than the GPU has room for warps: 8, 4 and 2 warps per group,
+    groups of one body, a stack that overflows on some of the warps, and a launch geometry with
+    fewer threads than the warps of a group.  The tolerances of the other walks."""
+    arrs = plummer(n, seed=91)
+    theta = kw.get("theta", 0.5)
+    g = gpu_sim(**{"theta": theta, "eps": 0.05, "dt": 0.01, "vote_width": vote, **kw})
+    g.load(*arrs)
+    g.step(2)
+    o = oracle_for(n, theta=theta, eps=0.05, dt=0.01, vote=vote, fma=True)
+    o.load(*arrs)
+    o.step(2)
+    assert g.stats()["interactions"] == o.interactions
+    if n > 1:
+        rel, _ = acc_rel(g.read(), o.state())
+        assert rel.max() <= 1e-4, rel.max()
