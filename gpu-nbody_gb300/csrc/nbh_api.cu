@@ -52,7 +52,7 @@ struct nbh_sim {
     int force_threads = 128;       // force launch geometry (nbh_autotune)
     int stack_cap = 256;
     bool force_list = true;        // whole-warp FMA walks (vote width 32, 64, 128): the lane-parallel list walk
-    int build_phases = 5;          // octree insertion launches
+    int build_phases = 3;          // octree insertion launches
     bool build_buckets = true;     // lock phases insert a sample, the rest is built per slot
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
@@ -562,7 +562,7 @@ int nbh_create(const nbh_config* cfg_in, nbh_sim** out) {
     sim->device = cfg.device;
     sim->force_threads = threads;
     sim->stack_cap = cap;
-    sim->build_phases = cfg.build_phases ? cfg.build_phases : 5;
+    sim->build_phases = cfg.build_phases ? cfg.build_phases : 3;
     sim->build_buckets = cfg.build_buckets != 2;
     sim->top_phase = cfg.top_phase;
     // precise mode keeps the reference's order of accumulation (the per-visit walk) unless asked

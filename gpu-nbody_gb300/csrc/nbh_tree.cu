@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
 //
 // Bucket counters of a sampled-tree cell live in its kids4 block, which summarize
 // overwrites later in the step: ints 0..7 = bodies headed for slot j (zeroed when the cell
-// is made; the scatter counts them back to zero, so a second pass starts from zero too),
+// is made, and again when the allocation has read them, so a second pass starts from zero too),
 // 8..15 = first entry of slot j's bucket in the work list (written by the allocation for
 // every slot with bodies before the scatter reads it), 16..19 = the cell's centre and
 // half-width.
@@ -568,7 +568,8 @@ __device__ __forceinline__ int* bucket_counters(const StepParams& p, int c) {
 constexpr BuildPhase kBucketBodies = {1, 16};   // the bodies outside the 1/16 sample
 
 // (1) locate: read-only descent of each remaining body to its slot; the slot index goes
-// to parent[b] (scratch: the link pass writes the body's parent later).
+// to parent[b] and the body's place in the slot's bucket, from the counter, to sorted[b]
+// (scratch: the link and sort passes write both later).
 __global__ void __launch_bounds__(256) bucket_locate_kernel(StepParams p, BuildPhase set, bool reset_counters) {
     if (load_status(p.st)) return;
     if (reset_counters && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -608,7 +609,9 @@ __global__ void __launch_bounds__(256) bucket_locate_kernel(StepParams p, BuildP
     }
     p.parent[b] = ((node - nbody) << 3) | path;
     int* bc = bucket_counters(p, node);
-    if (atomicAdd(bc + path, 1) == 0) {
+    const int place = atomicAdd(bc + path, 1);
+    p.sorted[b] = place;
+    if (place == 0) {
         // the first body headed for a slot of `node` records the cell's centre and
         // half-width for the subtree builder (every descent computes the same values)
         reinterpret_cast<float4*>(bc)[4] = make_float4(cx, cy, cz, r);
@@ -663,6 +666,8 @@ __global__ void __launch_bounds__(256) bucket_alloc_kernel(StepParams p) {
         bb = __shfl_sync(0xffffffffu, bb, 31) + tb - nb;
         if (!valid || total == 0) continue;
         int* bcw = bucket_counters(p, c);
+        reinterpret_cast<int4*>(bcw)[0] = make_int4(0, 0, 0, 0);   // a second pass counts from zero
+        reinterpret_cast<int4*>(bcw)[1] = make_int4(0, 0, 0, 0);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (cnt[j] <= 0) continue;
@@ -673,7 +678,7 @@ __global__ void __launch_bounds__(256) bucket_alloc_kernel(StepParams p) {
     }
 }
 
-// (3) scatter: each remaining body takes an entry of its slot's bucket.
+// (3) scatter: each remaining body goes to its entry of its slot's bucket.
 __global__ void __launch_bounds__(256) bucket_scatter_kernel(StepParams p, BuildPhase set) {
     if (load_status(p.st)) return;
     const int per = phase_bodies(set);
@@ -683,20 +688,21 @@ __global__ void __launch_bounds__(256) bucket_scatter_kernel(StepParams p, Build
     const int b = ck.y + phase_offset(set, (int)(g % per), g / per);
     if (b >= ck.z) return;
     const int slot = p.parent[b];
-    int* bc = bucket_counters(p, p.nbody + (slot >> 3));
-    const int j = slot & 7;
-    p.bwork[bc[8 + j] + atomicSub(bc + j, 1) - 1] = b;
+    const int place = p.sorted[b];
+    p.bwork[bucket_counters(p, p.nbody + (slot >> 3))[8 + (slot & 7)] + place] = b;
 }
 
-// (4) build: one warp per bucket builds the bucket's subtree by splitting its bodies by
-// octant, level by level (depth first over a task stack), writing each new cell's 8 slots
-// once with their final values, then stores the subtree's root into the slot.  Subtrees of
-// at most 32 bodies are built in registers (one body per lane, octants grouped by
-// match_any).  A warp takes kBucketChunk buckets per work-counter atomic; a counting pass
-// sizes the register subtrees of the whole chunk so that one allocator atomic takes all
-// their cells, then the writing pass hands each subtree its share, parents first.  (Both
-// counters sit on one L2 slice: one atomic per bucket each was the kernel's limit.)  Larger
-// buckets split through the two halves of bwork until a part has at most 32 bodies.
+// (4) build: a warp takes consecutive buckets and builds the subtrees of as many as fit its
+// lanes (32 bodies) at once, one body per lane.  A body's path below its bucket's slot, eight
+// octants, makes a key with the bucket above and the lane below; the lanes sort the keys, and the
+// tree follows from the octants that neighbours share: body i opens one cell for each level it
+// shares with body i + 1 but not with body i - 1 (a cell exists for every octant prefix of two
+// or more bodies), all cells of the warp come from one atomic, parents first, and every cell and
+// body writes itself into its parent's slot.  About 300 instructions for 27 bodies on average;
+// splitting one bucket after another octant by octant, in two passes, took 186 us for the 1M
+// sphere.  Buckets in which two bodies share all eight octants go through the register splitter
+// (small_subtree), larger ones through the two halves of bwork until a part has at most 32
+// bodies.
 struct BucketTask {
     int cell, level, lo, hi, buf;
     float cx, cy, cz, r;       // centre and half-width of `cell`
@@ -714,7 +720,7 @@ constexpr int kBucketWarps = 4;
 constexpr int kBucketStack = 232;
 constexpr int kSmallStack = 48;
 constexpr int kBucketBlocksPerSm = 9;
-constexpr int kBucketChunk = 4;      // buckets a warp takes per work-counter atomic
+constexpr int kBucketChunk = 8;      // most buckets a warp takes per work-counter atomic
 
 // Stack position of each child cell among the nc cells pushed now: the largest deepest.
 __device__ __forceinline__ int deeper_rank(int mycnt, int lane) {
@@ -826,6 +832,180 @@ __device__ int build_small(const StepParams& p, const int* __restrict__ src, int
     return small_subtree(p, src, lo, m, cell, level, cx, cy, cz, r, st, local_max, true, base, zero_counts);
 }
 
+// A part to build, one per lane: m bodies from src[start] on, the subtree of slot j of cell c,
+// which has the centre and half-width g; lev: level of the subtree's root.
+struct Part {
+    int c, j, start, m, lev;
+    float4 g;
+};
+
+// Parts that fit the lanes together: how many, from lane `first` on (at most kBucketChunk lanes hold
+// one); incl: inclusive sum of their bodies.
+__device__ __forceinline__ int parts_that_fit(const Part& part, int first, int end, int& incl) {
+    const int lane = threadIdx.x & 31;
+    const bool mine = lane >= first && lane < end;
+    incl = mine ? min(part.m, 64) : 0;
+#pragma unroll
+    for (int o = 1; o < kBucketChunk; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    return __popc(__ballot_sync(0xffffffffu, mine && incl <= 32));
+}
+
+// The subtrees of the parts of lanes [first, first + cnt), at most 32 bodies in all.  Parts of
+// no bodies among them are passed over.  Whole-warp call; false after raising an error.
+__device__ bool packed_subtrees(const StepParams& p, const int* src_list, const Part& part, const int incl,
+                                const int first, const int cnt, SmallTask* sstack, int& local_max,
+                                bool zero_counts) {
+    constexpr int kLevels = 8;                       // octants in a key: 3 bits bucket, 24 path, 5 lane
+    const int lane = threadIdx.x & 31;
+    const int nbody = p.nbody;
+    const int total = __shfl_sync(0xffffffffu, incl, first + cnt - 1);
+    int seg = 0;
+    for (int k = 0; k < cnt; ++k) seg += lane >= __shfl_sync(0xffffffffu, incl, first + k);
+    if (total == 0) return true;
+    const bool active = lane < total;
+    const int from = first + min(seg, cnt - 1);
+    const int at = __shfl_sync(0xffffffffu, part.start - (incl - part.m), from) + lane;
+    const int c = __shfl_sync(0xffffffffu, part.c, from), j = __shfl_sync(0xffffffffu, part.j, from);
+    const int rootlev = __shfl_sync(0xffffffffu, part.lev, from);
+    const float4 g = make_float4(__shfl_sync(0xffffffffu, part.g.x, from), __shfl_sync(0xffffffffu, part.g.y, from),
+                                 __shfl_sync(0xffffffffu, part.g.z, from), __shfl_sync(0xffffffffu, part.g.w, from));
+    int b = 0;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) {
+        b = src_list[at];
+        q = p.node4[b];
+    }
+    unsigned key = 0xffffffffu;
+    {
+        float r = g.w * 0.5f;
+        float cx = __fadd_rn(__fsub_rn(g.x, r), (j & 1) ? g.w : 0.0f);
+        float cy = __fadd_rn(__fsub_rn(g.y, r), (j & 2) ? g.w : 0.0f);
+        float cz = __fadd_rn(__fsub_rn(g.z, r), (j & 4) ? g.w : 0.0f);
+        unsigned path = 0;
+#pragma unroll
+        for (int k = 0; k < kLevels; ++k) {
+            const int o = octant(cx, cy, cz, q.x, q.y, q.z);
+            path = (path << 3) | (unsigned)o;
+            const float h = r * 0.5f;
+            cx = __fadd_rn(__fsub_rn(cx, h), (o & 1) ? r : 0.0f);
+            cy = __fadd_rn(__fsub_rn(cy, h), (o & 2) ? r : 0.0f);
+            cz = __fadd_rn(__fsub_rn(cz, h), (o & 4) ? r : 0.0f);
+            r = h;
+        }
+        if (active) key = ((unsigned)seg << 29) | (path << 5) | (unsigned)lane;
+    }
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+        for (int o = k >> 1; o > 0; o >>= 1) {
+            const unsigned other = __shfl_xor_sync(0xffffffffu, key, o);
+            const bool low = ((lane & o) == 0) == ((lane & k) == 0);   // this lane keeps the smaller
+            key = low ? min(key, other) : max(key, other);
+        }
+    // octants shared with the neighbours, -1 across buckets
+    const unsigned before = __shfl_up_sync(0xffffffffu, key, 1), after = __shfl_down_sync(0xffffffffu, key, 1);
+    const unsigned path = (key >> 5) & 0xffffffu;
+    const unsigned xl = ((before ^ key) >> 5) & 0xffffffu, xr = ((after ^ key) >> 5) & 0xffffffu;
+    const bool inl = active && lane > 0 && (before >> 29) == (key >> 29);
+    const bool inr = lane + 1 < total && (after >> 29) == (key >> 29);
+    if (__any_sync(0xffffffffu, inl && xl == 0)) {
+        // two bodies share every octant of their keys: one bucket after another
+        for (int k = first; k < first + cnt; ++k) {
+            const int kc = __shfl_sync(0xffffffffu, part.c, k), kj = __shfl_sync(0xffffffffu, part.j, k);
+            const int lo = __shfl_sync(0xffffffffu, part.start, k), km = __shfl_sync(0xffffffffu, part.m, k);
+            const int lev = __shfl_sync(0xffffffffu, part.lev, k);
+            const float4 kg =
+                make_float4(__shfl_sync(0xffffffffu, part.g.x, k), __shfl_sync(0xffffffffu, part.g.y, k),
+                            __shfl_sync(0xffffffffu, part.g.z, k), __shfl_sync(0xffffffffu, part.g.w, k));
+            int root;
+            if (km == 0) continue;
+            if (km == 1) {
+                root = src_list[lo];
+                local_max = max(local_max, lev);
+            } else {
+                if (lev + 1 > kMaxDepth) {
+                    raise_error(p.st, NBH_ERR_DEPTH);
+                    return false;
+                }
+                const float h = kg.w * 0.5f;
+                root = build_small(p, src_list, lo, km, -1, lev,
+                                   __fadd_rn(__fsub_rn(kg.x, h), (kj & 1) ? kg.w : 0.0f),
+                                   __fadd_rn(__fsub_rn(kg.y, h), (kj & 2) ? kg.w : 0.0f),
+                                   __fadd_rn(__fsub_rn(kg.z, h), (kj & 4) ? kg.w : 0.0f), h, sstack, local_max,
+                                   zero_counts);
+                if (root < 0) return false;
+            }
+            if (lane == 0) cell_child(p, kc)[kj] = root;
+        }
+        return true;
+    }
+    const int cl = inl ? (__clz((int)xl) - 8) / 3 : -1;      // levels (root = 0) shared with body i - 1
+    const int cr = inr ? (__clz((int)xr) - 8) / 3 : -1;
+    const int made = max(0, cr - cl);                        // cells that start here: levels cl + 1 .. cr
+    // bucket and body of the sorted place
+    const int src = (int)(key & 31u);
+    const int sc = __shfl_sync(0xffffffffu, c, src), sj = __shfl_sync(0xffffffffu, j, src);
+    const int sb = __shfl_sync(0xffffffffu, b, src), slev = __shfl_sync(0xffffffffu, rootlev, src);
+    if (active) local_max = max(local_max, slev + max(cl, cr) + 1);
+    if (__any_sync(0xffffffffu, made > 0 && slev + cr >= kMaxDepth)) {
+        raise_error(p.st, NBH_ERR_DEPTH);
+        return false;
+    }
+    int off = made;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += v;
+    }
+    const int cells = __shfl_sync(0xffffffffu, off, 31);
+    int base = 0;
+    if (cells > 0) {
+        if (lane == 0) base = atomicSub(&p.st->bottom, cells);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base - cells <= nbody) {
+            raise_error(p.st, NBH_ERR_POOL);
+            return false;
+        }
+    }
+    // cell of this place at level l: org - l
+    const int org = base - 1 - (off - made) + cl + 1;
+    // the cell at level cl that contains body i starts at the last place before it that shares
+    // less than cl + 1 levels to its left
+    int begin = 0;
+#pragma unroll
+    for (int l = 0; l < kLevels; ++l) {
+        const unsigned less = __ballot_sync(0xffffffffu, cl < l);
+        if (l == cl) begin = 31 - __clz((int)(less & ((1u << lane) - 1u)));
+    }
+    const int outer = __shfl_sync(0xffffffffu, org, begin) - cl;
+    for (int i = lane; i < 2 * cells; i += 32)
+        reinterpret_cast<int4*>(cell_child(p, base - cells))[i] = make_int4(kNull, kNull, kNull, kNull);
+    for (int i = lane; i < cells; i += 32) {
+        p.arrive[base - cells - nbody + i] = 0;
+        if (zero_counts) {                                   // bucket counters for a pass into this tree
+            int4* bc = reinterpret_cast<int4*>(bucket_counters(p, base - cells + i));
+            bc[0] = make_int4(0, 0, 0, 0);
+            bc[1] = make_int4(0, 0, 0, 0);
+        }
+    }
+    __syncwarp();
+    for (int l = cl + 1; l <= cr; ++l) {
+        const int cell = org - l;
+        p.clevel[cell - nbody] = slev + l;
+        const int up = l == 0 ? sc : (l == cl + 1 ? outer : cell + 1);
+        cell_child(p, up)[l == 0 ? sj : (int)((path >> (3 * (kLevels - l))) & 7u)] = cell;
+    }
+    if (active) {
+        const int l = max(cl, cr);                           // level of the body's cell, -1: none made
+        const int up = l < 0 ? sc : (cr > cl ? org - cr : outer);
+        cell_child(p, up)[l < 0 ? sj : (int)((path >> (3 * (kLevels - 1 - l))) & 7u)] = sb;
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepParams p, bool zero_counts) {
     __shared__ SmallTask small_all[kBucketWarps][kSmallStack];
     if (load_status(p.st)) return;
@@ -836,80 +1016,48 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
     const unsigned lt = (1u << lane) - 1u;
     const int nbody = p.nbody;
     const int nb = ld_relaxed(&p.st->nbuckets);
+    // one atomic hands out a chunk of buckets: few of them while there are warps without any
+    const int chunk = max(1, min(kBucketChunk, nb / (int)(gridDim.x * kBucketWarps)));
     int local_max = 1;
     for (;;) {
-        // a chunk of buckets per warp: one atomic hands out kBucketChunk of them
         int item0 = 0;
-        if (lane == 0) item0 = atomicAdd(&p.st->bucket_next, kBucketChunk);
+        if (lane == 0) item0 = atomicAdd(&p.st->bucket_next, chunk);
         item0 = __shfl_sync(0xffffffffu, item0, 0);
         if (item0 >= nb) break;
-        const int nitem = min(kBucketChunk, nb - item0);
+        const int nitem = min(chunk, nb - item0);
         // lane l < nitem holds bucket item0 + l; the body its slot already held joins the
         // bucket's entries
-        int4 bkt = make_int4(0, 0, 0, kNull);
+        Part part = {};
         if (lane < nitem) {
-            bkt = p.buckets[item0 + lane];
+            const int4 bkt = p.buckets[item0 + lane];
             if (bkt.w >= 0) p.bwork[bkt.y + bkt.z] = bkt.w;
+            part.c = nbody + (bkt.x >> 3);
+            part.j = bkt.x & 7;
+            part.start = bkt.y;
+            part.m = bkt.z + (bkt.w >= 0 ? 1 : 0);
+            part.lev = p.clevel[part.c - nbody] + 1;
+            // cell c's centre and half-width, recorded by the locate pass
+            part.g = reinterpret_cast<const float4*>(bucket_counters(p, part.c))[4];
         }
         __syncwarp();
-        // (A) count the new cells of every bucket of 2..32 bodies, then take them for the whole
-        // chunk with one allocation: bucket l's cells lie below chunk_base minus the cells of
-        // the chunk's buckets before it
-        int need = 0;                                // lane l: cells of bucket l
-        for (int it = 0; it < nitem; ++it) {
-            const int bx = __shfl_sync(0xffffffffu, bkt.x, it), start = __shfl_sync(0xffffffffu, bkt.y, it);
-            const int m = __shfl_sync(0xffffffffu, bkt.z, it) + (__shfl_sync(0xffffffffu, bkt.w, it) >= 0 ? 1 : 0);
-            if (m < 2 || m > 32) continue;
-            const int c = nbody + (bx >> 3), j = bx & 7;
-            const float4 g = reinterpret_cast<const float4*>(bucket_counters(p, c))[4];
-            const int clev = p.clevel[c - nbody];
-            if (clev + 2 > kMaxDepth) {
-                raise_error(p.st, NBH_ERR_DEPTH);
-                return;
-            }
-            const float h0 = g.w * 0.5f;
-            const int cells = small_subtree(p, p.bwork, start, m, -1, clev + 1,
-                                            __fadd_rn(__fsub_rn(g.x, h0), (j & 1) ? g.w : 0.0f),
-                                            __fadd_rn(__fsub_rn(g.y, h0), (j & 2) ? g.w : 0.0f),
-                                            __fadd_rn(__fsub_rn(g.z, h0), (j & 4) ? g.w : 0.0f), h0, sstack,
-                                            local_max, false, 0, false);
-            if (cells < 0) return;
-            if (lane == it) need = cells;
-        }
-        int incl = need;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int chunk_base = 0;
-        if (total > 0) {
-            if (lane == 0) chunk_base = atomicSub(&p.st->bottom, total);
-            chunk_base = __shfl_sync(0xffffffffu, chunk_base, 0);
-            if (chunk_base - total <= nbody) {
-                raise_error(p.st, NBH_ERR_POOL);
-                return;
-            }
-        }
-        const int my_base = chunk_base - (incl - need);
-        // (B) build each bucket's subtree
-        for (int it = 0; it < nitem; ++it) {
-            const int bx = __shfl_sync(0xffffffffu, bkt.x, it);
-            const int c = nbody + (bx >> 3), j = bx & 7;
-            const int start = __shfl_sync(0xffffffffu, bkt.y, it);
-            const int m = __shfl_sync(0xffffffffu, bkt.z, it) + (__shfl_sync(0xffffffffu, bkt.w, it) >= 0 ? 1 : 0);
-            const int sub_base = __shfl_sync(0xffffffffu, my_base, it);
-            // cell c's centre and half-width, recorded by the locate pass
-            const float4 g = reinterpret_cast<const float4*>(bucket_counters(p, c))[4];
-            const int clev = p.clevel[c - nbody];
-            int* slot = cell_child(p, c) + j;
-            if (m == 1) {                                 // a single body: the slot takes it
-                if (lane == 0) *slot = p.bwork[start];
-                local_max = max(local_max, clev + 1);
+        for (int it = 0; it < nitem;) {
+            int incl;
+            const int cnt = parts_that_fit(part, it, nitem, incl);
+            if (cnt > 0) {
+                if (!packed_subtrees(p, p.bwork, part, incl, it, cnt, sstack, local_max, zero_counts)) return;
+                it += cnt;
                 continue;
             }
-            if (clev + 2 > kMaxDepth) {
+            // a bucket of more than 32 bodies
+            const int c = __shfl_sync(0xffffffffu, part.c, it), j = __shfl_sync(0xffffffffu, part.j, it);
+            const int start = __shfl_sync(0xffffffffu, part.start, it), m = __shfl_sync(0xffffffffu, part.m, it);
+            const int lev = __shfl_sync(0xffffffffu, part.lev, it);
+            const float4 g =
+                make_float4(__shfl_sync(0xffffffffu, part.g.x, it), __shfl_sync(0xffffffffu, part.g.y, it),
+                            __shfl_sync(0xffffffffu, part.g.z, it), __shfl_sync(0xffffffffu, part.g.w, it));
+            ++it;
+            int* slot = cell_child(p, c) + j;
+            if (lev + 1 > kMaxDepth) {
                 raise_error(p.st, NBH_ERR_DEPTH);
                 return;
             }
@@ -919,20 +1067,13 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
             const float rcy = __fadd_rn(__fsub_rn(g.y, h0), (j & 2) ? g.w : 0.0f);
             const float rcz = __fadd_rn(__fsub_rn(g.z, h0), (j & 4) ? g.w : 0.0f);
             int root;
-            if (m <= 32) {
-                root = small_subtree(p, p.bwork, start, m, -1, clev + 1, rcx, rcy, rcz, h0, sstack, local_max, true,
-                                     sub_base, zero_counts);
-                if (root < 0) return;
-                if (lane == 0) *slot = root;
-                continue;
-            }
             if (lane == 0) root = atomicSub(&p.st->bottom, 1) - 1;
             root = __shfl_sync(0xffffffffu, root, 0);
             if (root <= nbody) {
                 raise_error(p.st, NBH_ERR_POOL);
                 return;
             }
-            if (lane == 0) stack[0] = BucketTask{root, clev + 1, start, start + m, 0, rcx, rcy, rcz, h0};
+            if (lane == 0) stack[0] = BucketTask{root, lev, start, start + m, 0, rcx, rcy, rcz, h0};
             int top = 1;
             __syncwarp();
             bool ok = true;
@@ -941,14 +1082,6 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                 __syncwarp();
                 const int* src = p.bwork + (t.buf ? nbody : 0);
                 int* dst = p.bwork + (t.buf ? 0 : nbody);
-                if (t.hi - t.lo <= 32) {                  // small enough for the register builder
-                    if (build_small(p, src, t.lo, t.hi - t.lo, t.cell, t.level, t.cx, t.cy, t.cz, t.r, sstack,
-                                    local_max, zero_counts) < 0) {
-                        ok = false;
-                        break;
-                    }
-                    continue;
-                }
                 // pass 1: bodies per octant (lane o < 8 holds octant o's count)
                 int mycnt = 0;
                 for (int base = t.lo; base < t.hi; base += 32) {
@@ -994,8 +1127,9 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                     if (o >= 0) dst[t.lo + slot_base - __popc(mine) + __popc(mine & lt)] = b;
                 }
                 __syncwarp();
-                // children: empty, one body, or a cell (allocated together)
-                const bool is_cell = lane < 8 && mycnt >= 2;
+                // octants of more than 32 bodies become cells to split further; the others are built
+                // below, as many at a time as fit the lanes
+                const bool is_cell = lane < 8 && mycnt > 32;
                 const unsigned balc = __ballot_sync(0xffffffffu, is_cell);
                 const int nc = __popc(balc);
                 int cbase = 0;
@@ -1013,13 +1147,10 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                         break;
                     }
                 }
-                const int deeper = deeper_rank(mycnt, lane);
+                const int deeper = deeper_rank(is_cell ? mycnt : 0, lane);
                 if (lane < 8) {
                     int v = kNull;
-                    if (mycnt == 1) {
-                        v = dst[t.lo + myoff];
-                        local_max = max(local_max, t.level + 1);
-                    } else if (mycnt >= 2) {
+                    if (is_cell) {
                         v = cbase - 1 - __popc(balc & lt);
                         const float h = t.r * 0.5f;
                         stack[top + deeper] = BucketTask{v, t.level + 1, t.lo + myoff, t.lo + myoff + mycnt, t.buf ^ 1,
@@ -1035,6 +1166,16 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                 }
                 if (zero_counts && lane < 2)
                     reinterpret_cast<int4*>(p.kids4 + ((size_t)(t.cell - nbody) << 3))[lane] = make_int4(0, 0, 0, 0);
+                __syncwarp();                             // the slots are empty before they are filled
+                const Part small = {t.cell, lane, t.lo + myoff, lane < 8 && !is_cell ? mycnt : 0, t.level + 1,
+                                    make_float4(t.cx, t.cy, t.cz, t.r)};
+                for (int o = 0; o < 8 && ok;) {
+                    int incl;
+                    const int cnt = parts_that_fit(small, o, 8, incl);
+                    ok = packed_subtrees(p, dst, small, incl, o, cnt, sstack, local_max, zero_counts);
+                    o += cnt;
+                }
+                if (!ok) break;
                 top += nc;
                 __syncwarp();
             }

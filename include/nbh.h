@@ -91,7 +91,7 @@ typedef struct nbh_config {
                               levels take the per-level walk; in the list walk (force_list)
                               the cells whose children are pending, and a group that would
                               hold more restarts on the per-level walk */
-    int32_t build_phases;  /* octree insertion launches: 1 (one pass), 3 or 5 (0: 5) */
+    int32_t build_phases;  /* octree insertion launches: 1 (one pass), 3 or 5 (0: 3) */
     int32_t build_buckets; /* 1 (or 0, the default): with 5 phases the lock phases insert a
                               1/16 sample of the bodies and every other body joins the
                               subtree of the sample-tree slot it descends to, built by one
