@@ -54,6 +54,8 @@ struct nbh_sim {
     bool force_list = true;        // whole-warp FMA walks (vote width 32, 64, 128): the lane-parallel list walk
     int build_phases = 3;          // octree insertion launches
     bool build_buckets = true;     // lock phases insert a sample, the rest is built per slot
+    int max_bodies = 0;            // bodies of the largest universe
+    bool small_tree = false;       // all tree stages in one launch, one block per universe
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
     int top_cells = 0;             // cells of each block's shared tree for these universes
@@ -218,15 +220,20 @@ void ensure_item_order(nbh_sim* sim) {
     sim->order_vote = sim->cfg.vote_width;
 }
 
-// Enqueue the six stages of one step (GPUBarnesHutNBodySimulation.java:258-263).  With
-// `vel_acc_ready`, the stages from the angle features on (the first to read velocities or
-// accelerations) wait for that event and first pack the staged components `staged_mask`
-// (2 velocities, 4 accelerations) into the state; the tree stages need positions only.
-void enqueue_step(nbh_sim* sim, bool timed, cudaEvent_t vel_acc_ready = nullptr, int staged_mask = 0) {
-    const StepParams p = step_params(sim);
+// The tree stages, on the current positions.  The first of them advances the step counter (a
+// caller that is not taking a step restores it).  The one launch for small universes counts as
+// the build stage.
+void enqueue_tree(nbh_sim* sim, const StepParams& p, bool timed = false) {
     const bool ref = sim->cfg.arith == NBH_ARITH_REFERENCE;
     cudaStream_t s = sim->stream;
     if (timed) cudaEventRecord(sim->ev[0], s);
+    if (sim->small_tree) {
+        if (timed) cudaEventRecord(sim->ev[1], s);
+        launch_small_tree(p, ref, sim->max_bodies, s);
+        if (timed)
+            for (int k : {2, 3, 7}) cudaEventRecord(sim->ev[k], s);
+        return;
+    }
     launch_bbox(p, sim->grid_bbox, s);
     if (timed) cudaEventRecord(sim->ev[1], s);
     launch_build(p, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
@@ -237,6 +244,17 @@ void enqueue_step(nbh_sim* sim, bool timed, cudaEvent_t vel_acc_ready = nullptr,
     if (timed) cudaEventRecord(sim->ev[3], s);
     launch_sort(p, sim->grid_sort, s);
     if (timed) cudaEventRecord(sim->ev[7], s);
+}
+
+// Enqueue the six stages of one step (GPUBarnesHutNBodySimulation.java:258-263).  With
+// `vel_acc_ready`, the stages from the angle features on (the first to read velocities or
+// accelerations) wait for that event and first pack the staged components `staged_mask`
+// (2 velocities, 4 accelerations) into the state; the tree stages need positions only.
+void enqueue_step(nbh_sim* sim, bool timed, cudaEvent_t vel_acc_ready = nullptr, int staged_mask = 0) {
+    const StepParams p = step_params(sim);
+    const bool ref = sim->cfg.arith == NBH_ARITH_REFERENCE;
+    cudaStream_t s = sim->stream;
+    enqueue_tree(sim, p, timed);
     if (vel_acc_ready) {
         cudaStreamWaitEvent(s, vel_acc_ready, 0);
         launch_pack(sim->nbody, sim->staging, staged_mask, sim->node4, sim->vel, sim->acc,
@@ -258,19 +276,6 @@ void enqueue_step(nbh_sim* sim, bool timed, cudaEvent_t vel_acc_ready = nullptr,
     if (timed) cudaEventRecord(sim->ev[5], s);
     launch_integrate(p, ref, sim->grid_int, s);
     if (timed) cudaEventRecord(sim->ev[6], s);
-}
-
-// The tree stages alone (for probes and features on the current positions).  The bbox
-// stage advances the step counter; the caller restores it.
-void enqueue_tree(nbh_sim* sim, const StepParams& p) {
-    const bool ref = sim->cfg.arith == NBH_ARITH_REFERENCE;
-    cudaStream_t s = sim->stream;
-    launch_bbox(p, sim->grid_bbox, s);
-    launch_build(p, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
-                 sim->top_split, s);
-    launch_link(p, sim->grid_sum, s);
-    launch_summarize(p, ref, sim->grid_sum, s);
-    launch_sort(p, sim->grid_sort, s);
 }
 
 // Rebuild the tree of the current positions without advancing the step counter.
@@ -649,6 +654,11 @@ int nbh_load_batch(nbh_sim* sim, int32_t nuniv, const int32_t* counts, const flo
     // global first phase, eight blocks 2 % slower), eight for up to 8192 chunks (a 1M-body
     // sphere, 4096 chunks: 3 % faster; one block: even), the global locks above (a 4M-body
     // disc, 16384 chunks: 11-15 % slower in shared memory)
+    sim->max_bodies = 0;
+    for (int u = 0; u < nuniv; ++u) sim->max_bodies = std::max(sim->max_bodies, (int)counts[u]);
+    // one launch for small universes unless the configuration names a schedule
+    sim->small_tree = sim->max_bodies <= small_tree_max_bodies(nuniv) && sim->cfg.build_phases == 0 &&
+                      sim->cfg.build_buckets == 0 && sim->cfg.top_phase == 0;
     sim->top_possible = max_chunks <= top_build_max_samples();
     sim->top_cells = top_build_cells(max_chunks);
     if (!sim->top_possible || sim->top_phase == 2) sim->top_split = 0;
@@ -1355,25 +1365,32 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
     const int phases_before = sim->build_phases;
     const bool buckets_before = sim->build_buckets;
     const int top_before = sim->top_split;
+    const bool small_before = sim->small_tree;
     const bool top_ok = sim->top_phase != 2 && sim->top_possible;
     float best_tree = 1e30f;
     int best_ph = phases_before;
     bool best_bk = buckets_before;
     int best_top = top_before;
+    bool best_small = small_before;
     struct TreeCand {
         float ms;
         int phases;
         bool buckets;
         int top;
+        bool small;
         bool in_place;   // the schedule in place before
     };
     std::vector<TreeCand> tcands;
-    const int tree_c[13][3] = {{1, 0, 0}, {3, 0, 0}, {5, 0, 0}, {3, 1, 0}, {5, 1, 0},
-                               {3, 0, 1}, {5, 0, 1}, {3, 1, 1}, {5, 1, 1},
-                               {3, 0, 8}, {5, 0, 8}, {3, 1, 8}, {5, 1, 8}};
+    // (fourth column: one launch for small universes, where that is in place; reported as the
+    // three-phase bucketed schedule with one block per universe, which it would be otherwise)
+    const int tree_c[14][4] = {{1, 0, 0, 0}, {3, 0, 0, 0}, {5, 0, 0, 0}, {3, 1, 0, 0}, {5, 1, 0, 0},
+                               {3, 0, 1, 0}, {5, 0, 1, 0}, {3, 1, 1, 0}, {5, 1, 1, 0},
+                               {3, 0, 8, 0}, {5, 0, 8, 0}, {3, 1, 8, 0}, {5, 1, 8, 0}, {3, 1, 1, 1}};
     for (const auto& tc : tree_c) {
         if (err != cudaSuccess) break;
         if (tc[2] && !top_ok) continue;
+        if (tc[3] && !small_before) continue;
+        sim->small_tree = tc[3] != 0;
         sim->build_phases = tc[0];
         sim->build_buckets = tc[1] != 0;
         sim->top_split = tc[2];
@@ -1383,15 +1400,18 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
         err = timed([&] { enqueue_tree(sim, p); }, &ms);
         if (err != cudaSuccess) break;
         add_trial(1, tc[0], tc[1], tc[2], ms);
-        const bool before = tc[0] == phases_before && (tc[1] != 0) == (buckets_before && phases_before != 1) &&
-                            tc[2] == (phases_before != 1 ? top_before : 0);
-        tcands.push_back({ms, tc[0], tc[1] != 0, tc[2], before});
+        const bool before = (tc[3] != 0) == small_before &&
+                            (small_before || (tc[0] == phases_before &&
+                                              (tc[1] != 0) == (buckets_before && phases_before != 1) &&
+                                              tc[2] == (phases_before != 1 ? top_before : 0)));
+        tcands.push_back({ms, tc[0], tc[1] != 0, tc[2], tc[3] != 0, before});
         if (before) out->ms_tree_before = ms;
         if (ms < best_tree) {
             best_tree = ms;
             best_ph = tc[0];
             best_bk = tc[1] != 0;
             best_top = tc[2];
+            best_small = tc[3] != 0;
         }
     }
     if (err == cudaSuccess && tcands.size() > 1) {
@@ -1411,6 +1431,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
                 sim->build_phases = c.phases;
                 sim->build_buckets = c.buckets;
                 sim->top_split = c.top;
+                sim->small_tree = c.small;
                 StepParams p = step_params(sim);
                 p.theta_body = nullptr;
                 enqueue_tree(sim, p);
@@ -1425,6 +1446,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
             best_ph = tcands[k].phases;
             best_bk = tcands[k].buckets;
             best_top = tcands[k].top;
+            best_small = tcands[k].small;
         }
     }
     cudaEventDestroy(a);
@@ -1432,6 +1454,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
     sim->build_phases = phases_before;
     sim->build_buckets = buckets_before;
     sim->top_split = top_before;
+    sim->small_tree = small_before;
     if (err != cudaSuccess) return cuda_fail(sim, "nbh_autotune", err);
     CK(cudaMemcpyAsync(sim->h_state, sim->st, sizeof(DevState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1449,6 +1472,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
     sim->build_phases = best_ph;
     sim->build_buckets = best_bk;
     sim->top_split = best_top;
+    sim->small_tree = best_small;
     if ((e = set_geometry(sim))) return e;
     drop_graph(sim);
     out->force_threads = best_t;

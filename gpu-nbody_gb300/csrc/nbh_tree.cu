@@ -21,6 +21,22 @@ namespace nbh {
 // empty children, start = the universe's first sorted position; it resets bottom and the
 // per-step counters and increments the step counter (boundingbox.cl:170-195).
 template <bool PRECISE>
+__device__ __forceinline__ void root_box(const float (&mn)[3], const float (&mx)[3], float4& rc, float& radius) {
+    if constexpr (PRECISE) {
+        const double e = fmax(fmax((double)mx[0] - (double)mn[0], (double)mx[1] - (double)mn[1]),
+                              (double)mx[2] - (double)mn[2]);
+        rc = make_float4((float)(0.5 * ((double)mn[0] + (double)mx[0])), (float)(0.5 * ((double)mn[1] + (double)mx[1])),
+                         (float)(0.5 * ((double)mn[2] + (double)mx[2])), -1.0f);
+        radius = (float)(0.5 * e);
+    } else {
+        rc = make_float4(__fmul_rn(0.5f, __fadd_rn(mn[0], mx[0])), __fmul_rn(0.5f, __fadd_rn(mn[1], mx[1])),
+                         __fmul_rn(0.5f, __fadd_rn(mn[2], mx[2])), -1.0f);
+        radius = __fmul_rn(0.5f, fmaxf(fmaxf(__fsub_rn(mx[0], mn[0]), __fsub_rn(mx[1], mn[1])),
+                                       __fsub_rn(mx[2], mn[2])));
+    }
+}
+
+template <bool PRECISE>
 __global__ void __launch_bounds__(256) bbox_kernel(StepParams p) {
     if (load_status(p.st)) return;
     __shared__ float red[6][8];
@@ -88,24 +104,12 @@ __global__ void __launch_bounds__(256) bbox_kernel(StepParams p) {
             mn[k] = ord2f(atomicAdd(box + k, 0u));
             mx[k] = ord2f(atomicAdd(box + 3 + k, 0u));
         }
-        float cx, cy, cz, radius;
-        if constexpr (PRECISE) {
-            double e = fmax(fmax((double)mx[0] - (double)mn[0], (double)mx[1] - (double)mn[1]),
-                            (double)mx[2] - (double)mn[2]);
-            cx = (float)(0.5 * ((double)mn[0] + (double)mx[0]));
-            cy = (float)(0.5 * ((double)mn[1] + (double)mx[1]));
-            cz = (float)(0.5 * ((double)mn[2] + (double)mx[2]));
-            radius = (float)(0.5 * e);
-        } else {
-            cx = __fmul_rn(0.5f, __fadd_rn(mn[0], mx[0]));
-            cy = __fmul_rn(0.5f, __fadd_rn(mn[1], mx[1]));
-            cz = __fmul_rn(0.5f, __fadd_rn(mn[2], mx[2]));
-            radius = __fmul_rn(0.5f, fmaxf(fmaxf(__fsub_rn(mx[0], mn[0]), __fsub_rn(mx[1], mn[1])),
-                                           __fsub_rn(mx[2], mn[2])));
-        }
+        float4 rc;
+        float radius;
+        root_box<PRECISE>(mn, mx, rc, radius);
         const int root = p.nnodes - u;
         const int k = root - p.nbody;
-        p.node4[root] = make_float4(cx, cy, cz, -1.0f);
+        p.node4[root] = rc;
         int4* c4 = reinterpret_cast<int4*>(cell_child(p, root));
         c4[0] = make_int4(kNull, kNull, kNull, kNull);
         c4[1] = make_int4(kNull, kNull, kNull, kNull);
@@ -355,6 +359,90 @@ __device__ __forceinline__ unsigned short ld_shared_volatile(const unsigned shor
     return *reinterpret_cast<const volatile unsigned short*>(a);
 }
 
+// One sample's insertion into the shared tree; body_of(k): body of sample k.  Returns false once
+// the tree has failed (more cells than it holds or a split too deep: 1; a wait that gave up: 2).
+template <class BodyOf>
+__device__ __forceinline__ bool shared_insert(const StepParams& p, unsigned short* slots, unsigned char* lvl,
+                                              int* ncell, int* failed, int cap, int smp, const float4 bp,
+                                              const float4 rc, float radius, int& local_max, BodyOf body_of) {
+    int node = 0, depth = 1;
+    float r = radius, cx = rc.x, cy = rc.y, cz = rc.z;
+    int path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
+    unsigned short* slot = slots + node * 8 + path;
+    unsigned short ch = ld_shared_volatile(slot);
+    long long spins = 0;
+    for (;;) {
+        while (ch != kTopNull && ch != kTopLock && (ch & kTopCell)) {
+            if (depth >= kMaxDepth) {
+                atomicExch(failed, 1);
+                break;
+            }
+            node = ch & 0x7fff;
+            ++depth;
+            const float h = r * 0.5f;
+            cx = __fadd_rn(__fsub_rn(cx, h), (path & 1) ? r : 0.0f);
+            cy = __fadd_rn(__fsub_rn(cy, h), (path & 2) ? r : 0.0f);
+            cz = __fadd_rn(__fsub_rn(cz, h), (path & 4) ? r : 0.0f);
+            r = h;
+            path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
+            slot = slots + node * 8 + path;
+            ch = ld_shared_volatile(slot);
+        }
+        if (*reinterpret_cast<volatile int*>(failed)) return false;
+        if (ch == kTopLock) {                          // a split in progress: wait, bounded
+            if (++spins > kTopSpin) {
+                raise_error(p.st, NBH_ERR_TIMEOUT);
+                atomicExch(failed, 2);
+                return false;
+            }
+            __nanosleep(32);
+            ch = ld_shared_volatile(slot);
+            continue;
+        }
+        const unsigned short seen = atomicCAS(slot, ch, kTopLock);
+        if (seen != ch) {
+            ch = seen;
+            continue;
+        }
+        if (ch == kTopNull) {
+            *reinterpret_cast<volatile unsigned short*>(slot) = (unsigned short)smp;
+            local_max = max(local_max, depth);
+            return true;
+        }
+        // split: the slot held sample `ch`; cells until the two separate
+        const float4 op = p.node4[body_of((int)ch)];
+        int patch = -1, cur = node, cpath = path;
+        for (;;) {
+            ++depth;
+            const int cell = atomicAdd(ncell, 1);
+            if (depth > kMaxDepth || cell >= cap) {
+                atomicExch(failed, 1);
+                return false;
+            }
+            const float ox = (cpath & 1) ? r : 0.0f;
+            const float oy = (cpath & 2) ? r : 0.0f;
+            const float oz = (cpath & 4) ? r : 0.0f;
+            r *= 0.5f;
+            cx = __fadd_rn(__fsub_rn(cx, r), ox);
+            cy = __fadd_rn(__fsub_rn(cy, r), oy);
+            cz = __fadd_rn(__fsub_rn(cz, r), oz);
+            lvl[cell] = (unsigned char)(depth - 1);
+            if (patch < 0) patch = cell;
+            else slots[cur * 8 + cpath] = (unsigned short)(kTopCell | cell);
+            const int opath = octant(cx, cy, cz, op.x, op.y, op.z);
+            slots[cell * 8 + opath] = ch;
+            cur = cell;
+            cpath = octant(cx, cy, cz, bp.x, bp.y, bp.z);
+            if (cpath != opath) break;
+        }
+        slots[cur * 8 + cpath] = (unsigned short)smp;
+        __threadfence_block();                         // the new cells before their index
+        *reinterpret_cast<volatile unsigned short*>(slot) = (unsigned short)(kTopCell | patch);
+        local_max = max(local_max, depth);
+        return true;
+    }
+}
+
 __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bool zero_counts, int cap,
                                                                  int split) {
     extern __shared__ __align__(16) unsigned char top_smem[];
@@ -396,89 +484,12 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
             const int b = ck.y + phase_offset(kFirstPhase, 0, ci);
             if (b >= ck.z) continue;
             const float4 bp = p.node4[b];
-            int node = 0, depth = 1;
-            float r = radius, cx = rc.x, cy = rc.y, cz = rc.z;
-            int path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
-            if (oct >= 0 && path != oct) continue;     // another block's octant
-            unsigned short* slot = slots + node * 8 + path;
-            unsigned short ch = ld_shared_volatile(slot);
-            bool done = false;
-            long long spins = 0;
-            while (!done) {
-                while (ch != kTopNull && ch != kTopLock && (ch & kTopCell)) {
-                    if (depth >= kMaxDepth) {
-                        atomicExch(&failed, 1);
-                        break;
-                    }
-                    node = ch & 0x7fff;
-                    ++depth;
-                    const float h = r * 0.5f;
-                    cx = __fadd_rn(__fsub_rn(cx, h), (path & 1) ? r : 0.0f);
-                    cy = __fadd_rn(__fsub_rn(cy, h), (path & 2) ? r : 0.0f);
-                    cz = __fadd_rn(__fsub_rn(cz, h), (path & 4) ? r : 0.0f);
-                    r = h;
-                    path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
-                    slot = slots + node * 8 + path;
-                    ch = ld_shared_volatile(slot);
-                }
-                if (*reinterpret_cast<volatile int*>(&failed)) break;
-                if (ch == kTopLock) {                  // a split in progress: wait, bounded
-                    if (++spins > kTopSpin) {
-                        raise_error(p.st, NBH_ERR_TIMEOUT);
-                        atomicExch(&failed, 2);
-                        break;
-                    }
-                    __nanosleep(32);
-                    ch = ld_shared_volatile(slot);
-                    continue;
-                }
-                const unsigned short seen = atomicCAS(slot, ch, kTopLock);
-                if (seen != ch) {
-                    ch = seen;
-                    continue;
-                }
-                if (ch == kTopNull) {
-                    *reinterpret_cast<volatile unsigned short*>(slot) = (unsigned short)smp;
-                    local_max = max(local_max, depth);
-                    done = true;
-                    break;
-                }
-                // split: the slot held sample `ch`; cells until the two separate
-                const int4 ock = p.chunks[c0 + ch];
-                const float4 op = p.node4[ock.y + phase_offset(kFirstPhase, 0, c0 + ch)];
-                int patch = -1, cur = node, cpath = path;
-                bool ok = true;
-                for (;;) {
-                    ++depth;
-                    const int cell = atomicAdd(&ncell, 1);
-                    if (depth > kMaxDepth || cell >= cap) {
-                        atomicExch(&failed, 1);
-                        ok = false;
-                        break;
-                    }
-                    const float ox = (cpath & 1) ? r : 0.0f;
-                    const float oy = (cpath & 2) ? r : 0.0f;
-                    const float oz = (cpath & 4) ? r : 0.0f;
-                    r *= 0.5f;
-                    cx = __fadd_rn(__fsub_rn(cx, r), ox);
-                    cy = __fadd_rn(__fsub_rn(cy, r), oy);
-                    cz = __fadd_rn(__fsub_rn(cz, r), oz);
-                    lvl[cell] = (unsigned char)(depth - 1);
-                    if (patch < 0) patch = cell;
-                    else slots[cur * 8 + cpath] = (unsigned short)(kTopCell | cell);
-                    const int opath = octant(cx, cy, cz, op.x, op.y, op.z);
-                    slots[cell * 8 + opath] = ch;
-                    cur = cell;
-                    cpath = octant(cx, cy, cz, bp.x, bp.y, bp.z);
-                    if (cpath != opath) break;
-                }
-                if (!ok) break;
-                slots[cur * 8 + cpath] = (unsigned short)smp;
-                __threadfence_block();                 // the new cells before their index
-                *reinterpret_cast<volatile unsigned short*>(slot) = (unsigned short)(kTopCell | patch);
-                local_max = max(local_max, depth);
-                done = true;
-            }
+            if (oct >= 0 && octant(rc.x, rc.y, rc.z, bp.x, bp.y, bp.z) != oct) continue;   // another block's octant
+            auto body_of = [&](int k) {
+                const int4 ok = p.chunks[c0 + k];
+                return ok.y + phase_offset(kFirstPhase, 0, c0 + k);
+            };
+            if (!shared_insert(p, slots, lvl, &ncell, &failed, cap, smp, bp, rc, radius, local_max, body_of)) break;
         }
     }
     atomicMax(&depth_max, local_max);
@@ -1374,6 +1385,296 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 }
 
 // -------------------------------------------------------------------------------------
+// Small universes: bounding box, build, link, summarize and sort in one launch, one block per
+// universe, with the whole tree in shared memory.  The stages of a thousand-body step are a
+// dozen dependent launches whose work is a few microseconds of round trips each (measured at
+// 1,000 bodies: bounding box 8, build 76, link 4, summarize 38, sort 8 us); here the levels of
+// the tree are summed between block barriers instead of by arrivals through global memory.
+// The same arithmetic in the same order as the stages it replaces, so the same tree.
+//
+// Per cell of the shared tree: 8 slots, level, centre of mass, body count, offset in its
+// parent's range and parent.  A universe whose tree does not fit (close pairs make chains of
+// single-child cells) or goes too deep is left to the last block to finish, which builds such
+// universes one after another in global memory, through the lock insertion.
+// Measured, us, one launch / the stages: one sphere of 300 bodies 38 / 124, 1,000 52 / 132,
+// 3,000 97 / 140, 5,000 134 / 158, 7,168 175 / 156; 8 of 7,168 184 / 197, 200 of 1,000
+// 134 / 227, 200 of 7,168 404 / 503: up to 7,168 bodies (what shared memory holds) from 8
+// universes on, up to 5,120 for fewer.
+constexpr int kSmallBodies = 7168, kSmallBodiesFew = 5120;
+constexpr size_t kSmallCellBytes = 8 * sizeof(unsigned short) + sizeof(float4) + 3 * sizeof(unsigned short) + 1;
+int small_tree_max_bodies(int universes) { return universes >= 8 ? kSmallBodies : kSmallBodiesFew; }
+// Cells held for universes of at most `bodies` bodies (an octree of k bodies has about k / 2).
+static int small_tree_cells(int bodies) { return (bodies * 3 / 4 + 64) / 16 * 16; }
+static size_t small_tree_smem(int cells) { return (size_t)cells * kSmallCellBytes; }
+
+struct SmallShared {
+    int status, ncell, failed, depth_max, gbase, last;
+    float lo[3][32], hi[3][32];
+};
+
+// The per-step counters that the bounding box stage resets (the slots a later bounding box must
+// empty stay on record).
+__device__ __forceinline__ void begin_step(const StepParams& p) {
+    DevState* st = p.st;
+    st->pool_low = min(st->pool_low, st->bottom);
+    st->bottom = p.nnodes - p.nuniv + 1;
+    st->bbox_ticket = 0;
+    st->step += 1;
+    st->force_next = 0;
+    for (int j = 0; j < kDiagSlots; ++j) st->lock_waits[j] = st->cas_misses[j] = 0;
+    st->interactions = 0ull;
+}
+__global__ void begin_step_kernel(StepParams p) {
+    if (!load_status(p.st)) begin_step(p);
+}
+
+// One universe's tree in global memory, by the whole block: lock insertion, then link, summarize
+// and sort over its cells, which are the ones taken from the pool meanwhile.
+template <bool REF, bool PRECISE>
+__device__ void rescue_universe(const StepParams& p, int u, int* shared_bottom) {
+    const int nbody = p.nbody, root = p.nnodes - u;
+    if (threadIdx.x == 0) *shared_bottom = ld_relaxed(&p.st->bottom);
+    __syncthreads();
+    const int above = *shared_bottom;                  // cells of this universe: [below, above) and the root
+    __syncthreads();
+    // the slots of the free cells, which the insertion expects to be empty
+    for (long long i = 2 + threadIdx.x; i < 2ll * (above - nbody); i += blockDim.x)
+        reinterpret_cast<int4*>(p.child)[i] = make_int4(kNull, kNull, kNull, kNull);
+    if (threadIdx.x < 8) cell_child(p, root)[threadIdx.x] = kNull;
+    __threadfence();
+    __syncthreads();
+    int lm = 1, waits = 0, misses = 0;
+    for (int b = p.ubody[u] + (int)threadIdx.x; b < p.ubody[u + 1]; b += blockDim.x)
+        if (!lock_insert(p, b, u, false, lm, waits, misses)) break;
+    atomicMax(&p.st->max_depth, lm);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) *shared_bottom = load_status(p.st) ? -1 : ld_relaxed(&p.st->bottom);
+    __syncthreads();
+    const int below = *shared_bottom;
+    __syncthreads();
+    if (below < 0) return;
+    const int cells = above - below + 1;               // the root last
+    for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+        const int c = i == cells - 1 ? root : below + i;
+        for (int j = 0; j < 8; ++j) {
+            const int ch = __ldcg(cell_child(p, c) + j);
+            if (ch >= 0) p.parent[ch] = c;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    for (int level = kMaxDepth - 1; level >= 0; --level) {
+        for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+            const int c = i == cells - 1 ? root : below + i;
+            if (__ldcg(p.clevel + (c - nbody)) != level) continue;
+            int sl[8];
+            int* ch8 = cell_child(p, c);
+            for (int j = 0; j < 8; ++j) sl[j] = __ldcg(ch8 + j);
+            p.node4[c] = (PRECISE && c == root) ? sum_children<REF, true>(p, c, sl, ch8)
+                                                : sum_children<REF, false>(p, c, sl, ch8);
+        }
+        __threadfence();
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+        const int c = i == cells - 1 ? root : below + i;
+        int s = p.ubody[u];
+        for (int x = c; x != root; x = __ldcg(p.parent + x)) s += __ldcg(p.loff + (x - nbody));
+        p.start[c - nbody] = s;
+        for (int j = 0; j < 8; ++j) {
+            const int ch = __ldcg(cell_child(p, c) + j);
+            if (ch >= nbody) s += __ldcg(p.count + (ch - nbody));
+            else if (ch >= 0) p.sorted[s++] = ch;
+        }
+    }
+    __syncthreads();
+}
+
+template <bool REF, bool PRECISE>
+__global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, int cap) {
+    extern __shared__ __align__(16) unsigned char top_smem[];
+    float4* const com = reinterpret_cast<float4*>(top_smem);
+    unsigned short* const slots = reinterpret_cast<unsigned short*>(com + cap);      // [cap][8]
+    unsigned short* const count = slots + (size_t)cap * 8;
+    unsigned short* const off = count + cap;
+    unsigned short* const par = off + cap;
+    unsigned char* const lvl = reinterpret_cast<unsigned char*>(par + cap);
+    __shared__ SmallShared S;
+    const int u = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
+    const int nbody = p.nbody, root = p.nnodes - u;
+    const int first = p.ubody[u], n = p.ubody[u + 1] - first;
+    if (tid == 0) {
+        S.status = load_status(p.st);
+        if (!S.status && p.nuniv == 1) begin_step(p);
+        S.ncell = 1;                                   // local cell 0 is the root
+        S.failed = 0;
+        S.depth_max = 1;
+        lvl[0] = 0;
+    }
+    for (int i = tid; i < cap * 4; i += blockDim.x) reinterpret_cast<unsigned*>(slots)[i] = 0xffffffffu;
+    // bounding box (see bbox_kernel)
+    float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+    for (int i = tid; i < n; i += blockDim.x) {
+        const float4 q = p.node4[first + i];
+        v[0] = fminf(v[0], q.x); v[1] = fminf(v[1], q.y); v[2] = fminf(v[2], q.z);
+        v[3] = fmaxf(v[3], q.x); v[4] = fmaxf(v[4], q.y); v[5] = fmaxf(v[5], q.z);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+            v[3 + k] = fmaxf(v[3 + k], __shfl_xor_sync(0xffffffffu, v[3 + k], o));
+        }
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) S.lo[k][wid] = v[k], S.hi[k][wid] = v[3 + k];
+    __syncthreads();
+    if (S.status) return;
+    float mn[3], mx[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        mn[k] = S.lo[k][0], mx[k] = S.hi[k][0];
+        for (int w = 1; w < warps; ++w) mn[k] = fminf(mn[k], S.lo[k][w]), mx[k] = fmaxf(mx[k], S.hi[k][w]);
+    }
+    float4 rc;
+    float radius;
+    root_box<PRECISE>(mn, mx, rc, radius);
+    if (tid == 0) {
+        p.node4[root] = rc;
+        p.uradius[u] = radius;
+        p.parent[root] = -1;
+        p.arrive[root - nbody] = 0;
+        p.clevel[root - nbody] = 0;
+    }
+    int local_max = 1;
+    for (int k = tid; k < n; k += blockDim.x)
+        if (!shared_insert(p, slots, lvl, &S.ncell, &S.failed, cap, k, p.node4[first + k], rc, radius, local_max,
+                           [&](int o) { return first + o; }))
+            break;
+    atomicMax(&S.depth_max, local_max);
+    __syncthreads();
+    const int nc = S.ncell;
+    if (tid == 0 && !S.failed) {
+        // local cell c (c >= 1) becomes pool cell gbase - c
+        S.gbase = nc > 1 ? atomicSub(&p.st->bottom, nc - 1) : 0;
+        if (nc > 1 && S.gbase - (nc - 1) <= nbody) {
+            raise_error(p.st, NBH_ERR_POOL);
+            S.failed = 2;
+        } else if (S.depth_max > ld_relaxed(&p.st->max_depth)) {
+            atomicMax(&p.st->max_depth, S.depth_max);
+        }
+    }
+    __syncthreads();
+    if (!S.failed) {
+        const int gb = S.gbase;
+        // summarize, deepest level first (see sum_children), and link
+        for (int level = S.depth_max - 1; level >= 0; --level) {
+            for (int c = tid; c < nc; c += blockDim.x) {
+                if (lvl[c] != level) continue;
+                const int gc = c == 0 ? root : gb - c, k = gc - nbody;
+                const uint4 packed = reinterpret_cast<const uint4*>(slots)[c];
+                const unsigned w[4] = {packed.x, packed.y, packed.z, packed.w};
+                float4* const kb = p.kids4 + ((size_t)k << 3);
+                int* const ch8 = cell_child(p, gc);
+                int used = 0, cnt = 0;
+                float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
+                double dm = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const unsigned short v16 = (unsigned short)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu);
+                    if (v16 == kTopNull) continue;
+                    int g;
+                    float4 q;
+                    if (v16 & kTopCell) {
+                        const int l = v16 & 0x7fff;
+                        g = gb - l;
+                        q = com[l];
+                        off[l] = (unsigned short)cnt;
+                        par[l] = (unsigned short)c;
+                        p.loff[g - nbody] = cnt;
+                        cnt += count[l];
+                    } else {
+                        g = first + v16;
+                        q = p.node4[g];
+                        ++cnt;
+                    }
+                    p.parent[g] = gc;
+                    if (PRECISE && c == 0) {
+                        dm += (double)q.w;
+                        dx += (double)q.x * (double)q.w;
+                        dy += (double)q.y * (double)q.w;
+                        dz += (double)q.z * (double)q.w;
+                    } else {
+                        cm = __fadd_rn(cm, q.w);
+                        sx = madd<REF>(q.x, q.w, sx);
+                        sy = madd<REF>(q.y, q.w, sy);
+                        sz = madd<REF>(q.z, q.w, sz);
+                    }
+                    slots[c * 8 + used] = v16;
+                    ch8[used] = g;
+                    kb[used] = q;
+                    ++used;
+                }
+                for (int j = used; j < 8; ++j) {
+                    slots[c * 8 + j] = kTopNull;
+                    ch8[j] = kNull;
+                    kb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                float4 centre;
+                if (PRECISE && c == 0) {
+                    centre = make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
+                } else {
+                    const float inv = __fdiv_rn(1.0f, cm);
+                    centre = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
+                }
+                com[c] = centre;
+                count[c] = (unsigned short)cnt;
+                p.node4[gc] = centre;
+                p.count[k] = cnt;
+                p.clevel[k] = level;
+            }
+            __syncthreads();
+        }
+        // sort (see sort_kernel)
+        for (int c = tid; c < nc; c += blockDim.x) {
+            int s = first;
+            for (int x = c; x != 0; x = par[x]) s += off[x];
+            p.start[(c == 0 ? root : gb - c) - nbody] = s;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const unsigned short v16 = slots[c * 8 + j];
+                if (v16 == kTopNull) continue;
+                if (v16 & kTopCell) s += count[v16 & 0x7fff];
+                else p.sorted[s++] = first + v16;
+            }
+        }
+    } else if (tid == 0) {
+        p.start[root - nbody] = -1;                    // for the last block (a wait that gave up or an
+                                                       // empty pool have set the status)
+    }
+    // the last block to finish builds what did not fit
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) S.last = S.failed || p.nuniv > 1 ? atomicAdd(&p.st->bbox_ticket, 1) == p.nuniv - 1 : 0;
+    __syncthreads();
+    if (!S.last) return;
+    __threadfence();
+    if (tid == 0) p.st->bbox_ticket = 0;
+    for (int w = 0; w < p.nuniv; ++w) {
+        if (__ldcg(p.start + (p.nnodes - w - nbody)) != -1) continue;
+        if (tid == 0) S.status = load_status(p.st);
+        __syncthreads();
+        const int status = S.status;
+        __syncthreads();
+        if (status) return;
+        rescue_universe<REF, PRECISE>(p, w, &S.gbase);
+    }
+}
+
+// -------------------------------------------------------------------------------------
 void launch_bbox(const StepParams& p, int grid, cudaStream_t s) {
     if (p.precise) bbox_kernel<true><<<grid, 256, 0, s>>>(p);
     else bbox_kernel<false><<<grid, 256, 0, s>>>(p);
@@ -1428,7 +1729,32 @@ void launch_build(const StepParams& p, int phases, bool buckets, int sms, int to
     if (buckets) launch_bucket_pass(p, kBucketBodies, true, false, sms, s);
 }
 
+template <bool REF, bool PRECISE>
+static void launch_small_t(const StepParams& p, int max_bodies, cudaStream_t s) {
+    const int cells = small_tree_cells(max_bodies);
+    int threads = 128;
+    while (threads < max_bodies && threads < kTopThreads) threads *= 2;
+    small_tree_kernel<REF, PRECISE><<<p.nuniv, threads, small_tree_smem(cells), s>>>(p, cells);
+}
+void launch_small_tree(const StepParams& p, bool ref, int max_bodies, cudaStream_t s) {
+    if (p.nuniv > 1) begin_step_kernel<<<1, 1, 0, s>>>(p);
+    if (ref) {
+        if (p.precise) launch_small_t<true, true>(p, max_bodies, s);
+        else launch_small_t<true, false>(p, max_bodies, s);
+    } else {
+        if (p.precise) launch_small_t<false, true>(p, max_bodies, s);
+        else launch_small_t<false, false>(p, max_bodies, s);
+    }
+}
+
 cudaError_t prepare_tree_kernels() {
+    const int sm = (int)small_tree_smem(small_tree_cells(kSmallBodies));
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(small_tree_kernel<false, false>, attr, sm)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(small_tree_kernel<false, true>, attr, sm)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(small_tree_kernel<true, false>, attr, sm)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(small_tree_kernel<true, true>, attr, sm)) != cudaSuccess) return e;
     return cudaFuncSetAttribute(top_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)top_build_smem(kTopCells));
 }

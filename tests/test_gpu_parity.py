@@ -759,3 +759,125 @@ def test_groups_shared_among_warps_match_the_oracle(vote, n, kw):
     if n > 1:
         rel, _ = acc_rel(g.read(), o.state())
         assert rel.max() <= 1e-4, rel.max()
+
+
+def _close_pairs(n, pairs, seed):
+    """n bodies in a cube, the first 2 * pairs of them in pairs 1e-6 apart: each pair makes a chain
+    of single-child cells."""
+    r = np.random.default_rng(seed)
+    pos = r.uniform(-1, 1, (n, 3)).astype(np.float32)
+    pos[1:2 * pairs:2] = pos[0:2 * pairs:2] + np.float32(1e-6) * np.array([1.0, 0.7, 0.3], np.float32)
+    zero = np.zeros(n, np.float32)
+    return (pos[:, 0].copy(), pos[:, 1].copy(), pos[:, 2].copy(), zero, zero, zero, np.full(n, 1.0 / n, np.float32))
+
+
+def _steps(kw, load, steps=3):
+    g = gpu_sim(eps=0.05, dt=0.01, **kw)
+    load(g)
+    g.step(steps)
+    out = g.read(), g.tree(), g.stats()
+    g.close()
+    return out
+
+
+def _assert_same_steps(a, b):
+    for k in KEYS:
+        np.testing.assert_array_equal(a[0][k], b[0][k], err_msg=k)
+    np.testing.assert_array_equal(a[1]["sorted"], b[1]["sorted"])
+    np.testing.assert_array_equal(a[1]["radius"], b[1]["radius"])
+    n = a[1]["nbody"]
+    for r in a[1]["roots"]:                          # roots: same record, count and first position
+        for key in ("count", "start"):
+            assert a[1][key][r - n] == b[1][key][r - n]
+        np.testing.assert_array_equal(a[1]["node4"][r], b[1]["node4"][r])
+    for key in ("cells", "max_depth", "interactions", "status"):
+        assert a[2][key] == b[2][key], key
+    # every cell's range, whatever its index
+    for key in ("count", "start"):
+        pa, pb = (np.sort(t[1][key][t[1]["bottom"] - n:]) for t in (a, b))
+        np.testing.assert_array_equal(pa, pb)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 129, 1000, 4097, 5120, 5121])
+@pytest.mark.parametrize("mode", ["fma", "reference", "precise"])
+def test_one_launch_tree_equals_the_staged_one(n, mode):
+    """Small universes build their tree in one launch: the staged kernels' tree, body for body and
+    bit for bit, at the edges of its range (5,121 bodies take the stages either way)."""
+    import nbh
+    kw = {"fma": {"theta": 0.5}, "reference": {"theta2": 1.5, "vote_width": 16, "arith": nbh.NBH_ARITH_REFERENCE},
+          "precise": {"theta": 0.5, "precise": True}}[mode]
+    arrs = plummer(n, seed=92)
+    a = _steps(kw, lambda g: g.load(*arrs))
+    _assert_same_steps(a, _steps({**kw, "build_phases": 3}, lambda g: g.load(*arrs)))
+    if n == 1000 and mode == "fma":
+        g = gpu_sim(theta=0.5, eps=0.05, dt=0.01)
+        g.load(*arrs)
+        g.step()
+        o = oracle_for(n, theta=0.5, eps=0.05, dt=0.01, vote=64, fma=True)
+        o.load(*arrs)
+        o.step()
+        t = g.tree()
+        assert assert_same_tree(t, o.tree_arrays(), n, t["nnodes"], o.nn) == t["nnodes"] + 1 - t["bottom"]
+
+
+def test_one_launch_tree_of_many_universes():
+    """Eight universes of up to 7,168 bodies, the most that shared memory holds."""
+    counts = [7168, 1, 2, 900, 5121, 33, 7000, 2500]
+    parts = [plummer(c, seed=80 + i) for i, c in enumerate(counts)]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    load = lambda g: g.load_batch(counts, *cat)      # noqa: E731
+    _assert_same_steps(_steps({"theta": 0.5}, load), _steps({"theta": 0.5, "build_phases": 3}, load))
+
+
+@pytest.mark.parametrize("universes", [1, 4])
+def test_one_launch_tree_hands_over_what_does_not_fit(universes):
+    """Chains of single-child cells between close pairs need more cells than shared memory holds;
+    those universes are built in global memory by the last block, the others are not touched."""
+    parts = [_close_pairs(2000, 300, 93)]
+    if universes > 1:
+        parts = [plummer(700, seed=94), parts[0], plummer(1, seed=95), _close_pairs(3000, 400, 96)]
+    counts = [p[0].size for p in parts]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    load = lambda g: g.load_batch(counts, *cat)      # noqa: E731
+    kw = {"theta": 0.5, "pool_factor": 4.0}          # room for the chains
+    _assert_same_steps(_steps(kw, load), _steps({**kw, "build_phases": 1}, load))
+
+
+def test_one_launch_tree_and_staged_tree_in_turn():
+    """The tuner may move a small universe from the one launch to the stages between steps."""
+    n = 3000
+    arrs = plummer(n, seed=97)
+    a, b = gpu_sim(theta=0.5, eps=0.05, dt=0.01), gpu_sim(theta=0.5, eps=0.05, dt=0.01, build_phases=1)
+    for g in (a, b):
+        g.load(*arrs)
+        g.step(2)
+    a.autotune()
+    for g in (a, b):
+        g.step(2)
+    sa, sb = a.read(), b.read()
+    for k in KEYS:
+        np.testing.assert_array_equal(sa[k], sb[k])
+    a.load(*plummer(500, seed=98))
+    a.step(2)
+    assert a.stats()["status"] == 0
+
+
+def test_one_launch_tree_reports_errors_and_recovers():
+    import nbh
+    from nbh import _lib as L
+    arrs = [v.copy() for v in plummer(500, seed=99)]
+    for k in range(3):
+        arrs[k][7] = arrs[k][11]                     # two bodies at one point never separate
+    g = gpu_sim()
+    g.load(*arrs)
+    with pytest.raises(nbh.NbhError) as ei:
+        g.step()
+    assert ei.value.code == L.NBH_ERR_DEPTH
+    g.load(*plummer(500, seed=99))
+    g.step(2)
+    assert g.stats()["status"] == 0
+    h = gpu_sim(pool_factor=0.5)                     # 16,384 nodes for 3,000 bodies with long chains
+    h.load(*_close_pairs(3000, 1500, 90))
+    with pytest.raises(nbh.NbhError) as ei:
+        h.step()
+    assert ei.value.code == L.NBH_ERR_POOL
