@@ -5,32 +5,18 @@
 namespace nbh {
 
 // Launch geometry is chosen at run time (nbh_autotune): threads per block (64 / 128 / 256)
-// and the entries of each group's shared-memory stack of pending children, each with its
-// preloaded node record.  Opening a cell at level l while every ancestor still has 7
-// pending children needs 7*l + 8 entries, so a stack of `cap` entries covers trees up to
-// fast_max_depth(cap) levels; deeper trees take the per-level (cell, next child) walk.
+// and the entries of each group's shared-memory stack.  A group whose stack would overflow
+// restarts on the per-level (cell, next child) walk.
 constexpr int kForceThreadsMax = 256;
 constexpr int kStackCapMax = 256;
 constexpr int kStackCapMin = 64;     // the deep walk keeps 2 * kMaxDepth ints in the same space
-__host__ __device__ constexpr int fast_max_depth(int cap) { return (cap - 8) / 7 + 1; }
-
-// Lanes of one vote group: W bodies on W lanes for W <= 32; W = 64 puts two bodies on
-// each lane of one warp.
-template <int W>
-__host__ __device__ constexpr int group_lanes() {
-    return W < 32 ? W : 32;
-}
-
-template <int W>
-constexpr size_t force_smem_bytes(int threads, int cap) {
-    return (size_t)(threads / group_lanes<W>()) * cap * (sizeof(float4) + sizeof(int2));
-}
 
 // The list walk (64-wide groups): per group, the records of accepted nodes awaiting
 // evaluation (at most 31 wait after an evaluation and one round adds at most 32; separate
 // arrays of x, y, z, m) with each record's full cell width^2 (for the error bound; 0 for a
-// body), the undecided cells of a round (at most 32, likewise as arrays), and a stack of `cap` cells whose children are still to be tested,
-// with their levels (a 64-entry stack also holds the per-level walk's 2 * kMaxDepth ints).
+// body), the undecided cells of a round (at most 32, likewise as arrays), the group's box and
+// representatives, and a stack of `cap` cells whose children are still to be tested, with their
+// level factors (a 64-entry stack also holds the per-level walk's 2 * kMaxDepth ints).
 constexpr int kListCap = 64;
 constexpr size_t list_group_bytes(int cap) {
     return kListCap * (sizeof(float4) + sizeof(float)) + 32 * sizeof(float4) + 4 * sizeof(float4) +
@@ -60,6 +46,21 @@ static int force_split(int groups, int sms) {
 }
 static_assert(kStackCapMin * sizeof(int2) >= 2 * kMaxDepth * sizeof(int), "the per-level walk fits the cell stack");
 
+// The ordered walk: per group, a stack of pending nodes (24 bytes for each of the `cap` entries
+// asked for, at 16 bytes each), with their widths^2 factors where error bounds are recorded,
+// the list of accepted records (each twice over where a lane has two or more bodies) with their
+// widths^2, the undecided cells of a round, and the group's box and representatives.
+__host__ __device__ constexpr int ordered_entries(int cap) { return cap + cap / 2; }
+template <int W>
+constexpr size_t force_smem_bytes(int threads, int cap, bool feat) {
+    return (size_t)(threads / 32) * ((size_t)ordered_entries(cap) * (sizeof(float4) + (feat ? sizeof(float) : 0)) +
+                                     kListCap * ((W >= 64 ? 2 : 1) * sizeof(float4) + sizeof(float)) +
+                                     32 * sizeof(float4) + 4 * sizeof(float4));
+}
+// Free entries below which the ordered walk opens one cell a round instead of four (4M disc: 32
+// and 80 the same at 256 entries asked for, 12073 and 12750 us at 192).
+constexpr int kOrderedSlack = 32;
+
 // Opening threshold of tree level L (root = 0): r^2/theta^2 * 4^-L + eps^2
 // (calculateforce.cl:52-67).  The walk carries s = 4^-L (exact powers of two) and forms
 // t0*s + eps^2, which equals ldexp(t0, -2L) + eps^2 in the normal range; below it eps^2
@@ -84,7 +85,7 @@ __device__ __forceinline__ void interact(const float4 q, const float dx, const f
                                          const float d2, float& ax, float& ay, float& az, float& eb,
                                          const float s2) {
     float rd;
-    if constexpr (REF) rd = __fdiv_rn(1.0f, __fsqrt_rn(d2));
+    if constexpr (REF) rd = __frcp_rn(__fsqrt_rn(d2));
     else rd = rsqrt_ftz(d2);
     const float f = __fmul_rn(__fmul_rn(__fmul_rn(q.w, rd), rd), rd);
     ax = madd<REF>(dx, f, ax);
@@ -151,28 +152,95 @@ __device__ __forceinline__ void eval4(const float* lst, const int at, const List
                         make_float2(S.z, S.w), b[k], eps2, a[k]);
 }
 
+// The ordered walk's arithmetic: `cnt` records of the list from `at` on, each body's sums
+// formed in list order.  Two or more bodies per lane (FMA arithmetic): FP32x2 over pairs of bodies,
+// the records stored twice over as (x, x, y, y) and (z, z, m, m).  One body per lane: scalar.  16
+// bodies on the warp's 32 lanes: the half-warps take one of two consecutive records each, and the
+// lower half, which holds the sums, adds its own record's terms and then the other's.
+template <int W, bool REF, bool FEAT>
+__device__ __forceinline__ void eval_ordered(const float4* lst, const float* lw, const int at, const int cnt,
+                                             const float4 (&pb)[W < 32 ? 1 : W / 32], const float eps2,
+                                             float (&ax)[W < 32 ? 1 : W / 32], float (&ay)[W < 32 ? 1 : W / 32],
+                                             float (&az)[W < 32 ? 1 : W / 32], float (&eb)[W < 32 ? 1 : W / 32]) {
+    if constexpr (W >= 64) {
+        static_assert(!REF, "two bodies per lane take FMA arithmetic");
+        const float2 e2 = make_float2(eps2, eps2);
+#pragma unroll 8
+        for (int i = at; i < at + cnt; ++i) {
+            const float4 xy = lst[2 * i], zm = lst[2 * i + 1];
+            const float s2 = FEAT ? lw[i] : 0.0f;
+#pragma unroll
+            for (int k = 0; k < W / 32; k += 2) {
+                const ListBody b = {make_float2(-pb[k].x, -pb[k + 1].x), make_float2(-pb[k].y, -pb[k + 1].y),
+                                    make_float2(-pb[k].z, -pb[k + 1].z)};
+                ListSum a = {make_float2(ax[k], ax[k + 1]), make_float2(ay[k], ay[k + 1]),
+                             make_float2(az[k], az[k + 1]), make_float2(eb[k], eb[k + 1])};
+                interact2<FEAT>(make_float2(xy.x, xy.y), make_float2(xy.z, xy.w), make_float2(zm.x, zm.y),
+                                make_float2(zm.z, zm.w), make_float2(s2, s2), b, e2, a);
+                ax[k] = a.x.x, ax[k + 1] = a.x.y, ay[k] = a.y.x, ay[k + 1] = a.y.y;
+                az[k] = a.z.x, az[k + 1] = a.z.y;
+                if constexpr (FEAT) eb[k] = a.e.x, eb[k + 1] = a.e.y;
+            }
+        }
+    } else if constexpr (W == 32) {
+#pragma unroll 4
+        for (int i = at; i < at + cnt; ++i) {
+            const float4 q = lst[i];
+            const float dx = __fsub_rn(q.x, pb[0].x), dy = __fsub_rn(q.y, pb[0].y), dz = __fsub_rn(q.z, pb[0].z);
+            interact<REF, FEAT>(q, dx, dy, dz, dist2<REF>(dx, dy, dz, eps2), ax[0], ay[0], az[0], eb[0],
+                                FEAT ? lw[i] : 0.0f);
+        }
+    } else {
+        const int half = (threadIdx.x >> 4) & 1;
+#pragma unroll 4
+        for (int i = 0; i < cnt; i += 2) {
+            // (the record past an odd last one is whatever lies there; its terms are not added)
+            const int r = (at + i + half) & (kListCap - 1);
+            const float4 q = lst[r];
+            const float dx = __fsub_rn(q.x, pb[0].x), dy = __fsub_rn(q.y, pb[0].y), dz = __fsub_rn(q.z, pb[0].z);
+            const float d2 = dist2<REF>(dx, dy, dz, eps2);
+            float rd;
+            if constexpr (REF) rd = __frcp_rn(__fsqrt_rn(d2));
+            else rd = rsqrt_ftz(d2);
+            const float f = __fmul_rn(__fmul_rn(__fmul_rn(q.w, rd), rd), rd);
+            ax[0] = madd<REF>(dx, f, ax[0]);
+            ay[0] = madd<REF>(dy, f, ay[0]);
+            az[0] = madd<REF>(dz, f, az[0]);
+            float g = 0.0f, s2 = 0.0f;
+            if constexpr (FEAT) {
+                s2 = lw[r];
+                g = __fmul_rn(f, rd);
+                eb[0] = __fmaf_rn(g, s2, eb[0]);
+            }
+            const float f1 = __shfl_down_sync(0xffffffffu, f, 16);
+            const float x1 = __shfl_down_sync(0xffffffffu, dx, 16), y1 = __shfl_down_sync(0xffffffffu, dy, 16),
+                        z1 = __shfl_down_sync(0xffffffffu, dz, 16);
+            float g1 = 0.0f, s1 = 0.0f;
+            if constexpr (FEAT) {
+                g1 = __shfl_down_sync(0xffffffffu, g, 16);
+                s1 = __shfl_down_sync(0xffffffffu, s2, 16);
+            }
+            if (i + 1 < cnt) {
+                ax[0] = madd<REF>(x1, f1, ax[0]);
+                ay[0] = madd<REF>(y1, f1, ay[0]);
+                az[0] = madd<REF>(z1, f1, az[0]);
+                if constexpr (FEAT) eb[0] = __fmaf_rn(g1, s1, eb[0]);
+            }
+        }
+    }
+}
+
 // -------------------------------------------------------------------------------------
-// Force (calculateforce.cl:52-185).  A group of W bodies (W = 32: one warp; W = 16: the
-// reference's work-group, :99,145; W = 64: one warp with two bodies per lane) takes W
-// consecutive bodies of the depth-first order and walks its universe's tree.  A body
-// child is always accepted; a cell child only if every body of the group sees
-// d^2 + eps^2 >= dq[level] (work_group_all, :145), else it is opened.  The walk is
-// depth-first in child order (children are compacted, so the first empty slot ends a
-// cell), so every body accumulates its interactions in the reference's order.  Every lane
-// of a group accepts the same children, so the group's interaction count is counted once
-// per opened cell, not per visit.
-//
-// GB300 schedule: opening a cell loads its 8 child slots and the 8 node records that
-// summarize stored next to them (kids4) with one load per lane -- one round trip per
-// opened cell -- and pushes them, first child on top, onto the group's shared-memory
-// stack with their opening threshold (fixed angle: t0 * 4^-level + eps^2, formed once at
-// the push; per-body angle: the level factor 4^-level) or -1 for bodies, which makes the
-// test pass; each visit reads one record from shared memory and needs no branch on its
-// kind.  With W = 64 every stack pop, vote and cell opening serves two bodies per lane.
-// Lanes past the end of a universe walk with their group's first body, so they never
-// change a vote and need no predicate.  Work items (32 bodies; 64 for W = 64) are handed
-// out dynamically.  After the walk: the leapfrog velocity correction for step > 0
-// (:174-181) and the acceleration store (:183-185).
+// Force (calculateforce.cl:52-185).  A group of W bodies (W = 16: the reference's work-group,
+// :99,145; W = 32, 64, 128: one, two, four bodies per lane) is W consecutive bodies of the
+// depth-first order, and one warp walks its universe's tree.  A body child is always accepted; a
+// cell child only if every body of the group sees d^2 + eps^2 >= dq[level] (work_group_all,
+// :145), else it is opened.  Every lane of a group accepts the same children, so the group's
+// interactions are counted once.  Lanes past the end of a universe walk with their group's
+// first body, and for W = 16 the upper half-warp holds the same bodies as the lower, so no
+// vote needs a predicate.  Work items (32 bodies; 64 and 128 for those widths) are handed out
+// dynamically.  After the walk: the leapfrog velocity correction for step > 0 (:174-181) and the
+// acceleration store (:183-185).
 //
 // REF: reference arithmetic (rounded products, 1/sqrt correctly rounded); otherwise FMA and
 // the hardware inverse square root.  PB: per-body opening angle from theta_body (with
@@ -182,19 +250,33 @@ __device__ __forceinline__ void eval4(const float* lst, const int at, const List
 // p.feat_gate set, a launch that does not match the step's place in the learned-theta
 // schedule returns at once (the step graph holds a recording and a plain launch).
 //
-// LIST (W = 32, 64 or 128: one warp per group; FMA arithmetic): the same votes, taken
-// lane-parallel.  Each round the lanes take the children of up to four cells from the
-// group's cell stack, one child per lane (8 lanes per cell), and decide each child on its
-// own lane: a body is accepted; a cell is accepted when even the group's bounding box
-// passes the test (the box's distance components bound every body's from below, and the
-// rounded subtractions, the fused squares and the comparison are monotone, so every body's
-// own test passes), and opened when the group's body nearest the box centre fails it (then
-// the vote fails; with per-body angles also when the body with the smallest angle fails
-// it).  Only the remaining cells take the vote of every body, one after another.  Accepted records go to a list in shared memory, evaluated 32 at a time in a
-// loop of arithmetic alone: the same interactions as the per-visit walk, accumulated in
-// list order (rounding may differ from it in the last bits).  A cell stack that would
-// overflow restarts the group on the per-level walk (stack_cap entries: 256 by default,
-// enough for every 64-body group of the benchmarked spheres, which needed at most 99).
+// The votes are taken lane-parallel, one child per lane: a body is accepted; a cell is accepted
+// when even the group's bounding box passes the test (the box's distance components bound every
+// body's from below, and the rounded subtractions, products or fused squares, sums and the
+// comparison are monotone, so every body's own test passes), and opened when the group's body
+// nearest the box centre fails it (then the vote fails; with per-body angles also when the body
+// with the smallest angle fails it).  Only the remaining cells take the vote of every body, two
+// cells after two.  Accepted records go to a list in shared memory, evaluated 32 at a time in a
+// loop of arithmetic alone.
+//
+// The ordered walk (LIST = false) keeps the reference's order of accumulation (depth-first,
+// children in order): its stack holds every pending node with its record, the next one in order
+// on top: the record of an accepted node, or the index of a cell to open.  A round looks at the
+// top 32, moves the accepted ones above the first cell to open to the list, decides the children
+// of the first four cells to open, and puts them in those cells' places, the accepted nodes
+// between them moving up.  Force stage against visiting one node at a time with a vote each, us:
+// 4M disc (W = 64) 11928 / 13747, 1M Plummer sphere 2748 / 3178 (W = 32: 3046 / 3757); reference
+// arithmetic at theta^2 1.5 with W = 16: 100,003 bodies 174 / 276, 1M 1378 / 2065 (one warp per
+// group of 16 in place of two groups in the halves of a warp, which ran one after the other),
+// with W = 32 182 / 231 and 1030 / 1021.
+//
+// LIST (W = 32, 64 or 128; FMA arithmetic): each round takes the children of up to four cells
+// from a stack of cells alone; the records are accumulated in list order (rounding may differ
+// from the ordered walk in the last bits).
+//
+// In both, a stack that would overflow restarts the group on the per-level walk (stack_cap
+// entries: 256 by default; the 64-body groups of the benchmarked spheres need at most 99 in the
+// list walk).
 //
 // SPLIT (with LIST): a block of S = 2, 4 or 8 warps shares one group.  A group's walk is one
 // chain of rounds, and a universe with fewer groups than the GPU has room for warps leaves
@@ -220,39 +302,37 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
         if (load_status(p.st)) return;
     }
     if (p.feat_gate && theta_bound_step(p.st, p.st->step) != (p.feat_gate == 1)) return;
-    constexpr int GL = group_lanes<W>();            // lanes per group
-    constexpr int BPL = W / GL;                     // bodies per lane
+    constexpr int BPL = W < 32 ? 1 : W / 32;        // bodies per lane
     const int cap = p.stack_cap;
-    const int groups = blockDim.x / GL;
-    // The stack entry carries the finished threshold when it is the same for every body
-    // of the group (fixed angle) and nothing else needs the level factor.
-    constexpr bool kStoreDq = !PB && !FEAT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* const sq_all = reinterpret_cast<float4*>(smem_raw);
-    int2* const se_all = reinterpret_cast<int2*>(sq_all + groups * cap);
     const int lane = threadIdx.x & 31;
-    const int grp = threadIdx.x / GL;
-    const int glane = threadIdx.x % GL;
-    const unsigned gmask = (GL == 32) ? 0xffffffffu : (0xffffu << (16 * (lane >> 4)));
-    float4* const sq = sq_all + grp * cap;           // node record of each pending child
-    int2* const se = se_all + grp * cap;             // (node index, bits of threshold or level factor)
+    const int grp = threadIdx.x >> 5;
+    // ordered walk
+    constexpr int kDup = BPL >= 2 ? 2 : 1;           // float4 per list record
+    const int ocap = ordered_entries(cap);
+    float4* const sq = reinterpret_cast<float4*>(smem_raw + grp * force_smem_bytes<W>(32, cap, FEAT));   // pending nodes
+    float4* const ol = sq + ocap;
+    float4* const ogc = ol + kDup * kListCap;
+    float* const oud = reinterpret_cast<float*>(ogc + 4);
+    float* const olw = oud + 4 * 32;
+    float* const ssl = olw + kListCap;               // FEAT: level factor of each pending node (0: a body)
     // list walk: the group's list of accepted records and its stack of (cell, level)
     float* const lst = reinterpret_cast<float*>(smem_raw + (size_t)grp * list_group_bytes(SPLIT ? max(cap, kSplitQueue) : cap));
-    float* const ud = lst + 5 * kListCap;            // undecided cells of a round: x, y, z, threshold
-    float4* const gc = reinterpret_cast<float4*>(ud + 4 * 32);     // the group's box and representatives
+    float* const ud = LIST ? lst + 5 * kListCap : oud;   // undecided cells of a round: x, y, z, threshold
+    float4* const gc = LIST ? reinterpret_cast<float4*>(ud + 4 * 32) : ogc;   // the group's box and representatives
     int2* const cst = reinterpret_cast<int2*>(gc + 4);
     // deep-tree walk: (cell, next) per level
-    int* const snode = LIST ? reinterpret_cast<int*>(cst) : reinterpret_cast<int*>(se);
+    int* const snode = LIST ? reinterpret_cast<int*>(cst) : reinterpret_cast<int*>(sq);
     int* const snext = snode + kMaxDepth;
     const int nbody = p.nbody;
     const float eps2 = p.eps2;
     const int step = p.st->step;
-    const bool fast = p.st->max_depth <= fast_max_depth(cap);
     const float4* __restrict__ node4 = p.node4;
     const int* __restrict__ child = p.child;
     const float4* __restrict__ kids4 = p.kids4;
     const int2* __restrict__ items = BPL == 4 ? p.items128 : (BPL == 2 ? p.items64 : p.warps);
-    const int nitems = BPL == 4 ? p.nitems128 : (BPL == 2 ? p.nitems64 : p.nwarps);
+    // 32-body items are two groups of 16
+    const int nitems = BPL == 4 ? p.nitems128 : (BPL == 2 ? p.nitems64 : (W < 32 ? 2 * p.nwarps : p.nwarps));
     unsigned long long my_inter = 0;
 
     for (;;) {
@@ -267,13 +347,14 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
             item = __shfl_sync(0xffffffffu, item, 0);
         }
         if (item >= nitems) break;
+        const int half = W < 32 ? item & 1 : 0;
+        if (W < 32) item >>= 1;
         if (p.item_order) item = p.item_order[item];   // costly items first (see item_order_kernel)
         const int2 wi = items[item];
         const int u = wi.y;
         const int uend = p.ubody[u + 1];
-        // Lanes past the universe's end take their group's first body.
-        const int gfirst = wi.x + (GL < 32 ? (lane / GL) * GL : 0);
-        const bool gvalid = gfirst < uend;       // the group has any body at all
+        const int gfirst = wi.x + 16 * half;
+        if (W < 32 && gfirst >= uend) continue;         // the item's second group has no bodies
         const float r = p.uradius[u];
         const float rr = __fmul_rn(r, r);
         float4 pb[BPL];
@@ -281,8 +362,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
         float ax[BPL], ay[BPL], az[BPL], eb[BPL];
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
-            const int sk = wi.x + 32 * k + lane;
-            const int bk = gvalid ? p.sorted[sk < uend ? sk : gfirst] : 0;
+            // lanes past the universe's end take their group's first body
+            const int sk = gfirst + 32 * k + (W < 32 ? lane & 15 : lane);
+            const int bk = p.sorted[sk < uend ? sk : gfirst];
             pb[k] = node4[bk];
             float th2 = p.theta2;
             if constexpr (PB) {
@@ -300,7 +382,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
 #pragma unroll
                 for (int k = 1; k < BPL; ++k) tm = fmaxf(tm, t0[k]);
 #pragma unroll
-                for (int o = GL / 2; o > 0; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(gmask, tm, o));
+                for (int o = 16; o > 0; o >>= 1) tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, o));
 #pragma unroll
                 for (int k = 0; k < BPL; ++k) t0[k] = tm;
             }
@@ -309,10 +391,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
         int visits = 0;                                 // cost of this group's walk
         const int root = p.nnodes - u;
 
-        if (gvalid) {
-            bool walked = false;
-            if constexpr (LIST) {
-                walked = true;
+        {
+            bool walked = true;
+            {
                 // the group's bounding box (lanes past the end hold the first body)
                 float lox = pb[0].x, loy = pb[0].y, loz = pb[0].z, hix = pb[0].x, hiy = pb[0].y, hiz = pb[0].z;
 #pragma unroll
@@ -403,7 +484,15 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     rp2.y = __shfl_sync(0xffffffffu, mine2.y, r2src);
                     rp2.z = __shfl_sync(0xffffffffu, mine2.z, r2src);
                 }
-                const unsigned lt = (1u << lane) - 1u;
+                if (lane == 0) {
+                    gc[0] = make_float4(lox, loy, loz, tlb);
+                    gc[1] = make_float4(hix, hiy, hiz, trep);
+                    gc[2] = rp;
+                    if constexpr (PB) gc[3] = rp2;
+                }
+            }
+            const unsigned lt = (1u << lane) - 1u;
+            if constexpr (LIST) {
                 // from here on the bodies are held as ListBody (the empty asm keeps the compiler
                 // from holding their plain coordinates beside it)
                 ListBody lb[BPL];
@@ -416,13 +505,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     ls[k].x = ls[k].y = ls[k].z = ls[k].e = make_float2(0.f, 0.f);
                 }
                 const float2 eps22 = make_float2(eps2, eps2);
-                if (lane == 0) {
-                    cst[0] = make_int2(root, __float_as_int(1.0f));
-                    gc[0] = make_float4(lox, loy, loz, tlb);
-                    gc[1] = make_float4(hix, hiy, hiz, trep);
-                    gc[2] = rp;
-                    if constexpr (PB) gc[3] = rp2;
-                }
+                if (lane == 0) cst[0] = make_int2(root, __float_as_int(1.0f));
                 int ctop = 1, opened = 0;              // every tested child is accepted or opened
                 // breadth first (SPLIT) until there are enough cells to share: the cells from
                 // `head` on wait in order; dealt: accepted records so far
@@ -634,81 +717,158 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     }
                     __syncwarp();
                 }
-            } else if (fast) {
-                walked = true;
-                int top = 0;
-                int pushed = 0, opened = -1;
-                int open = root;
-                float open_s = 1.0f;                      // 4^-level of open's children
-                bool ok = true;
-                for (;;) {
-                    // push the children of `open`, first child on top
-                    int chk = kNull;
-                    float4 qk = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (glane < 8) {
-                        const size_t o8 = ((size_t)(open - nbody) << 3) + glane;
-                        chk = __ldg(child + o8);
-                        qk = __ldg(kids4 + o8);
+            } else {
+                // a pending cell to open: its index, the level factor of its parent's children (the
+                // root: 4, so that its own children's is 1), and kOpenTag in place of the mass
+                constexpr int kOpenTag = -1;
+                if (lane == 0)
+                    sq[0] = make_float4(__int_as_float(root), 4.0f, 0.0f, __int_as_float(kOpenTag));
+                int top = 1, opened = 0, accepted = 0;
+                int lcnt = 0, lbase = 0;               // the list is a ring, as in the list walk
+                __syncwarp();
+                while (top > 0) {
+                    const int T = min(32, top);
+                    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float sl = 0.0f;
+                    if (lane < T) {
+                        q = sq[top - 1 - lane];
+                        if constexpr (FEAT) sl = ssl[top - 1 - lane];
                     }
-                    float tag = open_s;
-                    if constexpr (kStoreDq) {
-                        // level factor of open's children, 4^-level(open), exact; the same
-                        // threshold the visit would form from it
-                        const int lv = __ldg(p.clevel + (open - nbody));
-                        tag = __fadd_rn(__fmul_rn(t0[0], __int_as_float((127 - 2 * lv) << 23)), eps2);
-                    }
-                    const unsigned bal = __ballot_sync(gmask, glane < 8 && chk >= 0) & gmask;
-                    const int cnt = __popc(bal);
-                    if (top + cnt > cap) {                 // unreachable below fast_max_depth(cap)
-                        raise_error(p.st, NBH_ERR_DEPTH);
-                        ok = false;
-                        break;
-                    }
-                    if (glane < cnt) {
-                        const int slot = top + cnt - 1 - glane;
-                        sq[slot] = qk;
-                        se[slot] = make_int2(chk, __float_as_int(chk >= nbody ? tag : -1.0f));
-                    }
-                    top += cnt;
-                    pushed += cnt;
-                    ++opened;
-                    __syncwarp(gmask);
-                    // visit until a cell has to be opened or the stack is empty
-                    open = -1;
-                    while (top > 0) {
-                        --top;
-                        const int2 e = se[top];
-                        const float4 q = sq[top];
-                        const float sl = __int_as_float(e.y);
-                        float dx[BPL], dy[BPL], dz[BPL], d2[BPL];
-                        bool pass = true;
-#pragma unroll
-                        for (int k = 0; k < BPL; ++k) {
-                            dx[k] = __fsub_rn(q.x, pb[k].x);
-                            dy[k] = __fsub_rn(q.y, pb[k].y);
-                            dz[k] = __fsub_rn(q.z, pb[k].z);
-                            d2[k] = dist2<REF>(dx[k], dy[k], dz[k], eps2);
-                            // t0 * 4^-level is exact (a power of two), so one fused op gives the
-                            // same threshold as the rounded product and sum
-                            const float dq = kStoreDq ? sl : __fmaf_rn(t0[k], sl, eps2);
-                            pass = pass && d2[k] >= dq;
-                        }
-                        if (__all_sync(gmask, pass)) {
-                            const float s2 = FEAT ? __fmul_rn(rr, fmaxf(sl, 0.0f)) : 0.0f;
-#pragma unroll
-                            for (int k = 0; k < BPL; ++k)
-                                interact<REF, FEAT>(q, dx[k], dy[k], dz[k], d2[k], ax[k], ay[k], az[k], eb[k], s2);
+                    const bool opn = lane < T && __float_as_int(q.w) == kOpenTag;
+                    const unsigned om = __ballot_sync(0xffffffffu, opn);
+                    // accepted nodes above the first cell to open: next in order, to the list
+                    const int emit = om ? __ffs((int)om) - 1 : T;
+                    if (lane < emit) {
+                        const int at = (lbase + lcnt + lane) & (kListCap - 1);
+                        if constexpr (kDup == 2) {
+                            ol[2 * at] = make_float4(q.x, q.x, q.y, q.y);
+                            ol[2 * at + 1] = make_float4(q.z, q.z, q.w, q.w);
                         } else {
-                            open = e.x;
-                            if constexpr (!kStoreDq) open_s = __fmul_rn(sl, 0.25f);
+                            ol[at] = q;
+                        }
+                        if constexpr (FEAT) olw[at] = __fmul_rn(rr, sl);
+                    }
+                    lcnt += emit;
+                    if (!om) {
+                        top -= T;
+                    } else {
+                        // the first four cells to open, at most, at lanes at[0] < at[1] < ...
+                        int at[4], last = emit;
+                        unsigned m = om;
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            at[g] = m ? __ffs((int)m) - 1 : 32;
+                            if (m) last = at[g];
+                            m &= m - 1;
+                        }
+                        // one at a time when their children might not fit (group-uniform)
+                        if (top - 1 - emit + 32 > ocap - kOrderedSlack) {
+                            last = emit;
+                            at[1] = at[2] = at[3] = 32;
+                        }
+                        const int g = lane >> 3;
+                        const int from = g == 0 ? at[0] : (g == 1 ? at[1] : (g == 2 ? at[2] : at[3]));
+                        const int cell = __float_as_int(__shfl_sync(0xffffffffu, q.x, from & 31));
+                        const float csl = __fmul_rn(__shfl_sync(0xffffffffu, q.y, from & 31), 0.25f);
+                        int ch = kNull;
+                        float4 cq = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (from < 32) {
+                            const size_t o8 = ((size_t)(cell - nbody) << 3) + (lane & 7);
+                            ch = __ldg(child + o8);
+                            cq = __ldg(kids4 + o8);
+                        }
+                        // the children's votes
+                        bool keep = ch >= 0 && ch < nbody, inc = false;   // keep: accepted
+                        float qlb = 0.0f;
+                        if (ch >= nbody) {
+                            const float4 lo = gc[0], hi = gc[1];
+                            const float gx = fmaxf(fmaxf(__fsub_rn(cq.x, hi.x), __fsub_rn(lo.x, cq.x)), 0.0f);
+                            const float gy = fmaxf(fmaxf(__fsub_rn(cq.y, hi.y), __fsub_rn(lo.y, cq.y)), 0.0f);
+                            const float gz = fmaxf(fmaxf(__fsub_rn(cq.z, hi.z), __fsub_rn(lo.z, cq.z)), 0.0f);
+                            // t0 * 4^-level is exact, so the fused form gives the same threshold
+                            qlb = __fmaf_rn(lo.w, csl, eps2);
+                            if (dist2<REF>(gx, gy, gz, eps2) >= qlb) {
+                                keep = true;
+                            } else {
+                                const float4 r1 = gc[2];
+                                const float rx = __fsub_rn(cq.x, r1.x), ry = __fsub_rn(cq.y, r1.y),
+                                            rz = __fsub_rn(cq.z, r1.z);
+                                inc = !(dist2<REF>(rx, ry, rz, eps2) < (PB ? __fmaf_rn(hi.w, csl, eps2) : qlb));
+                                if constexpr (PB) {
+                                    const float4 r2 = gc[3];
+                                    const float sx = __fsub_rn(cq.x, r2.x), sy = __fsub_rn(cq.y, r2.y),
+                                                sz = __fsub_rn(cq.z, r2.z);
+                                    inc = inc && !(dist2<REF>(sx, sy, sz, eps2) < qlb);
+                                }
+                            }
+                        }
+                        const unsigned im = __ballot_sync(0xffffffffu, inc);
+                        if (im) {
+                            const int nud = __popc(im);
+                            const int mine = __popc(im & lt);
+                            if (inc)
+                                reinterpret_cast<float4*>(ud)[mine] = make_float4(cq.x, cq.y, cq.z, PB ? csl : qlb);
+                            __syncwarp();
+                            unsigned res = 0;
+#pragma unroll 2
+                            for (int j = 0; j < nud; ++j) {
+                                const float4 uq = reinterpret_cast<const float4*>(ud)[j];
+                                bool pass = true;
+#pragma unroll
+                                for (int k = 0; k < BPL; ++k) {
+                                    const float dx = __fsub_rn(uq.x, pb[k].x), dy = __fsub_rn(uq.y, pb[k].y),
+                                                dz = __fsub_rn(uq.z, pb[k].z);
+                                    pass = pass && dist2<REF>(dx, dy, dz, eps2) >=
+                                                       (PB ? __fmaf_rn(t0[k], uq.w, eps2) : uq.w);
+                                }
+                                res |= (__all_sync(0xffffffffu, pass) ? 1u : 0u) << j;
+                            }
+                            if (inc) keep = (res >> mine) & 1u;
+                        }
+                        const unsigned vm = __ballot_sync(0xffffffffu, ch >= 0);
+                        const unsigned am = ~om & ~((1u << emit) - 1u) & ((1u << last) - 1u);   // moving up
+                        const int n = __popc(am) + __popc(vm);
+                        const int base = top - 1 - last;
+                        if (base + n > ocap) {         // group-uniform
+                            walked = false;
                             break;
                         }
+                        opened += 1 + __popc(om & ((1u << last) - 1u));
+                        __syncwarp();                  // the window has been read
+                        if ((am >> lane) & 1u) {
+                            int ord = __popc(am & lt);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                if (at[k] < lane) ord += __popc((vm >> (8 * k)) & 0xffu);
+                            sq[base + n - 1 - ord] = q;
+                            if constexpr (FEAT) ssl[base + n - 1 - ord] = sl;
+                        }
+                        if (ch >= 0) {
+                            const int ord = __popc(am & ((1u << from) - 1u)) + __popc(vm & lt);
+                            sq[base + n - 1 - ord] =
+                                keep ? cq : make_float4(__int_as_float(ch), csl, 0.0f, __int_as_float(kOpenTag));
+                            if constexpr (FEAT) ssl[base + n - 1 - ord] = ch >= nbody ? csl : 0.0f;
+                        }
+                        top = base + n;
                     }
-                    if (open < 0) break;
-                    __syncwarp(gmask);     // every lane has read the stack before it is refilled
+                    __syncwarp();
+                    if (lcnt >= 32) {
+                        eval_ordered<W, REF, FEAT>(ol, olw, lbase, 32, pb, eps2, ax, ay, az, eb);
+                        accepted += 32;
+                        lcnt -= 32;
+                        lbase ^= 32;
+                        __syncwarp();
+                    }
                 }
-                if (ok) ninter = pushed - opened;
-                visits = pushed;
+                if (walked) {
+                    eval_ordered<W, REF, FEAT>(ol, olw, lbase, lcnt, pb, eps2, ax, ay, az, eb);
+                    ninter = accepted + lcnt;
+                    visits = accepted + lcnt + opened;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < BPL; ++k) ax[k] = ay[k] = az[k] = eb[k] = 0.0f;
+                }
+                __syncwarp();
             }
             if (!walked) {
                 // Deep trees: per-level (cell, next child) walk (calculateforce.cl:112-172).
@@ -742,7 +902,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         d2[k] = dist2<REF>(dx[k], dy[k], dz[k], eps2);
                         pass = pass && d2[k] >= dq[k];
                     }
-                    if (ch < nbody || __all_sync(gmask, pass)) {
+                    if (ch < nbody || __all_sync(0xffffffffu, pass)) {
                         const float s2 = ch >= nbody ? ldexpf(rr, -2 * depth) : 0.0f;
 #pragma unroll
                         for (int k = 0; k < BPL; ++k)
@@ -769,8 +929,8 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
 #pragma unroll
         for (int k = 0; k < BPL; ++k) {
             // looked up again rather than held in registers through the walk
-            const int sk = wi.x + 32 * k + lane;
-            if (sk >= p.ubody[u + 1]) continue;
+            const int sk = gfirst + 32 * k + lane;
+            if (sk >= p.ubody[u + 1] || (W < 32 && lane >= W)) continue;
             const int bk = p.sorted[sk];
             if (p.G != 1.0f) {
                 ax[k] = __fmul_rn(ax[k], p.G);
@@ -806,11 +966,10 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
             p.acc[bk] = make_float4(ax[k], ay[k], az[k], eb[k]);
         }
         if (p.item_cost) {
-            // the item's cost: its group's visits (the deep walk counts accepted children);
-            // two half-warp groups (W = 16) add up
-            int c = visits > 0 ? visits : (int)min(ninter, (long long)0x7fffffff);
-            if (GL < 32) c += __shfl_down_sync(0xffffffffu, c, 16);
-            if (lane == 0) p.item_cost[item] = c;
+            // the item's cost: its group's visits (the deep walk counts accepted children), the
+            // first of two groups' (W = 16)
+            const int c = visits > 0 ? visits : (int)min(ninter, (long long)0x7fffffff);
+            if (lane == 0 && half == 0) p.item_cost[item] = c;
         }
         __syncwarp();
     }
@@ -823,8 +982,8 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
 // bounds their registers: 3 (up to 80 registers) for all but the plain list walk, which fits in
 // 64 without spills and takes 4 (measured, us per step with 4 against 3: 256-universe ensemble
 // 6407 against 6488, 1M sphere 2618 against 2600; the list walk with per-body angles spills at
-// 64: 8 learned steps 18143 against 17435).  The per-visit walks end up with 64 registers (left
-// to itself the compiler takes 48, with less overlap in the visit loop: 0.7-1.6 % slower).
+// 64: 8 learned steps 18143 against 17435).  The ordered
+// walks take 79-80 (4M disc with 64 registers: 12291 against 11928).
 // The other widths keep the compiler's own choice.
 template <int W, bool REF, bool PB, bool FEAT, bool LIST = false>
 __global__ void __launch_bounds__(kForceThreadsMax) force_kernel(StepParams p) {
@@ -866,7 +1025,7 @@ static void launch_force_pf(const StepParams& p, bool feat, int grid, int thread
             return;
         }
     }
-    const size_t sm = force_smem_bytes<W>(threads, p.stack_cap);
+    const size_t sm = force_smem_bytes<W>(threads, p.stack_cap, feat);
     if (feat) force_entry<W, REF, PB, true>()<<<grid, threads, sm, s>>>(p);
     else force_entry<W, REF, PB, false>()<<<grid, threads, sm, s>>>(p);
 }
@@ -881,7 +1040,7 @@ static void launch_force_t(const StepParams& p, bool pb, bool feat, int grid, in
 template <int W, bool REF, bool PB, bool FEAT>
 static cudaError_t prep_force() {
     return cudaFuncSetAttribute(force_entry<W, REF, PB, FEAT>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)force_smem_bytes<W>(kForceThreadsMax, kStackCapMax));
+                                (int)force_smem_bytes<W>(kForceThreadsMax, kStackCapMax, true));
 }
 
 template <int W, bool REF>
@@ -933,12 +1092,10 @@ int prepare_force_kernels() {
 }
 
 bool force_geometry_valid(int vote, int threads, int cap) {
-    const int gl = vote < 32 ? vote : 32;
-    return (threads == 64 || threads == 128 || threads == 256) && threads % gl == 0 && cap >= kStackCapMin &&
+    (void)vote;
+    return (threads == 64 || threads == 128 || threads == 256) && cap >= kStackCapMin &&
            cap <= kStackCapMax && cap % 8 == 0;
 }
-
-int force_fast_max_depth(int cap) { return fast_max_depth(cap); }
 
 void launch_force(const StepParams& p, int vote, bool ref, bool feat, int grid, int threads, cudaStream_t s) {
     const bool pb = p.theta_body != nullptr;
@@ -1065,19 +1222,19 @@ int occupancy_force(int vote, bool ref, int threads, int cap, bool list, int* bl
     }
     if (vote == 128)
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_kernel<128, false, false, false>,
-                                                             threads, force_smem_bytes<128>(threads, cap));
+                                                             threads, force_smem_bytes<128>(threads, cap, false));
     if (vote == 64)
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_entry<64, false, false, false>(),
-                                                             threads, force_smem_bytes<64>(threads, cap));
+                                                             threads, force_smem_bytes<64>(threads, cap, false));
     if (vote == 16)
         return ref ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_kernel<16, true, false, false>,
-                                                                   threads, force_smem_bytes<16>(threads, cap))
+                                                                   threads, force_smem_bytes<16>(threads, cap, false))
                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_kernel<16, false, false, false>,
-                                                                   threads, force_smem_bytes<16>(threads, cap));
+                                                                   threads, force_smem_bytes<16>(threads, cap, false));
     return ref ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_kernel<32, true, false, false>,
-                                                               threads, force_smem_bytes<32>(threads, cap))
+                                                               threads, force_smem_bytes<32>(threads, cap, false))
                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, force_kernel<32, false, false, false>,
-                                                               threads, force_smem_bytes<32>(threads, cap));
+                                                               threads, force_smem_bytes<32>(threads, cap, false));
 }
 
 }  // namespace nbh

@@ -30,7 +30,6 @@ bool force_geometry_valid(int vote, int threads, int cap);
 // Work-item order of the force launches: longest walks first, from the last launch's costs.
 void launch_item_order(const int* cost, int nitems, int* order, cudaStream_t s);
 void launch_item_order_reset(int nitems, int* order, int* cost, cudaStream_t s);
-int force_fast_max_depth(int cap);   // deepest tree the stack of `cap` entries walks without the per-level walk
 void launch_integrate(const StepParams& p, bool ref, int grid, cudaStream_t s);
 
 void launch_pack(int n, const float* soa, int mask, float4* node4, float4* vel, float4* acc, int grid,

@@ -881,3 +881,43 @@ def test_one_launch_tree_reports_errors_and_recovers():
     with pytest.raises(nbh.NbhError) as ei:
         h.step()
     assert ei.value.code == L.NBH_ERR_POOL
+
+
+@pytest.mark.parametrize("kw", [{"precise": True}, {"force_list": 2, "vote_width": 128}, {"force_list": 2, "vote_width": 32},
+                                {"vote_width": 16}, {"vote_width": 16, "reference": True},
+                                {"vote_width": 32, "reference": True}],
+                         ids=["precise", "128", "32", "16", "16-reference", "32-reference"])
+@pytest.mark.parametrize("n", [1, 17, 65, 5000, 30000])
+def test_ordered_walk_is_the_per_level_walk_bit_for_bit(kw, n):
+    """The ordered walk accumulates depth-first, children in order, like the per-level walk its
+    groups restart on when their stack overflows: the same sums with stacks that hold 64, 96 and 256
+    nodes (small ones overflow for part of the groups at this angle), and the interactions of the
+    oracle; error bounds of a probe likewise."""
+    import nbh
+    from nbh import learned as LR
+    kw = dict(kw)
+    if kw.pop("reference", False):
+        kw["arith"] = nbh.NBH_ARITH_REFERENCE
+    arrs = plummer(n, seed=89)
+    out = []
+    for cap in (256, 96, 64):
+        g = gpu_sim(theta=0.3, eps=0.05, dt=0.01, stack_cap=cap, **kw)
+        g.load(*arrs)
+        g.step(2)
+        p = LR.probe(g, None)
+        out.append((g.read(), g.stats()["interactions"], p))
+    for state, inter, p in out[1:]:
+        assert inter == out[0][1]
+        for k in KEYS:
+            np.testing.assert_array_equal(state[k], out[0][0][k], err_msg=k)
+        for a, b in zip(p, out[0][2]):
+            np.testing.assert_array_equal(a, b)
+    vote = kw.get("vote_width", 64)
+    o = oracle_for(n, theta=0.3, eps=0.05, dt=0.01, vote=vote, fma="arith" not in kw)
+    o.load(*arrs)
+    o.step()
+    g = gpu_sim(theta=0.3, eps=0.05, dt=0.01, **{k: v for k, v in kw.items() if k != "precise"},
+                **({"force_list": 2} if kw.get("precise") else {}))
+    g.load(*arrs)
+    g.step()
+    assert g.stats()["interactions"] == o.interactions
