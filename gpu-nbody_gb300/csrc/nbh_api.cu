@@ -236,7 +236,7 @@ void enqueue_tree(nbh_sim* sim, const StepParams& p, bool timed = false) {
     }
     launch_bbox(p, sim->grid_bbox, s);
     if (timed) cudaEventRecord(sim->ev[1], s);
-    launch_build(p, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
+    launch_build(p, ref, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
                  sim->top_split, s);
     launch_link(p, sim->grid_sum, s);
     if (timed) cudaEventRecord(sim->ev[2], s);

@@ -59,7 +59,8 @@ struct DevState {
     int nbuckets;        // bucketed build: non-empty slots of the sampled tree
     int bucket_next;     // bucketed build: work counter of the subtree builders
     int pool_low;        // lowest cell whose slots a build may have written since the last reset
-    unsigned long long pad2;
+    int sum_low;         // cells below were summed as they were built, but for the listed ones
+    int nextra;          // cells below sum_low that were not, listed in start[]
     // Build contention meters, spread over kDiagSlots addresses so that counting does not
     // itself serialise: descents that found their slot locked, and lost lock races.
     int lock_waits[32];

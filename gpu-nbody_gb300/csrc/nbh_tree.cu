@@ -139,6 +139,8 @@ __global__ void __launch_bounds__(256) bbox_kernel(StepParams p) {
         st->bucket_fill = 0;
         st->nbuckets = 0;
         st->bucket_next = 0;
+        st->sum_low = 0;
+        st->nextra = 0;
         for (int j = 0; j < kDiagSlots; ++j) st->lock_waits[j] = st->cas_misses[j] = 0;
         st->interactions = 0ull;
     }
@@ -268,6 +270,7 @@ __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts,
                     reinterpret_cast<int4*>(cc)[0] = make_int4(kNull, kNull, kNull, kNull);
                     reinterpret_cast<int4*>(cc)[1] = make_int4(kNull, kNull, kNull, kNull);
                     p.arrive[cell - nbody] = 0;
+                    p.count[cell - nbody] = -1;           // not summed yet (see link_kernel)
                     p.clevel[cell - nbody] = depth - 1;   // root = level 0
                     if (zero_counts) {   // bucket counters of the sampled tree
                         int4* bc = reinterpret_cast<int4*>(p.kids4 + ((size_t)(cell - nbody) << 3));
@@ -546,6 +549,7 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
     for (int c = 1 + (int)threadIdx.x; c < nc; c += blockDim.x) {
         const int k = gb - c - nbody;
         p.arrive[k] = 0;
+        p.count[k] = -1;
         p.clevel[k] = lvl[c];
         if (zero_counts) {   // bucket counters of the sampled tree
             int4* bc = reinterpret_cast<int4*>(p.kids4 + ((size_t)k << 3));
@@ -581,8 +585,10 @@ constexpr BuildPhase kBucketBodies = {1, 16};   // the bodies outside the 1/16 s
 // (1) locate: read-only descent of each remaining body to its slot; the slot index goes
 // to parent[b] and the body's place in the slot's bucket, from the counter, to sorted[b]
 // (scratch: the link and sort passes write both later).
-__global__ void __launch_bounds__(256) bucket_locate_kernel(StepParams p, BuildPhase set, bool reset_counters) {
+__global__ void __launch_bounds__(256) bucket_locate_kernel(StepParams p, BuildPhase set, bool reset_counters,
+                                                            bool last_pass) {
     if (load_status(p.st)) return;
+    if (last_pass && blockIdx.x == 0 && threadIdx.x == 0) p.st->sum_low = ld_relaxed(&p.st->bottom);
     if (reset_counters && blockIdx.x == 0 && threadIdx.x == 0) {
         // a second pass: the work-list counters start over (the first pass is complete)
         p.st->bucket_fill = 0;
@@ -730,7 +736,7 @@ constexpr int kBucketWarps = 4;
 // of the grid) and 43 for the register subtrees of at most 32 bodies (shared memory).
 constexpr int kBucketStack = 232;
 constexpr int kSmallStack = 48;
-constexpr int kBucketBlocksPerSm = 9;
+constexpr int kBucketBlocksPerSm = 7;     // all resident, at 72 registers (9 blocks: 1M sphere 324 for 310 us)
 constexpr int kBucketChunk = 8;      // most buckets a warp takes per work-counter atomic
 
 // Stack position of each child cell among the nc cells pushed now: the largest deepest.
@@ -742,6 +748,12 @@ __device__ __forceinline__ int deeper_rank(int mycnt, int lane) {
         deeper += (n2 >= 2 && (n2 > mycnt || (n2 == mycnt && o2 < lane))) ? 1 : 0;
     }
     return deeper;
+}
+
+// A cell of the last pass that link and summarize must see to (the others of that pass are summed
+// as they are made); listed in start[], which the sort fills later.
+__device__ __forceinline__ void left_to_sum(const StepParams& p, int cell) {
+    p.start[atomicAdd(&p.st->nextra, 1)] = cell;
 }
 
 // The subtree of the m <= 32 bodies src[lo, lo + m) below a cell of level `level` with the
@@ -791,7 +803,9 @@ __device__ int small_subtree(const StepParams& p, const int* __restrict__ src, i
             if (lane < 8 && !((occ >> lane) & 1u)) cell_child(p, t.cell)[lane] = kNull;
             if (lane == 0) {
                 p.arrive[t.cell - nbody] = 0;
+                p.count[t.cell - nbody] = -1;
                 p.clevel[t.cell - nbody] = t.level;
+                if (!zero_counts) left_to_sum(p, t.cell);
             }
             if (zero_counts && lane < 2)   // bucket counters for a pass into this tree
                 reinterpret_cast<int4*>(p.kids4 + ((size_t)(t.cell - nbody) << 3))[lane] = make_int4(0, 0, 0, 0);
@@ -865,10 +879,15 @@ __device__ __forceinline__ int parts_that_fit(const Part& part, int first, int e
 }
 
 // The subtrees of the parts of lanes [first, first + cnt), at most 32 bodies in all.  Parts of
-// no bodies among them are passed over.  Whole-warp call; false after raising an error.
+// no bodies among them are passed over.  FINAL: nothing will be added to these subtrees, so they
+// are summed on the spot (see summarize_kernel), a level after the other from the deepest: a lane
+// holds the record of what begins at its place (its body, then the cells made of it) and stores it
+// in the parent's row at its rank, and the lane where a cell begins adds its children's records
+// in order.  Whole-warp call; false after raising an error.
+template <bool FINAL, bool REF>
 __device__ bool packed_subtrees(const StepParams& p, const int* src_list, const Part& part, const int incl,
-                                const int first, const int cnt, SmallTask* sstack, int& local_max,
-                                bool zero_counts) {
+                                const int first, const int cnt, SmallTask* sstack, int& local_max) {
+    constexpr bool zero_counts = !FINAL;             // bucket counters for a pass into this tree
     constexpr int kLevels = 8;                       // octants in a key: 3 bits bucket, 24 path, 5 lane
     const int lane = threadIdx.x & 31;
     const int nbody = p.nbody;
@@ -994,30 +1013,78 @@ __device__ bool packed_subtrees(const StepParams& p, const int* src_list, const 
     const int outer = __shfl_sync(0xffffffffu, org, begin) - cl;
     for (int i = lane; i < 2 * cells; i += 32)
         reinterpret_cast<int4*>(cell_child(p, base - cells))[i] = make_int4(kNull, kNull, kNull, kNull);
-    for (int i = lane; i < cells; i += 32) {
-        p.arrive[base - cells - nbody + i] = 0;
-        if (zero_counts) {                                   // bucket counters for a pass into this tree
+    if constexpr (!FINAL) {
+        for (int i = lane; i < cells; i += 32) {
+            p.arrive[base - cells - nbody + i] = 0;
+            p.count[base - cells - nbody + i] = -1;
             int4* bc = reinterpret_cast<int4*>(bucket_counters(p, base - cells + i));
             bc[0] = make_int4(0, 0, 0, 0);
             bc[1] = make_int4(0, 0, 0, 0);
         }
-    }
-    __syncwarp();
-    for (int l = cl + 1; l <= cr; ++l) {
-        const int cell = org - l;
-        p.clevel[cell - nbody] = slev + l;
-        const int up = l == 0 ? sc : (l == cl + 1 ? outer : cell + 1);
-        cell_child(p, up)[l == 0 ? sj : (int)((path >> (3 * (kLevels - l))) & 7u)] = cell;
-    }
-    if (active) {
-        const int l = max(cl, cr);                           // level of the body's cell, -1: none made
-        const int up = l < 0 ? sc : (cr > cl ? org - cr : outer);
-        cell_child(p, up)[l < 0 ? sj : (int)((path >> (3 * (kLevels - 1 - l))) & 7u)] = sb;
+        __syncwarp();
+        for (int l = cl + 1; l <= cr; ++l) {
+            const int cell = org - l;
+            p.clevel[cell - nbody] = slev + l;
+            const int up = l == 0 ? sc : (l == cl + 1 ? outer : cell + 1);
+            cell_child(p, up)[l == 0 ? sj : (int)((path >> (3 * (kLevels - l))) & 7u)] = cell;
+        }
+        if (active) {
+            const int l = max(cl, cr);                       // level of the body's cell, -1: none made
+            const int up = l < 0 ? sc : (cr > cl ? org - cr : outer);
+            cell_child(p, up)[l < 0 ? sj : (int)((path >> (3 * (kLevels - 1 - l))) & 7u)] = sb;
+        }
+    } else {
+        float4 rec = make_float4(__shfl_sync(0xffffffffu, q.x, src), __shfl_sync(0xffffffffu, q.y, src),
+                                 __shfl_sync(0xffffffffu, q.z, src), __shfl_sync(0xffffffffu, q.w, src));
+        int idx = sb;                                        // whose record it is
+        const unsigned lt = (1u << lane) - 1u;
+        __syncwarp();                                        // the slots are empty
+        for (int l = __reduce_max_sync(0xffffffffu, active ? cr : -1); l >= 0; --l) {
+            // places where a child of a level-l cell begins, and where such a cell ends
+            const unsigned starts = __ballot_sync(0xffffffffu, active && cl <= l);
+            const unsigned ends = __ballot_sync(0xffffffffu, !active || cl < l) & ~(lt | (1u << lane));
+            const bool own = active && cl < l && l <= cr;    // a level-l cell begins here
+            const int cell = org - l;
+            if (own || (active && cl == l)) {
+                const int up = own ? cell : outer, from_lane = own ? lane : begin;
+                const int rank = __popc(starts & lt & ~((1u << from_lane) - 1u));
+                cell_child(p, up)[rank] = idx;
+                p.kids4[((size_t)(up - nbody) << 3) + rank] = rec;
+                p.parent[idx] = up;
+                if (idx >= nbody) p.loff[idx - nbody] = lane - from_lane;
+            }
+            const int end = ends ? __ffs((int)ends) - 1 : 32;
+            unsigned kids = own ? starts & ~lt & (end < 32 ? (1u << end) - 1u : 0xffffffffu) : 0u;
+            float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
+            while (__any_sync(0xffffffffu, kids != 0u)) {
+                const int k = kids ? __ffs((int)kids) - 1 : lane;
+                const float x = __shfl_sync(0xffffffffu, rec.x, k), y = __shfl_sync(0xffffffffu, rec.y, k);
+                const float z = __shfl_sync(0xffffffffu, rec.z, k), w = __shfl_sync(0xffffffffu, rec.w, k);
+                if (kids) {
+                    cm = __fadd_rn(cm, w);
+                    sx = madd<REF>(x, w, sx);
+                    sy = madd<REF>(y, w, sy);
+                    sz = madd<REF>(z, w, sz);
+                }
+                kids &= kids - 1u;
+            }
+            if (own) {
+                const float inv = __fdiv_rn(1.0f, cm);
+                rec = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
+                idx = cell;
+                p.node4[cell] = rec;
+                p.count[cell - nbody] = end - lane;
+                p.clevel[cell - nbody] = slev + l;
+            }
+        }
+        if (active && cl < 0) cell_child(p, sc)[sj] = idx;
     }
     return true;
 }
 
-__global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepParams p, bool zero_counts) {
+template <bool FINAL, bool REF>
+__global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepParams p) {
+    constexpr bool zero_counts = !FINAL;
     __shared__ SmallTask small_all[kBucketWarps][kSmallStack];
     if (load_status(p.st)) return;
     BucketTask* stack = static_cast<BucketTask*>(p.bstack) +
@@ -1055,7 +1122,7 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
             int incl;
             const int cnt = parts_that_fit(part, it, nitem, incl);
             if (cnt > 0) {
-                if (!packed_subtrees(p, p.bwork, part, incl, it, cnt, sstack, local_max, zero_counts)) return;
+                if (!packed_subtrees<FINAL, REF>(p, p.bwork, part, incl, it, cnt, sstack, local_max)) return;
                 it += cnt;
                 continue;
             }
@@ -1173,7 +1240,9 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                 }
                 if (lane == 0) {
                     p.arrive[t.cell - nbody] = 0;
+                    p.count[t.cell - nbody] = -1;
                     p.clevel[t.cell - nbody] = t.level;
+                    if (FINAL) left_to_sum(p, t.cell);
                 }
                 if (zero_counts && lane < 2)
                     reinterpret_cast<int4*>(p.kids4 + ((size_t)(t.cell - nbody) << 3))[lane] = make_int4(0, 0, 0, 0);
@@ -1183,7 +1252,7 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
                 for (int o = 0; o < 8 && ok;) {
                     int incl;
                     const int cnt = parts_that_fit(small, o, 8, incl);
-                    ok = packed_subtrees(p, dst, small, incl, o, cnt, sstack, local_max, zero_counts);
+                    ok = packed_subtrees<FINAL, REF>(p, dst, small, incl, o, cnt, sstack, local_max);
                     o += cnt;
                 }
                 if (!ok) break;
@@ -1204,15 +1273,30 @@ __global__ void __launch_bounds__(32 * kBucketWarps) bucket_build_kernel(StepPar
 // Link: parent[] of every node from the finished tree (one pass over the cells), for the
 // bottom-up summarize, the sort's walk-up and the learned angle's features (a body's leaf
 // cell).  Keeping it out of the build means an insertion publishes nothing but a slot value.
-// It also tags each cell's count with its number of cell children k, as -1 - k: summarize
-// decides from this tag, which nothing changes until the cell is summed, and never from the
-// cell's slots, which the cell's summation rewrites (compaction) while other threads run.
+// It also tags each cell's count with its number of cell children that are still to be summed, k,
+// as -1 - k: summarize decides from this tag, which nothing changes until the cell is summed,
+// and never from the cell's slots, which the cell's summation rewrites (compaction) while
+// other threads run.  Cells are made with a count of -1; the ones that the last bucketed pass
+// summed have a positive count and are linked already, and so this pass and summarize go over
+// the cells from sum_low up and the ones that pass listed (1M sphere: 32,000 of 504,000 cells and
+// a few of the list).
+__device__ __forceinline__ int cells_to_sum(const StepParams& p, int& low) {
+    low = max(p.st->bottom, p.st->sum_low);
+    return p.nnodes + 1 - low + p.st->nextra;
+}
+__device__ __forceinline__ int cell_to_sum(const StepParams& p, int low, int i) {
+    const int c = low + i;
+    return c <= p.nnodes ? c : p.start[c - p.nnodes - 1];
+}
+
 __global__ void __launch_bounds__(256) link_kernel(StepParams p) {
     if (load_status(p.st)) return;
-    const int bottom = p.st->bottom;
+    int low;
+    const int cells = cells_to_sum(p, low);
     const int nbody = p.nbody;
     const int stride = gridDim.x * blockDim.x;
-    for (int c = bottom + (int)(blockIdx.x * blockDim.x + threadIdx.x); c <= p.nnodes; c += stride) {
+    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < cells; i += stride) {
+        const int c = cell_to_sum(p, low, i);
         const int* ch8 = cell_child(p, c);
         const int4 s0 = reinterpret_cast<const int4*>(ch8)[0];
         const int4 s1 = reinterpret_cast<const int4*>(ch8)[1];
@@ -1221,7 +1305,7 @@ __global__ void __launch_bounds__(256) link_kernel(StepParams p) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (sl[j] >= 0) p.parent[sl[j]] = c;
-            kc += sl[j] >= nbody;
+            if (sl[j] >= nbody) kc += p.count[sl[j] - nbody] <= 0;
         }
         p.count[c - nbody] = -1 - kc;
     }
@@ -1243,7 +1327,10 @@ __global__ void __launch_bounds__(256) link_kernel(StepParams p) {
 //     sort stage derives every start without waiting (sort.cl:44-58 hands these offsets
 //     down from the root instead).
 // Arrivals after a write are release atomics and the last arriver acquires, in place of
-// full fences.
+// full fences.  What is left here by the bucketed build (see link_kernel) is the top of the tree,
+// bound by the latency of its climb, a round trip each for a cell's slots, its children's
+// records and the arrival: 49 us at 1M bodies (124 with every cell and the children's
+// records loaded one after another), 94 for 256 universes (321), 270 at 16M (1320).
 __device__ __forceinline__ int arrive_acq_rel(int* p) {
     int old;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
@@ -1261,17 +1348,24 @@ __device__ __forceinline__ float4 sum_children(const StepParams& p, int c, const
     float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
     double dm = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
     float4* kb = p.kids4 + ((size_t)(c - nbody) << 3);
+    // every load before the first store (which might be to the same place, for all the compiler
+    // knows), so that the children's round trips overlap
+    float4 rec[8];
+    int bodies[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        rec[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        bodies[j] = 1;
+        if (sl[j] >= 0) rec[j] = ld_cg4(p.node4 + sl[j]);
+        if (sl[j] >= nbody) bodies[j] = __ldcg(p.count + (sl[j] - nbody));
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int ch = sl[j];
         if (ch < 0) continue;
-        const float4 q = ld_cg4(p.node4 + ch);
-        if (ch >= nbody) {
-            p.loff[ch - nbody] = cnt;
-            cnt += __ldcg(p.count + (ch - nbody));
-        } else {
-            cnt += 1;
-        }
+        const float4 q = rec[j];
+        if (ch >= nbody) p.loff[ch - nbody] = cnt;
+        cnt += bodies[j];
         if constexpr (F64) {
             dm += (double)q.w;
             dx += (double)q.x * (double)q.w;
@@ -1290,10 +1384,7 @@ __device__ __forceinline__ float4 sum_children(const StepParams& p, int c, const
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (j >= used) {
-            ch8[j] = kNull;
-            kb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        if (j >= used) ch8[j] = kNull;              // (no record: nothing reads an empty slot's)
     p.count[c - nbody] = cnt;
     if constexpr (F64) {
         return make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
@@ -1309,8 +1400,10 @@ __global__ void __launch_bounds__(256) summarize_kernel(StepParams p) {
     const int nbody = p.nbody;
     const int first_root = p.nnodes - p.nuniv + 1;
     const int stride = gridDim.x * blockDim.x;
-    const int bottom = ld_relaxed(&p.st->bottom);
-    for (int c0 = bottom + (int)(blockIdx.x * blockDim.x + threadIdx.x); c0 <= p.nnodes; c0 += stride) {
+    int low;
+    const int cells = cells_to_sum(p, low);
+    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < cells; i += stride) {
+        const int c0 = cell_to_sum(p, low, i);
         // link's tag -1 - (cell children): only a cell without cell children starts here; the
         // others are summed by their last cell child (tag < -1), perhaps already (tag >= 0)
         if (p.count[c0 - nbody] != -1) continue;
@@ -1680,18 +1773,22 @@ void launch_bbox(const StepParams& p, int grid, cudaStream_t s) {
     else bbox_kernel<false><<<grid, 256, 0, s>>>(p);
 }
 // One bucketed completion: the bodies of `set` join the subtrees of the slots of the tree
-// built so far.  zero_counts: the new cells get bucket counters for a later pass.
-static void launch_bucket_pass(const StepParams& p, BuildPhase set, bool first, bool zero_counts, int sms,
+// built so far.  The last pass sums the subtrees it builds; before it, the new cells get bucket
+// counters for the next.
+static void launch_bucket_pass(const StepParams& p, BuildPhase set, bool first, bool last, bool ref, int sms,
                                cudaStream_t s) {
     const long long rest = (long long)p.nchunks * phase_bodies(set);
     const unsigned grid_rest = (unsigned)((rest + 255) / 256);
-    bucket_locate_kernel<<<grid_rest, 256, 0, s>>>(p, set, !first);
+    bucket_locate_kernel<<<grid_rest, 256, 0, s>>>(p, set, !first, last);
     // every cell of the tree so far: at most one per inserted body (1/16 of each chunk) plus
     // the roots
     const long long cells = (long long)p.nchunks * 16 + p.nuniv;
     bucket_alloc_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(p);
     bucket_scatter_kernel<<<grid_rest, 256, 0, s>>>(p, set);
-    bucket_build_kernel<<<kBucketBlocksPerSm * sms, 32 * kBucketWarps, 0, s>>>(p, zero_counts);
+    const int grid = kBucketBlocksPerSm * sms, threads = 32 * kBucketWarps;
+    if (!last) bucket_build_kernel<false, false><<<grid, threads, 0, s>>>(p);
+    else if (ref) bucket_build_kernel<true, true><<<grid, threads, 0, s>>>(p);
+    else bucket_build_kernel<true, false><<<grid, threads, 0, s>>>(p);
 }
 
 // The first phase (one body per chunk) of the multi-phase schedules: in shared memory (one
@@ -1705,14 +1802,15 @@ static void launch_first_phase(const StepParams& p, bool zero_counts, int top_ce
             p, kFirstPhase, zero_counts);
 }
 
-void launch_build(const StepParams& p, int phases, bool buckets, int sms, int top, int split, cudaStream_t s) {
+void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int sms, int top, int split,
+                  cudaStream_t s) {
     buckets = buckets && phases != 1;
     if (buckets && phases == 3) {
         // one lock phase (1/256 of each chunk), then the rest of the 1/16 sample as bucket
         // subtrees of that tree, then every other body as bucket subtrees of the sample's
         launch_first_phase(p, true, top, split, s);
-        launch_bucket_pass(p, kThreePhases[1], true, true, sms, s);
-        launch_bucket_pass(p, kBucketBodies, false, false, sms, s);
+        launch_bucket_pass(p, kThreePhases[1], true, false, ref, sms, s);
+        launch_bucket_pass(p, kBucketBodies, false, true, ref, sms, s);
         return;
     }
     const BuildPhase* sched = phases == 1 ? kOnePass : (phases == 5 ? kFivePhases : kThreePhases);
@@ -1726,7 +1824,7 @@ void launch_build(const StepParams& p, int phases, bool buckets, int sms, int to
         const long long bodies = (long long)p.nchunks * phase_bodies(sched[k]);
         build_kernel<<<(unsigned)((bodies + 255) / 256), 256, 0, s>>>(p, sched[k], buckets);
     }
-    if (buckets) launch_bucket_pass(p, kBucketBodies, true, false, sms, s);
+    if (buckets) launch_bucket_pass(p, kBucketBodies, true, true, ref, sms, s);
 }
 
 template <bool REF, bool PRECISE>
