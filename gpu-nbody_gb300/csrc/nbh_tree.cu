@@ -362,12 +362,12 @@ __device__ __forceinline__ unsigned short ld_shared_volatile(const unsigned shor
     return *reinterpret_cast<const volatile unsigned short*>(a);
 }
 
-// One sample's insertion into the shared tree; body_of(k): body of sample k.  Returns false once
+// One sample's insertion into the shared tree; place_of(k): position of sample k.  Returns false once
 // the tree has failed (more cells than it holds or a split too deep: 1; a wait that gave up: 2).
-template <class BodyOf>
+template <class PlaceOf>
 __device__ __forceinline__ bool shared_insert(const StepParams& p, unsigned short* slots, unsigned char* lvl,
                                               int* ncell, int* failed, int cap, int smp, const float4 bp,
-                                              const float4 rc, float radius, int& local_max, BodyOf body_of) {
+                                              const float4 rc, float radius, int& local_max, PlaceOf place_of) {
     int node = 0, depth = 1;
     float r = radius, cx = rc.x, cy = rc.y, cz = rc.z;
     int path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
@@ -413,7 +413,7 @@ __device__ __forceinline__ bool shared_insert(const StepParams& p, unsigned shor
             return true;
         }
         // split: the slot held sample `ch`; cells until the two separate
-        const float4 op = p.node4[body_of((int)ch)];
+        const float4 op = place_of((int)ch);
         int patch = -1, cur = node, cpath = path;
         for (;;) {
             ++depth;
@@ -488,11 +488,11 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
             if (b >= ck.z) continue;
             const float4 bp = p.node4[b];
             if (oct >= 0 && octant(rc.x, rc.y, rc.z, bp.x, bp.y, bp.z) != oct) continue;   // another block's octant
-            auto body_of = [&](int k) {
+            auto place_of = [&](int k) {
                 const int4 ok = p.chunks[c0 + k];
-                return ok.y + phase_offset(kFirstPhase, 0, c0 + k);
+                return p.node4[ok.y + phase_offset(kFirstPhase, 0, c0 + k)];
             };
-            if (!shared_insert(p, slots, lvl, &ncell, &failed, cap, smp, bp, rc, radius, local_max, body_of)) break;
+            if (!shared_insert(p, slots, lvl, &ncell, &failed, cap, smp, bp, rc, radius, local_max, place_of)) break;
         }
     }
     atomicMax(&depth_max, local_max);
@@ -1486,7 +1486,7 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 // The same arithmetic in the same order as the stages it replaces, so the same tree.
 //
 // Per cell of the shared tree: 8 slots, level, centre of mass, body count, offset in its
-// parent's range and parent.  A universe whose tree does not fit (close pairs make chains of
+// parent's range, parent, and the list of the cells by level.  A universe whose tree does not fit (close pairs make chains of
 // single-child cells) or goes too deep is left to the last block to finish, which builds such
 // universes one after another in global memory, through the lock insertion.
 // Measured, us, one launch / the stages: one sphere of 300 bodies 38 / 124, 1,000 52 / 132,
@@ -1494,14 +1494,29 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 // 134 / 227, 200 of 7,168 404 / 503: up to 7,168 bodies (what shared memory holds) from 8
 // universes on, up to 5,120 for fewer.
 constexpr int kSmallBodies = 7168, kSmallBodiesFew = 5120;
-constexpr size_t kSmallCellBytes = 8 * sizeof(unsigned short) + sizeof(float4) + 3 * sizeof(unsigned short) + 1;
+constexpr size_t kSmallCellBytes = 8 * sizeof(unsigned short) + sizeof(float4) + 4 * sizeof(unsigned short) + 1;
 int small_tree_max_bodies(int universes) { return universes >= 8 ? kSmallBodies : kSmallBodiesFew; }
-// Cells held for universes of at most `bodies` bodies (an octree of k bodies has about k / 2).
-static int small_tree_cells(int bodies) { return (bodies * 3 / 4 + 64) / 16 * 16; }
+// Universes of at most kSortedBodies bodies, a body per thread, are built by sorting the bodies'
+// paths below the root: kSortedLevels octants and the body's index in 64 bits, kept in the
+// place of the centres of mass until the tree stands.
+constexpr int kSortedBodies = 1024, kSortedIndexBits = 10, kSortedLevels = 18;
+static_assert(kSortedBodies <= kTopThreads && kSortedBodies <= 1 << kSortedIndexBits &&
+                  3 * kSortedLevels + kSortedIndexBits == 64,
+              "a path and an index");
+// Cells held for universes of at most `bodies` bodies (an octree of k bodies has about k / 2), with
+// room for the sorted paths (a power of two of them, 8 bytes each) in the centres' place.
+static int small_tree_cells(int bodies) {
+    int keys = 64;
+    while (keys < bodies && keys < kSortedBodies) keys *= 2;
+    const int cells = (bodies * 3 / 4 + 64) / 16 * 16;
+    return cells > keys / 2 ? cells : keys / 2;
+}
 static size_t small_tree_smem(int cells) { return (size_t)cells * kSmallCellBytes; }
 
 struct SmallShared {
     int status, ncell, failed, depth_max, gbase, last;
+    int level[kMaxDepth + 1];                        // first place of each level's cells in the list
+    int tie, sum[32];
     float lo[3][32], hi[3][32];
 };
 
@@ -1588,11 +1603,16 @@ template <bool REF, bool PRECISE>
 __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, int cap) {
     extern __shared__ __align__(16) unsigned char top_smem[];
     float4* const com = reinterpret_cast<float4*>(top_smem);
+    unsigned long long* const keys = reinterpret_cast<unsigned long long*>(com);
     unsigned short* const slots = reinterpret_cast<unsigned short*>(com + cap);      // [cap][8]
     unsigned short* const count = slots + (size_t)cap * 8;
     unsigned short* const off = count + cap;
     unsigned short* const par = off + cap;
-    unsigned char* const lvl = reinterpret_cast<unsigned char*>(par + cap);
+    unsigned short* const list = par + cap;
+    unsigned char* const lvl = reinterpret_cast<unsigned char*>(list + cap);
+    // during an insertion, the centres' place holds the bodies' positions (three quarters of a cell
+    // per body): a split reads one while its slot is locked
+    float* const pos = reinterpret_cast<float*>(com);
     __shared__ SmallShared S;
     const int u = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, warps = blockDim.x >> 5;
@@ -1604,6 +1624,7 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
         S.ncell = 1;                                   // local cell 0 is the root
         S.failed = 0;
         S.depth_max = 1;
+        S.tie = n < 2 || n > kSortedBodies;
         lvl[0] = 0;
     }
     for (int i = tid; i < cap * 4; i += blockDim.x) reinterpret_cast<unsigned*>(slots)[i] = 0xffffffffu;
@@ -1626,12 +1647,20 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
         for (int k = 0; k < 3; ++k) S.lo[k][wid] = v[k], S.hi[k][wid] = v[3 + k];
     __syncthreads();
     if (S.status) return;
-    float mn[3], mx[3];
+    if (wid == 0) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        mn[k] = S.lo[k][0], mx[k] = S.hi[k][0];
-        for (int w = 1; w < warps; ++w) mn[k] = fminf(mn[k], S.lo[k][w]), mx[k] = fmaxf(mx[k], S.hi[k][w]);
+        for (int k = 0; k < 3; ++k) {
+            float lo = lane < warps ? S.lo[k][lane] : FLT_MAX, hi = lane < warps ? S.hi[k][lane] : -FLT_MAX;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+            if (lane == 0) S.lo[k][0] = lo, S.hi[k][0] = hi;
+        }
     }
+    __syncthreads();
+    const float mn[3] = {S.lo[0][0], S.lo[1][0], S.lo[2][0]}, mx[3] = {S.hi[0][0], S.hi[1][0], S.hi[2][0]};
     float4 rc;
     float radius;
     root_box<PRECISE>(mn, mx, rc, radius);
@@ -1642,11 +1671,119 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
         p.arrive[root - nbody] = 0;
         p.clevel[root - nbody] = 0;
     }
+    // Build by sorting: every body's path of octants (the descent's arithmetic, no memory), sorted;
+    // then the cells follow from the octants that neighbours share, as in packed_subtrees.
+    // Larger universes, and those in which two bodies share all the octants of a path, take the
+    // lock insertion, whose time goes into waiting for locked slots.  The lock insertion against
+    // the sort, thousand cycles: 1,000 bodies 36 / 16; a radix sort of several keys per thread was
+    // no faster than the insertion (5,000 bodies 102 / 101), a bitonic one slower (190).
     int local_max = 1;
-    for (int k = tid; k < n; k += blockDim.x)
-        if (!shared_insert(p, slots, lvl, &S.ncell, &S.failed, cap, k, p.node4[first + k], rc, radius, local_max,
-                           [&](int o) { return first + o; }))
-            break;
+    if (n >= 2 && n <= kSortedBodies) {
+        int nk = 64;                                   // this universe's power of two
+        while (nk < n) nk *= 2;
+        unsigned long long key = ~0ull;
+        if (tid < n) {
+            const float4 q = p.node4[first + tid];
+            float r = radius, cx = rc.x, cy = rc.y, cz = rc.z;
+            key = 0;
+#pragma unroll
+            for (int l = 0; l < kSortedLevels; ++l) {
+                const int o = octant(cx, cy, cz, q.x, q.y, q.z);
+                key = (key << 3) | (unsigned)o;
+                const float h = r * 0.5f;
+                cx = __fadd_rn(__fsub_rn(cx, h), (o & 1) ? r : 0.0f);
+                cy = __fadd_rn(__fsub_rn(cy, h), (o & 2) ? r : 0.0f);
+                cz = __fadd_rn(__fsub_rn(cz, h), (o & 4) ? r : 0.0f);
+                r = h;
+            }
+            key = (key << kSortedIndexBits) | (unsigned)tid;
+        }
+        // bitonic sort: a key per thread; partners in other warps through shared memory
+        for (int k = 2; k <= nk; k <<= 1)
+            for (int o = k >> 1; o > 0; o >>= 1) {
+                unsigned long long other;
+                if (o >= 32) {
+                    __syncthreads();                   // the last exchange has been read
+                    if (tid < nk) keys[tid] = key;
+                    __syncthreads();
+                    other = tid < nk ? keys[tid ^ o] : 0ull;
+                } else {
+                    other = __shfl_xor_sync(0xffffffffu, key, o);
+                }
+                const bool low = ((tid & o) == 0) == ((tid & k) == 0);   // keeps the smaller
+                if (tid < nk && (other < key) == low) key = other;
+            }
+        __syncthreads();
+        if (tid < nk) keys[tid] = key;
+        __syncthreads();
+        // levels shared with the place before (-1 for the first); ties
+        auto shared_levels = [&](int i) {
+            if (i <= 0 || i >= n) return -1;
+            const unsigned long long x = (keys[i - 1] ^ keys[i]) >> kSortedIndexBits;
+            if (x == 0) S.tie = 1;
+            return (__clzll((long long)x) - kSortedIndexBits) / 3;
+        };
+        const int i = tid, cl = shared_levels(i), cr = shared_levels(i + 1);
+        const int made = i < n ? max(0, cr - cl) : 0;
+        int upto = made;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += t;
+        }
+        if (lane == 31) S.sum[wid] = upto;
+        __syncthreads();
+        int cells = upto - made, all = 0;              // cells before this place; in all
+        for (int w = 0; w < warps; ++w) {
+            cells += w < wid ? S.sum[w] : 0;
+            all += S.sum[w];
+        }
+        if (!S.tie && all <= cap) {
+            // cell of place i at level l: org[i] + l
+            short* const org = reinterpret_cast<short*>(count);
+            if (i < n) org[i] = (short)(cells - cl - 1);
+            __syncthreads();
+            if (i < n) {
+                auto digit = [&](int l) { return (int)(key >> (kSortedIndexBits + 3 * (kSortedLevels - 1 - l))) & 7; };
+                int outer = 0;                         // the cell at level cl that contains body i
+                if (cl >= 0) {
+                    // it starts at the first place with the same first cl octants
+                    const unsigned long long prefix = cl ? key >> (64 - 3 * cl) << (64 - 3 * cl) : 0ull;
+                    int lo = 0, hi = i;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (keys[mid] < prefix) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    outer = org[lo] + cl;
+                }
+                for (int l = cl + 1; l <= cr; ++l) {
+                    const int c = org[i] + l;
+                    lvl[c] = (unsigned char)l;
+                    if (l > 0) slots[(l == cl + 1 ? outer : c - 1) * 8 + digit(l - 1)] = (unsigned short)(kTopCell | c);
+                }
+                const int l = max(cl, cr);
+                slots[(cr > cl ? org[i] + cr : outer) * 8 + digit(l)] =
+                    (unsigned short)(key & ((1u << kSortedIndexBits) - 1u));
+                local_max = max(local_max, l + 1);
+            }
+            if (tid == 0) S.ncell = all;
+        }
+    }
+    __syncthreads();
+    if (S.tie || S.ncell == 1) {
+        // (a root of bodies alone is built again: the same)
+        for (int i = tid; i < cap * 4; i += blockDim.x) reinterpret_cast<unsigned*>(slots)[i] = 0xffffffffu;
+        for (int i = tid; i < n; i += blockDim.x) {
+            const float4 q = p.node4[first + i];
+            pos[3 * i] = q.x, pos[3 * i + 1] = q.y, pos[3 * i + 2] = q.z;
+        }
+        __syncthreads();
+        auto place_of = [&](int k) { return make_float4(pos[3 * k], pos[3 * k + 1], pos[3 * k + 2], 0.0f); };
+        for (int k = tid; k < n; k += blockDim.x)
+            if (!shared_insert(p, slots, lvl, &S.ncell, &S.failed, cap, k, place_of(k), rc, radius, local_max, place_of))
+                break;
+    }
     atomicMax(&S.depth_max, local_max);
     __syncthreads();
     const int nc = S.ncell;
@@ -1663,71 +1800,108 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
     __syncthreads();
     if (!S.failed) {
         const int gb = S.gbase;
-        // summarize, deepest level first (see sum_children), and link
+        // the cells by level (counting sort)
+        for (int i = tid; i <= kMaxDepth; i += blockDim.x) S.level[i] = 0;
+        __syncthreads();
+        for (int c = tid; c < nc; c += blockDim.x) atomicAdd(&S.level[lvl[c] + 1], 1);
+        __syncthreads();
+        if (tid < 32) {
+            int a0 = S.level[2 * lane + 1], a1 = S.level[2 * lane + 2];
+            int sum = a0 + a1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += t;
+            }
+            S.level[2 * lane + 1] = sum - a1;
+            S.level[2 * lane + 2] = sum;
+        }
+        __syncthreads();
+        for (int c = tid; c < nc; c += blockDim.x) {
+            const unsigned same = __match_any_sync(__activemask(), lvl[c]);
+            const int leader = __ffs((int)same) - 1;
+            int at = 0;
+            if (lane == leader) at = atomicAdd(&S.level[lvl[c]], __popc(same));
+            at = __shfl_sync(same, at, leader) + __popc(same & ((1u << lane) - 1u));
+            list[at] = (unsigned short)c;
+        }
+        __syncthreads();                               // S.level[l] is now the end of level l
+        // summarize, deepest level first, eight lanes per cell, a lane per slot (the sums of
+        // sum_children, in its order), and link
+        const int j = tid & 7;
+        const unsigned gmask = 0xffu << (lane & 24);
         for (int level = S.depth_max - 1; level >= 0; --level) {
-            for (int c = tid; c < nc; c += blockDim.x) {
-                if (lvl[c] != level) continue;
+            for (int i = (level ? S.level[level - 1] : 0) + (tid >> 3); i < S.level[level]; i += blockDim.x >> 3) {
+                const int c = list[i];
                 const int gc = c == 0 ? root : gb - c, k = gc - nbody;
-                const uint4 packed = reinterpret_cast<const uint4*>(slots)[c];
-                const unsigned w[4] = {packed.x, packed.y, packed.z, packed.w};
-                float4* const kb = p.kids4 + ((size_t)k << 3);
-                int* const ch8 = cell_child(p, gc);
-                int used = 0, cnt = 0;
+                const unsigned short v16 = slots[c * 8 + j];
+                const bool some = v16 != kTopNull;
+                const bool cell = some && (v16 & kTopCell);
+                const int l = v16 & 0x7fff;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                int bodies = 0, g = kNull;
+                if (cell) {
+                    q = com[l];
+                    bodies = count[l];
+                    g = gb - l;
+                } else if (some) {
+                    q = p.node4[first + v16];
+                    bodies = 1;
+                    g = first + v16;
+                }
+                const unsigned have = (__ballot_sync(gmask, some) >> (lane & 24)) & 0xffu;
+                int upto = bodies;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    const int t = __shfl_up_sync(gmask, upto, o, 8);
+                    if (j >= o) upto += t;
+                }
+                const int total = __shfl_sync(gmask, upto, 7, 8);
+                if (cell) {
+                    off[l] = (unsigned short)(upto - bodies);
+                    par[l] = (unsigned short)c;
+                    p.loff[g - nbody] = upto - bodies;
+                }
+                if (some) p.parent[g] = gc;
+                // children to the front (every lane has read its slot: the ballot above)
+                const unsigned below = (1u << j) - 1u;
+                const int at = some ? __popc(have & below) : __popc(have) + __popc(~have & below);
+                slots[c * 8 + at] = v16;
+                cell_child(p, gc)[at] = g;
+                if (some) p.kids4[((size_t)k << 3) + at] = q;
                 float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
                 double dm = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const unsigned short v16 = (unsigned short)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu);
-                    if (v16 == kTopNull) continue;
-                    int g;
-                    float4 q;
-                    if (v16 & kTopCell) {
-                        const int l = v16 & 0x7fff;
-                        g = gb - l;
-                        q = com[l];
-                        off[l] = (unsigned short)cnt;
-                        par[l] = (unsigned short)c;
-                        p.loff[g - nbody] = cnt;
-                        cnt += count[l];
-                    } else {
-                        g = first + v16;
-                        q = p.node4[g];
-                        ++cnt;
-                    }
-                    p.parent[g] = gc;
+                for (int t = 0; t < 8; ++t) {
+                    const float x = __shfl_sync(gmask, q.x, t, 8), y = __shfl_sync(gmask, q.y, t, 8);
+                    const float z = __shfl_sync(gmask, q.z, t, 8), w = __shfl_sync(gmask, q.w, t, 8);
+                    if (!((have >> t) & 1u)) continue;
                     if (PRECISE && c == 0) {
-                        dm += (double)q.w;
-                        dx += (double)q.x * (double)q.w;
-                        dy += (double)q.y * (double)q.w;
-                        dz += (double)q.z * (double)q.w;
+                        dm += (double)w;
+                        dx += (double)x * (double)w;
+                        dy += (double)y * (double)w;
+                        dz += (double)z * (double)w;
                     } else {
-                        cm = __fadd_rn(cm, q.w);
-                        sx = madd<REF>(q.x, q.w, sx);
-                        sy = madd<REF>(q.y, q.w, sy);
-                        sz = madd<REF>(q.z, q.w, sz);
+                        cm = __fadd_rn(cm, w);
+                        sx = madd<REF>(x, w, sx);
+                        sy = madd<REF>(y, w, sy);
+                        sz = madd<REF>(z, w, sz);
                     }
-                    slots[c * 8 + used] = v16;
-                    ch8[used] = g;
-                    kb[used] = q;
-                    ++used;
                 }
-                for (int j = used; j < 8; ++j) {
-                    slots[c * 8 + j] = kTopNull;
-                    ch8[j] = kNull;
-                    kb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j == 0) {
+                    float4 centre;
+                    if (PRECISE && c == 0) {
+                        centre = make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
+                    } else {
+                        const float inv = __fdiv_rn(1.0f, cm);
+                        centre = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
+                    }
+                    com[c] = centre;
+                    count[c] = (unsigned short)total;
+                    p.node4[gc] = centre;
+                    p.count[k] = total;
+                    p.clevel[k] = level;
                 }
-                float4 centre;
-                if (PRECISE && c == 0) {
-                    centre = make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
-                } else {
-                    const float inv = __fdiv_rn(1.0f, cm);
-                    centre = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
-                }
-                com[c] = centre;
-                count[c] = (unsigned short)cnt;
-                p.node4[gc] = centre;
-                p.count[k] = cnt;
-                p.clevel[k] = level;
             }
             __syncthreads();
         }

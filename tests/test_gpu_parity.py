@@ -921,3 +921,17 @@ def test_ordered_walk_is_the_per_level_walk_bit_for_bit(kw, n):
     g.load(*arrs)
     g.step()
     assert g.stats()["interactions"] == o.interactions
+
+
+@pytest.mark.parametrize("n", [32, 64, 65, 127, 512, 513, 700, 1024, 1025])
+def test_sorted_paths_build_the_staged_tree(n):
+    """The sort of the one-launch build at the powers of two it pads to and where it gives way to
+    the insertion, with two bodies closer than its paths resolve (which take the insertion) at
+    every other size."""
+    arrs = [a.copy() for a in plummer(n, seed=88)]
+    if n % 2:
+        for k in range(3):
+            arrs[k][5] = arrs[k][9] = np.float32(0.3)
+        arrs[0][9] = np.nextafter(np.float32(0.3), np.float32(1.0))
+    load = lambda g: g.load(*arrs)                   # noqa: E731
+    _assert_same_steps(_steps({"theta": 0.5}, load), _steps({"theta": 0.5, "build_phases": 3}, load))
