@@ -74,7 +74,7 @@ struct nbh_sim {
     int nchunks = 0, nwarps = 0, nitems64 = 0, nitems128 = 0;
     std::vector<int> h_ubody;
     // launch geometry
-    int grid_bbox = 0, grid_sum = 0, grid_sort = 0, grid_force = 0, grid_int = 0;
+    int grid_bbox = 0, grid_sum = 0, grid_sort = 0, grid_force = 0;
     // graph of one step
     cudaGraphExec_t exec = nullptr;
     // host mirrors
@@ -157,6 +157,11 @@ void drop_graph(nbh_sim* sim) {
     sim->exec = nullptr;
 }
 
+// Force work items of a vote width: 32-body items for widths 16 and 32, else 64 or 128.
+int nitems_for_vote(const nbh_sim* sim, int vote) {
+    return vote == 128 ? sim->nitems128 : (vote == 64 ? sim->nitems64 : sim->nwarps);
+}
+
 StepParams step_params(const nbh_sim* sim) {
     StepParams p{};
     p.node4 = sim->node4;
@@ -181,8 +186,10 @@ StepParams step_params(const nbh_sim* sim) {
     p.buckets = sim->buckets;
     p.bwork = sim->bwork;
     p.bstack = sim->bstack;
-    p.item_order = sim->item_order;
-    p.item_cost = sim->item_cost;
+    // up to four groups per SM all start at once, in any order
+    const bool ordered = nitems_for_vote(sim, sim->cfg.vote_width) > 4 * sim->sms;
+    p.item_order = ordered ? sim->item_order : nullptr;
+    p.item_cost = ordered ? sim->item_cost : nullptr;
     p.st = sim->st;
     p.ubody = sim->ubody;
     p.ubox = sim->ubox;
@@ -205,11 +212,6 @@ StepParams step_params(const nbh_sim* sim) {
     p.G = c.G;
     p.precise = c.precise;
     return p;
-}
-
-// Force work items of a vote width: 32-body items for widths 16 and 32, else 64 or 128.
-int nitems_for_vote(const nbh_sim* sim, int vote) {
-    return vote == 128 ? sim->nitems128 : (vote == 64 ? sim->nitems64 : sim->nwarps);
 }
 
 // The work-item order belongs to one item table (one vote width): start it over (index
@@ -271,10 +273,9 @@ void enqueue_step(nbh_sim* sim, bool timed, cudaEvent_t vel_acc_ready = nullptr,
     } else {
         launch_force(p, sim->cfg.vote_width, ref, sim->theta_active, sim->grid_force, sim->force_threads, s);
     }
-    // the next step hands out the longest walks first
-    launch_item_order(sim->item_cost, nitems_for_vote(sim, sim->cfg.vote_width), sim->item_order, s);
     if (timed) cudaEventRecord(sim->ev[5], s);
-    launch_integrate(p, ref, sim->grid_int, s);
+    // the next step hands out the longest walks first
+    launch_integrate(p, ref, p.item_order ? nitems_for_vote(sim, sim->cfg.vote_width) : 0, sim->item_order, s);
     if (timed) cudaEventRecord(sim->ev[6], s);
 }
 
@@ -312,7 +313,6 @@ int set_geometry(nbh_sim* sim) {
     sim->grid_sum = std::max(1, (sim->nbody + 255) / 256);
     sim->grid_sort = std::max(1, std::min(occ_sort * sms, (sim->ncells + 255) / 256));
     sim->grid_force = std::max(1, occ_force * sms);
-    sim->grid_int = std::max(1, std::min((sim->nbody + 255) / 256, 4 * sms));
     return NBH_OK;
 }
 

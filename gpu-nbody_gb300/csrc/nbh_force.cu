@@ -1112,88 +1112,6 @@ void launch_force(const StepParams& p, int vote, bool ref, bool feat, int grid, 
     }
 }
 
-// Order of the force work items for the next step: longest walks first (longest-
-// processing-time first), so the few long walks -- bodies near a dense centre, or small
-// per-body angles -- start early instead of running alone at the end of the launch.  A
-// counting sort by cost class, descending: four classes per power of two (the two bits
-// below the leading one), so that items of one class differ by at most 19 %; within a
-// class the order is arbitrary.  One block; warp-aggregated shared-memory atomics.
-constexpr int kOrderThreads = 1024;
-constexpr int kOrderClasses = 128;
-__device__ __forceinline__ int cost_class(int c) {
-    c = max(c, 1);
-    const int e = 31 - __clz(c);
-    const int frac = e >= 2 ? (c >> (e - 2)) & 3 : (c << (2 - e)) & 3;
-    return 4 * e + frac;
-}
-__global__ void __launch_bounds__(kOrderThreads) item_order_kernel(const int* __restrict__ cost, int nitems,
-                                                                   int* order) {
-    __shared__ int cnt[kOrderClasses], off[kOrderClasses];
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    if (threadIdx.x < kOrderClasses) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    // four items per thread per round: their cost loads are in flight together
-    constexpr int kU = 4;
-    const int stride = blockDim.x;
-    for (int i0 = 0; i0 < nitems; i0 += kU * stride) {
-        int c[kU];
-#pragma unroll
-        for (int k = 0; k < kU; ++k) {
-            const int i = i0 + k * stride + threadIdx.x;
-            c[k] = i < nitems ? cost[i] : -1;
-        }
-#pragma unroll
-        for (int k = 0; k < kU; ++k) {
-            const bool v = c[k] >= 0;
-            const int cls = v ? cost_class(c[k]) : -1;
-            const unsigned grp = __match_any_sync(0xffffffffu, cls);
-            if (v && lane == __ffs(grp) - 1) atomicAdd(&cnt[cls], __popc(grp));
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        // first position of each class, largest costs first: lane l holds classes
-        // 127 - 4l .. 124 - 4l; a warp scan of the lanes' sums
-        static_assert(kOrderClasses == 128, "four classes per lane");
-        const int c0 = kOrderClasses - 1 - 4 * lane;
-        const int n0 = cnt[c0], n1 = cnt[c0 - 1], n2 = cnt[c0 - 2], n3 = cnt[c0 - 3];
-        const int mine = n0 + n1 + n2 + n3;
-        int incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int base = incl - mine;
-        off[c0] = base;
-        off[c0 - 1] = base + n0;
-        off[c0 - 2] = base + n0 + n1;
-        off[c0 - 3] = base + n0 + n1 + n2;
-    }
-    __syncthreads();
-    for (int i0 = 0; i0 < nitems; i0 += kU * stride) {
-        int c[kU];
-#pragma unroll
-        for (int k = 0; k < kU; ++k) {
-            const int i = i0 + k * stride + threadIdx.x;
-            c[k] = i < nitems ? cost[i] : -1;
-        }
-#pragma unroll
-        for (int k = 0; k < kU; ++k) {
-            const int i = i0 + k * stride + threadIdx.x;
-            const bool v = c[k] >= 0;
-            const int cls = v ? cost_class(c[k]) : -1;
-            const unsigned grp = __match_any_sync(0xffffffffu, cls);
-            const int leader = __ffs(grp) - 1;
-            int base = 0;
-            if (v && lane == leader) base = atomicAdd(&off[cls], __popc(grp));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (v) order[base + __popc(grp & lt)] = i;
-        }
-    }
-}
-
 __global__ void item_order_reset_kernel(int nitems, int* order, int* cost) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nitems; i += gridDim.x * blockDim.x) {
         order[i] = i;
@@ -1201,9 +1119,6 @@ __global__ void item_order_reset_kernel(int nitems, int* order, int* cost) {
     }
 }
 
-void launch_item_order(const int* cost, int nitems, int* order, cudaStream_t s) {
-    if (nitems > 0) item_order_kernel<<<1, kOrderThreads, 0, s>>>(cost, nitems, order);
-}
 void launch_item_order_reset(int nitems, int* order, int* cost, cudaStream_t s) {
     if (nitems > 0) item_order_reset_kernel<<<(nitems + 255) / 256, 256, 0, s>>>(nitems, order, cost);
 }

@@ -28,10 +28,10 @@ void launch_summarize(const StepParams& p, bool ref, int grid, cudaStream_t s);
 void launch_sort(const StepParams& p, int grid, cudaStream_t s);
 void launch_force(const StepParams& p, int vote, bool ref, bool feat, int grid, int threads, cudaStream_t s);
 bool force_geometry_valid(int vote, int threads, int cap);
-// Work-item order of the force launches: longest walks first, from the last launch's costs.
-void launch_item_order(const int* cost, int nitems, int* order, cudaStream_t s);
 void launch_item_order_reset(int nitems, int* order, int* cost, cudaStream_t s);
-void launch_integrate(const StepParams& p, bool ref, int grid, cudaStream_t s);
+// items > 0: also the work-item order of the next force launch, longest walks first, from the last
+// launch's costs (p.item_cost), into `order`.
+void launch_integrate(const StepParams& p, bool ref, int items, int* order, cudaStream_t s);
 
 void launch_pack(int n, const float* soa, int mask, float4* node4, float4* vel, float4* acc, int grid,
                  cudaStream_t s);
