@@ -59,6 +59,8 @@ struct nbh_sim {
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
     int top_cells = 0;             // cells of each block's shared tree for these universes
+    int top_direct = 0;            // cells of each block's tree when the blocks build the whole 1/16
+                                   // sample (universes small enough for it; 0: 1/256 of the bodies)
     int top_split = 0;             // in use: 0 global locks, 1 or 8 shared-memory blocks per universe
                                    // (from top_phase and the universes, or the tuner's choice)
     int4* buckets = nullptr;       // bucketed build: nbody records
@@ -91,6 +93,14 @@ struct nbh_sim {
 };
 
 namespace {
+
+// Universes of at most this many 1/16 samples (32,768 bodies) have the sample built in shared
+// memory as one phase, not 1/256 there and the rest by a bucketed pass: build of 16,384 bodies 98 ->
+// 84 us, 4 x 30,000 141 -> 127, 256 x 16,384 724 -> 660.  Beyond, the one block's chain of lock
+// rounds takes longer than the pass it saves (40,000 bodies 119 -> 128 us, 8 x 60,000 204 -> 216),
+// unless the pass is that of many universes: from 1M bodies in all the limit is twice as high
+// (256 of 1K-64K bodies 668 -> 617 us, 32 x 60,000 414 -> 384).
+constexpr int kDirectSamples = 2048, kDirectManyChunks = 4096;
 
 thread_local std::string g_create_error;
 
@@ -239,7 +249,7 @@ void enqueue_tree(nbh_sim* sim, const StepParams& p, bool timed = false) {
     launch_bbox(p, sim->grid_bbox, s);
     if (timed) cudaEventRecord(sim->ev[1], s);
     launch_build(p, ref, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
-                 sim->top_split, s);
+                 sim->top_split, sim->top_split ? sim->top_direct : 0, s);
     launch_link(p, sim->grid_sum, s);
     if (timed) cudaEventRecord(sim->ev[2], s);
     launch_summarize(p, ref, sim->grid_sum, s);
@@ -665,6 +675,8 @@ int nbh_load_batch(nbh_sim* sim, int32_t nuniv, const int32_t* counts, const flo
     else if (sim->top_phase == 1) sim->top_split = 1;
     else if (sim->top_phase == 3) sim->top_split = 8;
     else sim->top_split = max_chunks <= 512 ? 1 : (max_chunks <= 8192 ? 8 : 0);
+    const int direct = (int)chunks.size() >= kDirectManyChunks ? 2 * kDirectSamples : kDirectSamples;
+    sim->top_direct = sim->top_phase == 0 && max_chunks * 16 <= direct ? top_build_cells(max_chunks * 16) : 0;
     for (int u = 0; u < nuniv; ++u)
         for (int s = sim->h_ubody[u]; s < sim->h_ubody[u + 1]; s += 64) warps.push_back(make_int2(s, u));
     const int nw64 = (int)warps.size() - nw32;

@@ -13,7 +13,9 @@ void launch_bbox(const StepParams& p, int grid, cudaStream_t s);
 // top > 0: the first phase of a multi-phase schedule builds in shared memory, `split` (1 or
 // 8) blocks per universe holding `top` cells each (for universes of at most
 // top_build_max_samples() chunks; top_build_cells() sizes it); 0: through the global locks
-void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int sms, int top, int split,
+// direct > 0: with three phases and buckets, the blocks build the whole 1/16 sample (`direct` cells
+// each) and only the last bucketed pass follows
+void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int sms, int top, int split, int direct,
                   cudaStream_t s);
 // All tree stages of `universes` universes of at most small_tree_max_bodies() bodies each, one block per
 // universe (max_bodies: bodies of the largest).

@@ -446,8 +446,8 @@ __device__ __forceinline__ bool shared_insert(const StepParams& p, unsigned shor
     }
 }
 
-__global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bool zero_counts, int cap,
-                                                                 int split) {
+__global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, BuildPhase phase,
+                                                                 bool zero_counts, int cap, int split) {
     extern __shared__ __align__(16) unsigned char top_smem[];
     unsigned short* slots = reinterpret_cast<unsigned short*>(top_smem);          // [cap][8]
     unsigned char* lvl = top_smem + (size_t)cap * 8 * sizeof(unsigned short);
@@ -460,7 +460,8 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
     const int u = split == 8 ? (int)(blockIdx.x >> 3) : (int)blockIdx.x;   // universe
     const int oct = split == 8 ? (int)(blockIdx.x & 7) : -1;   // this block's octant of the root (-1: all)
     const int nbody = p.nbody;
-    const int nsamp = (p.ubody[u + 1] - p.ubody[u] + 255) / 256;    // chunks of universe u
+    const int per = phase_bodies(phase);                                    // samples of a chunk
+    const int nsamp = (p.ubody[u + 1] - p.ubody[u] + 255) / 256 * per;      // of universe u
     if (threadIdx.x == 0) {
         int lo = 0, hi = p.nchunks;              // first chunk of universe u
         while (lo < hi) {
@@ -479,19 +480,21 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
     const int root = p.nnodes - u;
     const float4 rc = p.node4[root];
     const float radius = p.uradius[u];
+    // body of sample k, -1 past the universe's end
+    auto body_of = [&](int k) {
+        const long long ci = c0 + k / per;
+        const int4 ck = p.chunks[ci];
+        const int b = ck.y + phase_offset(phase, k % per, ci);
+        return b < ck.z ? b : -1;
+    };
     int local_max = 1;
     if (!failed) {
         for (int smp = threadIdx.x; smp < nsamp; smp += blockDim.x) {
-            const long long ci = c0 + smp;
-            const int4 ck = p.chunks[ci];
-            const int b = ck.y + phase_offset(kFirstPhase, 0, ci);
-            if (b >= ck.z) continue;
+            const int b = body_of(smp);
+            if (b < 0) continue;
             const float4 bp = p.node4[b];
             if (oct >= 0 && octant(rc.x, rc.y, rc.z, bp.x, bp.y, bp.z) != oct) continue;   // another block's octant
-            auto place_of = [&](int k) {
-                const int4 ok = p.chunks[c0 + k];
-                return p.node4[ok.y + phase_offset(kFirstPhase, 0, c0 + k)];
-            };
+            auto place_of = [&](int k) { return p.node4[body_of(k)]; };
             if (!shared_insert(p, slots, lvl, &ncell, &failed, cap, smp, bp, rc, radius, local_max, place_of)) break;
         }
     }
@@ -503,10 +506,8 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
         int lm = 1, waits = 0, misses = 0;
         const float4 rc0 = p.node4[root];
         for (int smp = threadIdx.x; smp < nsamp; smp += blockDim.x) {
-            const long long ci = c0 + smp;
-            const int4 ck = p.chunks[ci];
-            const int b = ck.y + phase_offset(kFirstPhase, 0, ci);
-            if (b >= ck.z) continue;
+            const int b = body_of(smp);
+            if (b < 0) continue;
             const float4 bp = p.node4[b];
             if (oct >= 0 && octant(rc0.x, rc0.y, rc0.z, bp.x, bp.y, bp.z) != oct) continue;   // another block's
             if (!lock_insert(p, b, u, zero_counts, lm, waits, misses)) break;
@@ -536,12 +537,7 @@ __global__ void __launch_bounds__(kTopThreads) top_build_kernel(StepParams p, bo
         const unsigned short v = slots[i];
         int g = kNull;
         if (v != kTopNull) {
-            if (v & kTopCell) {
-                g = gb - (v & 0x7fff);
-            } else {
-                const long long ci = c0 + v;
-                g = p.chunks[ci].y + phase_offset(kFirstPhase, 0, ci);
-            }
+            g = v & kTopCell ? gb - (v & 0x7fff) : body_of(v);
         }
         const int gc = c == 0 ? root : gb - c;
         cell_child(p, gc)[i & 7] = g;
@@ -1969,16 +1965,24 @@ static void launch_bucket_pass(const StepParams& p, BuildPhase set, bool first, 
 // block per universe) when `top`, else through the global locks.
 static void launch_first_phase(const StepParams& p, bool zero_counts, int top_cells, int split, cudaStream_t s) {
     if (top_cells > 0)
-        top_build_kernel<<<split * p.nuniv, kTopThreads, top_build_smem(top_cells), s>>>(p, zero_counts, top_cells,
-                                                                                       split);
+        top_build_kernel<<<split * p.nuniv, kTopThreads, top_build_smem(top_cells), s>>>(p, kFirstPhase, zero_counts,
+                                                                                       top_cells, split);
     else
         build_kernel<<<(unsigned)((p.nchunks * (long long)phase_bodies(kFirstPhase) + 255) / 256), 256, 0, s>>>(
             p, kFirstPhase, zero_counts);
 }
 
-void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int sms, int top, int split,
+void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int sms, int top, int split, int direct,
                   cudaStream_t s) {
     buckets = buckets && phases != 1;
+    if (buckets && phases == 3 && direct > 0) {
+        // the whole 1/16 sample in shared memory, then every other body as bucket subtrees: five
+        // launches fewer than below for small universes
+        top_build_kernel<<<split * p.nuniv, kTopThreads, top_build_smem(direct), s>>>(p, BuildPhase{16, 0}, true, direct,
+                                                                                    split);
+        launch_bucket_pass(p, kBucketBodies, true, true, ref, sms, s);
+        return;
+    }
     if (buckets && phases == 3) {
         // one lock phase (1/256 of each chunk), then the rest of the 1/16 sample as bucket
         // subtrees of that tree, then every other body as bucket subtrees of the sample's

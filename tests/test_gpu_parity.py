@@ -843,6 +843,31 @@ def test_one_launch_tree_hands_over_what_does_not_fit(universes):
     _assert_same_steps(_steps(kw, load), _steps({**kw, "build_phases": 1}, load))
 
 
+@pytest.mark.parametrize("counts", [[5121], [16384], [32768], [32769], [30000, 1, 260, 7169, 17],
+                                    [1000] * 40 + [20011], [65536] * 16, [65537] + [65000] * 16], ids=lambda c: f"{len(c)}x{max(c)}")
+def test_sample_built_in_shared_memory(counts):
+    """Mid-size universes build their 1/16 sample in one block: the lock phases' tree bit for bit, at
+    the edges of the range (5,120 bodies take one launch, 32,769 a smaller sample)."""
+    parts = [plummer(c, seed=60 + i) for i, c in enumerate(counts)]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    load = lambda g: g.load_batch(counts, *cat)      # noqa: E731
+    _assert_same_steps(_steps({"theta": 0.5}, load), _steps({"theta": 0.5, "build_phases": 1}, load))
+
+
+def test_sample_that_does_not_fit_shared_memory():
+    """Chains between the sample's close pairs outgrow the block's cells: that universe's sample goes
+    through the locks, the other stays in shared memory."""
+    pairs = _close_pairs(20000, 4000, 91)
+    order = np.arange(20000)                         # the halves of a pair 16 apart: both or neither sampled
+    order[:8000] = order[:8000].reshape(-1, 16, 2).transpose(0, 2, 1).reshape(-1)
+    parts = [[v[order] for v in pairs], plummer(9000, seed=61)]
+    counts = [p[0].size for p in parts]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    load = lambda g: g.load_batch(counts, *cat)      # noqa: E731
+    kw = {"theta": 0.5, "pool_factor": 8.0}
+    _assert_same_steps(_steps(kw, load), _steps({**kw, "build_phases": 1}, load))
+
+
 def test_one_launch_tree_and_staged_tree_in_turn():
     """The tuner may move a small universe from the one launch to the stages between steps."""
     n = 3000
