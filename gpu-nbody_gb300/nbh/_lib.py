@@ -138,6 +138,7 @@ SIGNATURES = {
     "nbh_read_theta": (C.c_int, [_P, _P]),
     "nbh_force_probe": (C.c_int, [_P, _P, _P, _P, _P, _P, C.POINTER(C.c_int64)]),
     "nbh_theta_features": (C.c_int, [_P, _P, C.c_int32]),
+    "nbh_mlp_normalize": (C.c_int, [_P, C.c_int32, C.c_float, _P, _P, _P]),
     "nbh_mlp_train": (C.c_int, [C.c_int32, _P, _P, _P, C.c_int32, C.c_float, C.c_int32, C.c_float, _F]),
     "nbh_mlp_grad": (C.c_int, [C.c_int32, _P, _P, _P, C.c_int32, C.c_float, _P, _F]),
     "nbh_mlp_forward": (C.c_int, [C.c_int32, _P, _P, C.c_int32, _P]),

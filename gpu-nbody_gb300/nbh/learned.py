@@ -102,13 +102,27 @@ def init_params(seed=0):
     return p.astype(np.float32)
 
 
+def _normalize(X, std_floor):
+    """(mean, std, (X - mean) / std) over the rows, std at least std_floor."""
+    plain = X.ndim == 2 and X.shape[1] == 12 and 0 < X.shape[0] < 2**31 and X.flags.c_contiguous
+    if plain and np.isscalar(std_floor) and std_floor == std_floor:
+        # natively, the same sums in the same order
+        mean, std, Xn = np.empty(12, np.float32), np.empty(12, np.float32), np.empty_like(X)
+        L.check(L.load().nbh_mlp_normalize(X.ctypes.data, X.shape[0], float(std_floor), mean.ctypes.data,
+                                           std.ctypes.data, Xn.ctypes.data))
+        if np.isfinite(std).all() and (std > 0).all():
+            return mean, std, Xn
+    # other shapes, orders and per-column floors; zeros and infinities with numpy's warnings
+    mean = X.mean(0).astype(np.float32)
+    std = np.maximum(X.std(0), std_floor).astype(np.float32)
+    return mean, std, np.ascontiguousarray((X - mean) / std, dtype=np.float32)
+
+
 def train(X, Y, quantile=0.2, iters=1500, lr=3e-3, seed=0, device=0, std_floor=0.05):
     """Normalise the features and fit the MLP on the device.  Returns the model dict."""
     X = np.asarray(X, dtype=np.float32)
     Y = np.asarray(Y, dtype=np.float32)
-    mean = X.mean(0).astype(np.float32)
-    std = np.maximum(X.std(0), std_floor).astype(np.float32)
-    Xn = np.ascontiguousarray((X - mean) / std, dtype=np.float32)
+    mean, std, Xn = _normalize(X, std_floor)
     p = init_params(seed)
     loss = C.c_float()
     L.check(L.load().nbh_mlp_train(device, p.ctypes.data, Xn.ctypes.data, Y.ctypes.data, Xn.shape[0],

@@ -370,6 +370,10 @@ int nbh_mlp_grad(int32_t device, const float* params, const float* X, const floa
                  float quantile, float* grad, float* loss);
 int nbh_mlp_forward(int32_t device, const float* params, const float* X, int32_t n, float* y);
 
+/* Normalises raw features X[n*12] on the host: per column the mean and the standard deviation
+ * (at least std_floor), sums in FP32 row after row, and Xn = (X - mean) / std. */
+int nbh_mlp_normalize(const float* X, int32_t n, float std_floor, float* mean, float* std, float* Xn);
+
 /* Same FP64 direct sum as nbh_direct_f64, for callers that cannot allocate device memory
  * while they run (an application whose device memory is handed out up front by its own pool
  * or budget, or a time-critical loop in which cudaMalloc/cudaFree would synchronise the

@@ -4,6 +4,7 @@ import os
 import sys
 
 import numpy as np
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 if ROOT not in sys.path:
@@ -67,3 +68,29 @@ def test_p99_ratio_interval_of_paired_errors():
     point = np.percentile(el, 99, axis=1).mean() / np.percentile(ep, 99, axis=1).mean()
     lo, hi = bench._p99_ratio_interval(el, ep, np)
     assert lo < point < hi and hi - lo < 0.2
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 1000])
+def test_feature_normalisation(n):
+    """Row after row in FP32; other memory orders and a column that divides by zero as in numpy."""
+    from nbh import learned
+    r = np.random.default_rng(n)
+    X = (r.standard_normal((n, 12)) * np.exp(r.uniform(-4, 4, 12)) + 3).astype(np.float32)
+    X[:, 5] = 2.0
+    s = np.zeros(12, np.float32)
+    for row in X:
+        s += row
+    mean = s / np.float32(n)
+    s[:] = 0
+    for row in (X - mean) * (X - mean):
+        s += row
+    std = np.maximum(np.sqrt(s / np.float32(n)), np.float32(0.05))
+    got = learned._normalize(X, 0.05)
+    for a, b in zip(got, (mean, std, (X - mean) / std)):
+        assert a.dtype == np.float32 and a.flags.c_contiguous
+        np.testing.assert_array_equal(a, b)
+    other = learned._normalize(np.asfortranarray(X), 0.05)       # sums in another order
+    bound = n * 2.0 ** -24 * np.abs(X).sum(0) / n                # of either order's sum
+    assert (np.abs(other[0] - mean) <= 2 * bound).all() and other[2].flags.c_contiguous
+    with np.errstate(invalid="ignore", divide="ignore"):
+        assert np.isnan(learned._normalize(X, 0.0)[2][:, 5]).all()
