@@ -41,8 +41,9 @@ DEFAULT_VOTE = 64                   # libnbh's default vote width (nbh_config_de
 
 
 def graph_launches(build_phases=5, build_buckets=1):
-    """Kernels in one fixed-angle step graph: bbox, the build's launches, link, summarize,
-    sort, force, the work-item order of the next force launch, integrate.  The build is
+    """Kernels of one fixed-angle step with the work-item order of the next force launch as a
+    launch of its own: bbox, the build's launches, link, summarize, sort, force, work-item
+    order, integrate.  The build is
     `build_phases` lock phases, or with the bucketed completion: five phases -> the three
     lock phases of the 1/16 sample and one bucketed pass (locate, alloc, scatter, subtree
     build); three phases -> one lock phase (1/256) and two bucketed passes."""
@@ -53,6 +54,23 @@ def graph_launches(build_phases=5, build_buckets=1):
     else:
         build = 1 + 2 * 4
     return 7 + build
+
+
+def step_launches(counts, tune=None):
+    """Kernels in one fixed-angle step graph of universes of `counts` bodies: the work-item order
+    is part of the integrate launch; small universes build their tree in one launch, mid-size
+    ones the whole 1/16 sample in the first phase (include/nbh.h, top_phase)."""
+    phases, buckets, top = ((3, 1, 1) if tune is None else
+                            (tune["build_phases"], tune["build_buckets"], tune["top_phase"]))
+    largest, chunks = max(counts), sum((c + 255) // 256 for c in counts)
+    if (phases, buckets, top) == (3, 1, 1):
+        if largest <= (7168 if len(counts) >= 8 else 5120):
+            return 3 + (len(counts) > 1)      # (step counter of a batch,) tree, force, integrate
+        if largest <= (65536 if chunks >= 4096 else 32768):
+            return graph_launches(3, 1) - 1 - 4
+    return graph_launches(phases, buckets) - 1
+
+
 FLOPS_PER_INTERACTION = 20          # 3 sub, 3 fma (d^2+eps^2), rsqrt, 3 mul, 3 fma, ~7 more
 HBM_FALLBACK_GBS = 6800.0
 # DRAM bytes (read + write) of one force launch (vote width 64) on the 1,048,576-body
@@ -296,7 +314,7 @@ def _config(args, nbodies=None, counts=None):
     if counts is not None:
         c.update({"universes": len(counts), "min_universe": int(min(counts)), "max_universe": int(max(counts))})
     if getattr(args, "force_list", 0):
-        c["force_walk"] = "list" if args.force_list == 1 else "per-visit"
+        c["force_walk"] = "list" if args.force_list == 1 else "ordered"
     return c
 
 
@@ -399,7 +417,7 @@ def main():
     ap.add_argument("--stack-cap", type=int, default=0,
                     help="stack entries per vote group of a --profile-only run (0: the library default)")
     ap.add_argument("--force-list", type=int, default=0, choices=(0, 1, 2),
-                    help="nbh_config.force_list: 1 the list walk, 2 the per-visit walk, 0 the library "
+                    help="nbh_config.force_list: 1 the list walk, 2 the ordered walk, 0 the library "
                          "default (the list walk except in precise mode)")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
@@ -666,8 +684,7 @@ def main():
                     "d2h_bytes_per_step": 36 * n, "wall_ms_per_step": wall_ms,
                     "path": "nbh_step_io: pinned host arrays in, one step, pinned host arrays out, one wait",
                     "three_calls": e2e_three},
-            "gpu_launches": graph_launches(**({"build_phases": tune["build_phases"], "build_buckets": tune["build_buckets"]}
-                                              if tune else {})) * args.steps,
+            "gpu_launches": step_launches([n] if counts is None else [int(c) for c in counts], tune) * args.steps,
             "clocks": clock_info,
             "cpu_baseline": cpu,
             "learned_theta": learned,

@@ -59,8 +59,8 @@ struct nbh_sim {
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
     int top_cells = 0;             // cells of each block's shared tree for these universes
-    int top_direct = 0;            // cells of each block's tree when the blocks build the whole 1/16
-                                   // sample (universes small enough for it; 0: 1/256 of the bodies)
+    int top_direct = 0;            // cells of the block's tree where one block per universe builds the
+                                   // whole 1/16 sample (small enough universes; 0: 1/256 of the bodies)
     int top_split = 0;             // in use: 0 global locks, 1 or 8 shared-memory blocks per universe
                                    // (from top_phase and the universes, or the tuner's choice)
     int4* buckets = nullptr;       // bucketed build: nbody records
@@ -249,7 +249,7 @@ void enqueue_tree(nbh_sim* sim, const StepParams& p, bool timed = false) {
     launch_bbox(p, sim->grid_bbox, s);
     if (timed) cudaEventRecord(sim->ev[1], s);
     launch_build(p, ref, sim->build_phases, sim->build_buckets, sim->sms, sim->top_split ? sim->top_cells : 0,
-                 sim->top_split, sim->top_split ? sim->top_direct : 0, s);
+                 sim->top_split, sim->top_split == 1 ? sim->top_direct : 0, s);
     launch_link(p, sim->grid_sum, s);
     if (timed) cudaEventRecord(sim->ev[2], s);
     launch_summarize(p, ref, sim->grid_sum, s);
@@ -580,7 +580,7 @@ int nbh_create(const nbh_config* cfg_in, nbh_sim** out) {
     sim->build_phases = cfg.build_phases ? cfg.build_phases : 3;
     sim->build_buckets = cfg.build_buckets != 2;
     sim->top_phase = cfg.top_phase;
-    // precise mode keeps the reference's order of accumulation (the per-visit walk) unless asked
+    // precise mode keeps the reference's order of accumulation (the ordered walk) unless asked
     sim->force_list = cfg.force_list == 1 || (cfg.force_list == 0 && !cfg.precise);
     sim->sms = prop.multiProcessorCount;
     if ((e = cudaSetDevice(cfg.device)) != cudaSuccess ||
@@ -676,7 +676,7 @@ int nbh_load_batch(nbh_sim* sim, int32_t nuniv, const int32_t* counts, const flo
     else if (sim->top_phase == 3) sim->top_split = 8;
     else sim->top_split = max_chunks <= 512 ? 1 : (max_chunks <= 8192 ? 8 : 0);
     const int direct = (int)chunks.size() >= kDirectManyChunks ? 2 * kDirectSamples : kDirectSamples;
-    sim->top_direct = sim->top_phase == 0 && max_chunks * 16 <= direct ? top_build_cells(max_chunks * 16) : 0;
+    sim->top_direct = max_chunks * 16 <= direct ? top_build_cells(max_chunks * 16) : 0;
     for (int u = 0; u < nuniv; ++u)
         for (int s = sim->h_ubody[u]; s < sim->h_ubody[u + 1]; s += 64) warps.push_back(make_int2(s, u));
     const int nw64 = (int)warps.size() - nw32;

@@ -75,7 +75,7 @@ struct StepParams {
     float4* kpos;        // Kahan compensation of positions (precise mode), may be null
     float4* kvel;        // Kahan compensation of velocities (precise mode), may be null
     int* child;          // 8 * ncells
-    float4* kids4;       // 8 * ncells: node records of each cell's children (slot order)
+    float4* kids4;       // 8 * ncells: node records of each cell's children (slot order, the compacted ones only)
     int* count;          // ncells
     int* start;          // ncells: first depth-first position of each cell
     int* loff;           // ncells: offset of a cell inside its parent's depth-first range

@@ -105,16 +105,21 @@ typedef struct nbh_config {
                               eight (one per octant of the root), 2 never (global locks);
                               0 (default): one block up to 512 * 256 bodies per universe,
                               eight up to 8192 * 256, the global locks above (the measured
-                              fastest); nbh_autotune times all three where possible */
+                              fastest); nbh_autotune times all three where possible.  One
+                              block per universe builds the whole 1/16 sample of the 3-phase
+                              bucketed schedule where no universe has more than 128 * 256
+                              bodies (256 * 256 in batches of 4096 * 256 and more).
+                              With build_phases, build_buckets and top_phase all 0, universes
+                              of at most 5120 bodies (7168 each from 8 universes on) take one
+                              launch for the whole tree, one block per universe */
     int32_t force_list;    /* the whole-warp walks (vote width 32, 64 or 128; FMA arithmetic;
                               fixed or per-body angle): 1 decides each tested child on its own
                               lane (the group's bounding box and its most central body settle
                               most votes) and evaluates the accepted records from a list in
-                              shared memory; 2 visits one child at a time with the vote of
-                              every body.  The same interactions either way; the sums may
-                              differ in the last bits (list order).  0: the default, 1 except
-                              in precise mode, which keeps the reference's order of
-                              accumulation */
+                              shared memory; 2 keeps the reference's order of accumulation
+                              (depth-first, children in order).  The same interactions either
+                              way; the sums may differ in the last bits.  0: the default, 1
+                              except in precise mode, which keeps the reference's order */
     int32_t reserved[2];
 } nbh_config;
 
@@ -253,7 +258,7 @@ int nbh_direct_f64(nbh_sim* sim, int32_t nidx, const int32_t* idx,
  * printDepth, printImpulse), reduced on the GPU in FP64 from the current state, in a fixed
  * order.  Energies and momenta use the state as stored: after a step, positions and
  * velocities at the end of that step. */
-#define NBH_DIAG_POTENTIAL 1   /* also the O(N^2) pair potential (0.8 s at 1M bodies on GB300) */
+#define NBH_DIAG_POTENTIAL 1   /* also the O(N^2) pair potential (0.24 s at 1M bodies on GB300) */
 typedef struct nbh_diag {
     double mass;                   /* sum m */
     double com[3];                 /* sum m x / sum m */
