@@ -500,110 +500,135 @@ __global__ void __launch_bounds__(kTrainThreads, kTrainBlocksPerSm)
     }
 }
 
-// Weight gradients of one chunk of samples.  blockIdx.x < 64 / R: rows R blockIdx.x .. of gW2
-// and gb2, a thread R / 8 rows (tid % 8 + 8 i) by four columns (tid / 8 + 16 c); the next
-// block gW1 and gb1, two threads per unit; the last gW3 and gb3.  Tiles come in through four
-// stages of asynchronous copies (with two the kernel waited for them: 67 us a pass at 100,000
-// samples).  R = 16 for many chunks; 8 spreads few chunks (small batches) over more blocks,
-// where the chains of dependent multiply-adds are what takes the time.
-constexpr int kWeightThreads = 128;
-constexpr int kWeightStages = 4;
-constexpr int kStageFloats = (16 + kMlpHid) * kRow;
-constexpr size_t kWeightSmem = sizeof(float) * kWeightStages * kStageFloats;
-static_assert(kStageFloats >= (kMlpHid + kMlpIn) * kRow, "a stage holds what any block takes of a tile");
-__device__ __forceinline__ void async_copy(float* dst, const float* src, int floats) {
-    for (int i = 4 * threadIdx.x; i < floats; i += 4 * kWeightThreads) {
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + i);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + i) : "memory");
-    }
-}
+// Weight gradients of one chunk of samples, each output one chain of multiply-adds in sample
+// order.  blockIdx.x < 64 / R * Q: R rows of gW2 (and gb2) by 64 / Q columns, a thread rows
+// tid % 8 + 8 i by every (THREADS / 8)-th column; the next Q blocks 64 / Q units of gW1 and gb1;
+// the last Q as many of gW3, and gb3.  Tiles come in through stages of asynchronous copies (with
+// two the kernel waited for them: 67 us a pass at 100,000 samples).
+// <16, 1, 128, 4> for many chunks, bound by shared-memory loads (6 for 32 multiply-adds; 8 for 32
+// with 256 threads: 135 us a training step at 100,000 samples against 125).
+// <8, 4, 128, 8> for few chunks (small batches), whose blocks leave SMs idle while each walks its
+// chunk tile after tile: smaller blocks copy and load a third per tile, and a
+// warp's few instructions per tile (the steps unrolled, the copies' places worked out once) are
+// what takes the time.  A training step at 5,000 samples 65.7 -> 41 us against <8, 1, 128, 4>, at
+// 20,000 70 -> 57; at 100,000 (the copies' places only) 125 -> 122.
+template <int R, int Q, int THREADS, int STAGES>
+struct WeightSplit {
+    static constexpr int kUnits = kMlpHid / Q;                            // columns or units of a block
+    static constexpr int kRowBlocks = kMlpHid / R, kBlocks = kRowBlocks * Q + 2 * Q;
+    static constexpr int kColGroups = THREADS / 8, kCols = kUnits / kColGroups;   // gW2 columns of a thread
+    static constexpr int kFeatGroups = THREADS / kUnits;
+    static constexpr int kFeat = (kMlpIn + kFeatGroups - 1) / kFeatGroups;        // gW1 features of a thread
+    static constexpr int kRows = kUnits + (R > kMlpIn ? R : kMlpIn);              // of a stage
+    static constexpr size_t kSmem = sizeof(float) * STAGES * kRows * kRow;
+    static_assert(kCols * kColGroups == kUnits && kFeat * kFeatGroups >= kMlpIn && kUnits < THREADS,
+                  "every output has a thread");
+};
 __device__ __forceinline__ void chain4(float& acc, const float4 a, const float4 b) {
     acc = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
 __device__ __forceinline__ void sum4(float& acc, const float4 a) { acc = (((acc + a.x) + a.y) + a.z) + a.w; }
 
-template <int R>
-__global__ void __launch_bounds__(kWeightThreads) mlp_weights_kernel(const TrainTile* __restrict__ in, int n,
-                                                                     float* __restrict__ part) {
+template <int R, int Q, int THREADS, int STAGES>
+__global__ void __launch_bounds__(THREADS) mlp_weights_kernel(const TrainTile* __restrict__ in, int n,
+                                                              float* __restrict__ part) {
     extern __shared__ __align__(16) unsigned char train_smem[];
+    using Split = WeightSplit<R, Q, THREADS, STAGES>;
+    constexpr int kUnits = Split::kUnits, kCols = Split::kCols, kColGroups = Split::kColGroups, kFeat = Split::kFeat;
+    constexpr int kStageFloats = Split::kRows * kRow;
     float* const buf = reinterpret_cast<float*>(train_smem);
-    constexpr int RI = R / 8;
+    constexpr int RI = R / 8, kSteps = Q > 1 ? kTile / 4 : 4;      // four samples each, unrolled
     const int tid = threadIdx.x;
     const int chunk = (n + gridDim.y - 1) / gridDim.y;
     const int s0 = blockIdx.y * chunk, s1 = min(n, s0 + chunk);
     float* const g = part + (size_t)blockIdx.y * kMlpParams;
-    const int kind = max(0, (int)blockIdx.x - kMlpHid / R + 1);    // 0: gW2 rows, 1: gW1, 2: gW3
-    const int row0 = R * (int)blockIdx.x;
-    const int arows = kind == 0 ? R : (kind == 1 ? kMlpHid : 1);   // gradients; activations follow
+    const int bx = (int)blockIdx.x - Split::kRowBlocks * Q;
+    const int kind = bx < 0 ? 0 : (bx < Q ? 1 : 2);                // gW2 rows, gW1, gW3
+    const int row0 = R * ((int)blockIdx.x % Split::kRowBlocks);
+    const int q = bx < 0 ? (int)blockIdx.x / Split::kRowBlocks : bx % Q;
+    const int u0 = q * kUnits;                                     // first column or unit
+    const int arows = kind == 0 ? R : (kind == 1 ? kUnits : 1);    // gradients; activations follow
     const int t0 = s0 / kTile, t1 = s1 > s0 ? (s1 + kTile - 1) / kTile : t0;
+    // a tile comes as two runs of rows; this thread's 16-byte pieces of them
+    constexpr int kTileFloats = sizeof(TrainTile) / sizeof(float);
+    const float* const first = kind == 0 ? in->d2[row0] : (kind == 1 ? in->d1[u0] : in->dy);
+    const float* const second = kind == 0 ? in->h1[u0] : (kind == 1 ? in->x[0] : in->h2[u0]);
+    const int split = arows * kRow, floats = split + (kind == 1 ? kMlpIn : kUnits) * kRow;
+    constexpr int kPieces = (kStageFloats / 4 + THREADS - 1) / THREADS;
+    int from[kPieces];
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int e = 4 * (tid + i * THREADS);
+        from[i] = e < split ? e : e - split + (int)(second - first);
+    }
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(buf) + 16 * tid;
     auto fetch = [&](int t) {
         if (t < t1) {
-            float* const w = buf + (t % kWeightStages) * kStageFloats;
-            if (kind == 0) {
-                async_copy(w, in[t].d2[row0], R * kRow);
-                async_copy(w + R * kRow, in[t].h1[0], kMlpHid * kRow);
-            } else if (kind == 1) {
-                async_copy(w, in[t].d1[0], kMlpHid * kRow);
-                async_copy(w + kMlpHid * kRow, in[t].x[0], kMlpIn * kRow);
-            } else {
-                async_copy(w, in[t].dy, kRow);
-                async_copy(w + kRow, in[t].h2[0], kMlpHid * kRow);
+            const unsigned d = dst + (t % STAGES) * (unsigned)(kStageFloats * sizeof(float));
+            const float* const src = first + (size_t)t * kTileFloats;
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) {
+                if (4 * (tid + i * THREADS) < floats)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i * THREADS),
+                                 "l"(src + from[i])
+                                 : "memory");
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");       // perhaps empty
     };
-    constexpr int kHalf = kMlpIn / 2;
     const int r = tid % 8, c = tid / 8;                            // gW2
-    const int unit = tid % kMlpHid, f0 = tid < kMlpHid ? 0 : kHalf;   // gW1, gW3
-    float acc[RI][4] = {}, gb[RI] = {};
-    float w1[kHalf] = {}, u = 0.f;
+    const int unit = tid % kUnits, f0 = tid / kUnits * kFeat;      // gW1, gW3
+    float acc[RI][kCols] = {}, gb[RI] = {};
+    float w1[kFeat] = {}, u = 0.f;
 #pragma unroll
-    for (int k = 0; k < kWeightStages - 1; ++k) fetch(t0 + k);
+    for (int k = 0; k < STAGES - 1; ++k) fetch(t0 + k);
     for (int t = t0; t < t1; ++t) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kWeightStages - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();                              // tile t is here, tile t - 1 done with
-        fetch(t + kWeightStages - 1);
-        float* const a = buf + (t % kWeightStages) * kStageFloats;
+        fetch(t + STAGES - 1);
+        float* const a = buf + (t % STAGES) * kStageFloats;
         const float* const b = a + arows * kRow;
         const int lo = max(0, s0 - t * kTile), hi = min(kTile, s1 - t * kTile);
         if (lo > 0 || hi < kTile) {
             // samples of the neighbouring chunks (or none) count as zero gradients
-            for (int i = tid; i < arows * kTile; i += kWeightThreads) {
+            for (int i = tid; i < arows * kTile; i += THREADS) {
                 const int s = i % kTile;
                 if (s < lo || s >= hi) a[(i / kTile) * kRow + s] = 0.f;
             }
             __syncthreads();
         }
         if (kind == 0) {
-#pragma unroll 4
+#pragma unroll kSteps
             for (int s = 0; s < kTile; s += 4) {
-                float4 av[RI], bv[4];
+                float4 av[RI], bv[kCols];
 #pragma unroll
                 for (int i = 0; i < RI; ++i) av[i] = ld4(a + (r + 8 * i) * kRow + s);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) bv[k] = ld4(b + (c + 16 * k) * kRow + s);
+                for (int k = 0; k < kCols; ++k) bv[k] = ld4(b + (c + kColGroups * k) * kRow + s);
 #pragma unroll
                 for (int i = 0; i < RI; ++i)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) chain4(acc[i][k], av[i], bv[k]);
-                if (c == 0)
+                    for (int k = 0; k < kCols; ++k) chain4(acc[i][k], av[i], bv[k]);
+                if (c == 0 && q == 0)
 #pragma unroll
                     for (int i = 0; i < RI; ++i) sum4(gb[i], av[i]);
             }
         } else if (kind == 1) {
-#pragma unroll 2
-            for (int s = 0; s < kTile; s += 4) {
-                const float4 dv = ld4(a + unit * kRow + s);
+            if (f0 < kMlpIn) {
+#pragma unroll kSteps
+                for (int s = 0; s < kTile; s += 4) {
+                    const float4 dv = ld4(a + unit * kRow + s);
 #pragma unroll
-                for (int f = 0; f < kHalf; ++f) chain4(w1[f], dv, ld4(b + (f0 + f) * kRow + s));
-                sum4(u, dv);
+                    for (int f = 0; f < kFeat; ++f) chain4(w1[f], dv, ld4(b + (f0 + f) * kRow + s));
+                    sum4(u, dv);
+                }
             }
-        } else if (tid <= kMlpHid) {
+        } else if (tid <= kUnits) {
             // unit tid of gW3; the thread after them gb3
 #pragma unroll 4
             for (int s = 0; s < kTile; s += 4) {
                 const float4 yv = ld4(a + s);
-                if (tid < kMlpHid) chain4(u, yv, ld4(b + tid * kRow + s));
+                if (tid < kUnits) chain4(u, yv, ld4(b + tid * kRow + s));
                 else sum4(u, yv);
             }
         }
@@ -615,15 +640,17 @@ __global__ void __launch_bounds__(kWeightThreads) mlp_weights_kernel(const Train
 #pragma unroll
         for (int i = 0; i < RI; ++i) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) gw2[(row0 + r + 8 * i) * kMlpHid + c + 16 * k] = acc[i][k];
-            if (c == 0) gb2[row0 + r + 8 * i] = gb[i];
+            for (int k = 0; k < kCols; ++k) gw2[(row0 + r + 8 * i) * kMlpHid + u0 + c + kColGroups * k] = acc[i][k];
+            if (c == 0 && q == 0) gb2[row0 + r + 8 * i] = gb[i];
         }
     } else if (kind == 1) {
+        if (f0 < kMlpIn) {
 #pragma unroll
-        for (int f = 0; f < kHalf; ++f) g[unit * kMlpIn + f0 + f] = w1[f];
-        if (f0 == 0) gb1[unit] = u;
-    } else if (tid <= kMlpHid) {
-        gb2[kMlpHid + tid] = u;                       // gW3, then gb3
+            for (int f = 0; f < kFeat; ++f) g[(u0 + unit) * kMlpIn + f0 + f] = w1[f];
+        }
+        if (f0 == 0) gb1[u0 + unit] = u;
+    } else if (tid < kUnits || (tid == kUnits && q == Q - 1)) {
+        gb2[kMlpHid + u0 + tid] = u;                  // gW3, then gb3
     }
 }
 
@@ -673,15 +700,18 @@ int train_tiles(int n) { return (n + kTile - 1) / kTile; }
 int train_grid(int n, int sms) { return std::max(1, std::min(train_tiles(n), kTrainBlocksPerSm * sms)); }
 int train_chunks(int n) { return std::max(1, std::min(64, n / 2048)); }
 
+using Many = WeightSplit<16, 1, 128, 4>;
+using Few = WeightSplit<8, 4, 128, 8>;
+
 void train_pass(const float* prm, const float* X, const float* T, int n, float q, TrainWork w, float* grad,
                 float* loss, AdamStep ad, int sms, cudaStream_t s) {
     TrainTile* tiles = static_cast<TrainTile*>(w.tiles);
     const int grid = train_grid(n, sms), chunks = train_chunks(n);
     mlp_samples_kernel<true><<<grid, kTrainThreads, sizeof(TrainSmem), s>>>(prm, X, T, n, q, nullptr, tiles, w.lossp);
-    if (chunks * 6 >= sms)
-        mlp_weights_kernel<16><<<dim3(6, chunks), kWeightThreads, kWeightSmem, s>>>(tiles, n, w.part);
+    if (chunks * Many::kBlocks >= sms)
+        mlp_weights_kernel<16, 1, 128, 4><<<dim3(Many::kBlocks, chunks), 128, Many::kSmem, s>>>(tiles, n, w.part);
     else
-        mlp_weights_kernel<8><<<dim3(10, chunks), kWeightThreads, kWeightSmem, s>>>(tiles, n, w.part);
+        mlp_weights_kernel<8, 4, 128, 8><<<dim3(Few::kBlocks, chunks), 128, Few::kSmem, s>>>(tiles, n, w.part);
     mlp_reduce_kernel<<<(kMlpParams + kReduceThreads - 1) / kReduceThreads + 1, kReduceThreads, 0, s>>>(
         w.part, chunks, w.lossp, grid, grad, loss, ad);
 }
@@ -703,8 +733,8 @@ cudaError_t prepare_train_kernels() {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if ((e = cudaFuncSetAttribute(mlp_samples_kernel<true>, a, (int)sizeof(TrainSmem))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(mlp_samples_kernel<false>, a, (int)sizeof(TrainSmem))) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(mlp_weights_kernel<8>, a, (int)kWeightSmem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(mlp_weights_kernel<16>, a, (int)kWeightSmem);
+    if ((e = cudaFuncSetAttribute(mlp_weights_kernel<8, 4, 128, 8>, a, (int)Few::kSmem)) != cudaSuccess) return e;
+    return cudaFuncSetAttribute(mlp_weights_kernel<16, 1, 128, 4>, a, (int)Many::kSmem);
 }
 
 void mlp_forward(const float* prm, const float* X, int n, float* Y, int sms, cudaStream_t s) {

@@ -197,7 +197,7 @@ def test_trained_model_gains_over_fixed_theta():
     assert r["learned"]["p99_max"] <= r["plain"]["p99_max"]
 
 
-@pytest.mark.parametrize("n", [1, 5, 63, 64, 65, 3001, 40000])
+@pytest.mark.parametrize("n", [1, 5, 63, 64, 65, 3001, 40000, 60001])
 def test_mlp_passes_at_tile_edges(n):
     """Partial tiles, one tile, a ragged last tile, and more tiles than blocks.  FP32 sums against
     FP64, relative to the gradient's scale; at most 4 of the samples may fall on the other side
