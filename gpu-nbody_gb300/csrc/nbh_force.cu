@@ -77,6 +77,15 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
+// max(a, b, 0), NaN if one of them is.  The centre of a cell of massless bodies is not a number
+// (0 / 0) and passes no body's distance test; fmaxf would drop it and leave a distance of zero to
+// the group's box.
+__device__ __forceinline__ float gap_nan(float a, float b) {
+    float y;
+    asm("max.NaN.f32 %0, %1, %2, 0f00000000;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+}
+
 // One accepted interaction (calculateforce.cl:146-151).  With FEAT it also accumulates
 // the quadrupole error bound m s^2 / d^4 of an accepted cell of full width^2 s2 (0 for a
 // body), the feature the learned opening angle is predicted from.
@@ -782,9 +791,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                         float qlb = 0.0f;
                         if (ch >= nbody) {
                             const float4 lo = gc[0], hi = gc[1];
-                            const float gx = fmaxf(fmaxf(__fsub_rn(cq.x, hi.x), __fsub_rn(lo.x, cq.x)), 0.0f);
-                            const float gy = fmaxf(fmaxf(__fsub_rn(cq.y, hi.y), __fsub_rn(lo.y, cq.y)), 0.0f);
-                            const float gz = fmaxf(fmaxf(__fsub_rn(cq.z, hi.z), __fsub_rn(lo.z, cq.z)), 0.0f);
+                            const float gx = gap_nan(__fsub_rn(cq.x, hi.x), __fsub_rn(lo.x, cq.x));
+                            const float gy = gap_nan(__fsub_rn(cq.y, hi.y), __fsub_rn(lo.y, cq.y));
+                            const float gz = gap_nan(__fsub_rn(cq.z, hi.z), __fsub_rn(lo.z, cq.z));
                             // t0 * 4^-level is exact, so the fused form gives the same threshold
                             qlb = __fmaf_rn(lo.w, csl, eps2);
                             if (dist2<REF>(gx, gy, gz, eps2) >= qlb) {

@@ -960,3 +960,40 @@ def test_sorted_paths_build_the_staged_tree(n):
         arrs[0][9] = np.nextafter(np.float32(0.3), np.float32(1.0))
     load = lambda g: g.load(*arrs)                   # noqa: E731
     _assert_same_steps(_steps({"theta": 0.5}, load), _steps({"theta": 0.5, "build_phases": 3}, load))
+
+
+@pytest.mark.parametrize("kw", [{"vote_width": 16}, {"vote_width": 16, "reference": True}, {"vote_width": 32, "reference": True},
+                                {"vote_width": 32, "force_list": 2}, {"force_list": 2}, {"vote_width": 128, "force_list": 2}],
+                         ids=["16", "16-reference", "32-reference", "32", "64", "128"])
+def test_ordered_walk_opens_cells_of_massless_bodies(kw):
+    """The centre of a cell of massless bodies is not a number (0 / 0): no body's distance test passes
+    on it, so it is opened, however small it is beside the softening, and its bodies add nothing."""
+    import nbh
+    kw = dict(kw)
+    reference = kw.pop("reference", False)
+    if reference:
+        kw["arith"] = nbh.NBH_ARITH_REFERENCE
+    n = 3000
+    arrs = [a.copy() for a in ball(n, seed=31)]
+    for i in range(0, 80, 2):                        # pairs of tracers 4e-7 apart: cells of level 20 or so
+        for k in range(3):
+            arrs[k][i + 1] = arrs[k][i]
+        arrs[0][i] = arrs[0][i + 1] = np.float32(0.25) * (arrs[0][i] / np.abs(arrs[0]).max())
+        arrs[0][i + 1] += np.float32(4e-7)
+        arrs[6][i] = arrs[6][i + 1] = 0.0
+    g = gpu_sim(theta=0.5, eps=0.05, dt=0.01, **kw)
+    g.load(*arrs)
+    g.step()
+    o = oracle_for(n, theta=0.5, eps=0.05, dt=0.01, vote=kw.get("vote_width", 64), fma=not reference)
+    o.load(*arrs)
+    assert o.step() == 0
+    gs, os_ = g.read(), o.state()
+    assert all(np.isfinite(os_[k]).all() for k in KEYS)
+    assert all(np.isfinite(gs[k]).all() for k in KEYS)
+    assert g.stats()["interactions"] == o.interactions
+    if reference:
+        for k in KEYS:
+            np.testing.assert_array_equal(gs[k], os_[k], err_msg=k)
+    else:
+        rel, _ = acc_rel(gs, os_)
+        assert rel.max() <= FMA_ACC_REL_MAX and np.median(rel) <= FMA_ACC_REL_MEDIAN, (rel.max(), np.median(rel))
