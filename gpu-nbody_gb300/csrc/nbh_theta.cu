@@ -654,8 +654,8 @@ __global__ void __launch_bounds__(THREADS) mlp_weights_kernel(const TrainTile* _
     }
 }
 
-// Adds the chunks, in order (many of them in FP64), into grad, or (lr > 0) into one Adam step of prm; the last block
-// adds the loss.
+// Adds the chunks, in order (many of them in FP64), into grad, or (grad null) into one Adam step of prm
+// (whose rate may have fallen to zero); the last block adds the loss.
 struct AdamStep {
     float *prm, *m1, *m2;
     float lr, b1, b2, eps, c1, c2;
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kReduceThreads)
         for (int c = 0; c < chunks; ++c) sum += (double)part[(size_t)c * kMlpParams + i];
         gi = (float)sum;
     }
-    if (ad.lr > 0.f) {
+    if (!grad) {
         const float a = ad.b1 * ad.m1[i] + (1.f - ad.b1) * gi;
         const float v = ad.b2 * ad.m2[i] + (1.f - ad.b2) * gi * gi;
         ad.m1[i] = a;

@@ -218,3 +218,21 @@ def test_mlp_passes_at_tile_edges(n):
     assert abs(loss.value - rl) <= 1e-5 * max(1.0, abs(rl))
     assert np.abs(g - rg).max() <= 2e-5 * np.abs(rg).max() + kinks * 12.0 / n
     np.testing.assert_allclose(y, mlp_ref.forward(p, X), rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("n", [200, 40000])
+@pytest.mark.parametrize("lr", [1e-45, 1e-40])
+def test_training_with_a_rate_that_falls_to_zero(n, lr):
+    """The rate falls over the last steps, the smallest ones to zero: steps that change nothing."""
+    import mlp_ref
+    L, lib = _lib()
+    rng = np.random.default_rng(3)
+    p0 = (rng.standard_normal(mlp_ref.NPARAMS) * 0.2).astype(np.float32)
+    p = p0.copy()
+    X = rng.standard_normal((n, 12)).astype(np.float32)
+    T = rng.standard_normal(n).astype(np.float32)
+    loss = C.c_float()
+    L.check(lib.nbh_mlp_train(0, p.ctypes.data, X.ctypes.data, T.ctypes.data, n, 0.2, 10, lr, C.byref(loss)))
+    np.testing.assert_array_equal(p, p0)             # rates far below a parameter's last bit
+    rl, _ = mlp_ref.grad(p0, X, T, 0.2)
+    assert abs(loss.value - rl) <= 1e-5 * max(1.0, abs(rl))
