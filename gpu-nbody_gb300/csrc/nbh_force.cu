@@ -692,7 +692,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     }
                 }
                 if constexpr (SPLIT) {
-                    // the warps' sums through shared memory (each in its own list's place)
+                    // the warps' sums through shared memory (each in its own list's place, which every
+                    // lane has finished reading)
+                    __syncwarp();
                     float4* const out = reinterpret_cast<float4*>(lst);
 #pragma unroll
                     for (int k = 0; k < BPL; ++k) out[32 * k + lane] = make_float4(ax[k], ay[k], az[k], eb[k]);

@@ -997,3 +997,35 @@ def test_ordered_walk_opens_cells_of_massless_bodies(kw):
     else:
         rel, _ = acc_rel(gs, os_)
         assert rel.max() <= FMA_ACC_REL_MAX and np.median(rel) <= FMA_ACC_REL_MEDIAN, (rel.max(), np.median(rel))
+
+
+@pytest.mark.parametrize("vote", [32, 64, 128])
+def test_shared_groups_whose_lists_end_empty(vote):
+    """A full octree (16 bodies a side) of which every cell is opened: each of the 8 warps of a group
+    takes 8 cells of 64 bodies, 16 lists of exactly 32 records, and goes from its last evaluation
+    straight to handing its sums over in the same shared memory.  The oracle's sums, and the same
+    bits every time."""
+    side = 16
+    n = side ** 3
+    r = np.random.default_rng(5)
+    i = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij")).reshape(3, n)
+    pos = (i + 0.5) / side + np.where((i > 0) & (i < side - 1), r.uniform(-1e-4, 1e-4, (3, n)), 0.0)
+    zero = np.zeros(n, np.float32)
+    arrs = (*pos.astype(np.float32), zero, zero, zero, r.uniform(0.5, 1.5, n).astype(np.float32) / n)
+    g = gpu_sim(theta=0.01, eps=0.05, dt=0.0, vote_width=vote)
+    g.load(*arrs)
+    g.step()
+    first = g.read()
+    assert g.stats()["interactions"] == n * n
+    o = oracle_for(n, theta=0.01, eps=0.05, dt=0.0, vote=vote, fma=True)
+    o.load(*arrs)
+    assert o.step() == 0 and o.interactions == n * n
+    # accelerations nearly cancel inside the cube: errors against the largest one
+    scale = np.sqrt(sum(first[k].astype(np.float64) ** 2 for k in ("ax", "ay", "az"))).max()
+    for k in ("ax", "ay", "az"):
+        assert np.abs(first[k] - o.state()[k]).max() <= 1e-5 * scale
+    for _ in range(20):
+        g.step()
+        again = g.read()
+        for k in KEYS[6:]:
+            np.testing.assert_array_equal(again[k], first[k])
