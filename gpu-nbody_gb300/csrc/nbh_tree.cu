@@ -187,9 +187,14 @@ constexpr BuildPhase kThreePhases[3] = {{256, 0}, {16, 16}, {1, 16}};
 constexpr BuildPhase kFivePhases[5] = {{256, 0}, {64, 4}, {16, 4}, {4, 4}, {1, 4}};
 
 // One body's lock insertion into its universe's tree (see build_kernel).  Returns false
-// after raising an error (depth, pool, timeout).
+// after raising an error (depth, pool, timeout).  CHAIN: slots are read with acquire loads, so that
+// the pool need not have been emptied, and the thread's new cells are linked through start[] from
+// `chain` on.
+template <bool CHAIN = false>
 __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts, int& local_max, int& waits,
-                            int& misses) {
+                            int& misses, int* chain = nullptr) {
+    auto read_slot = [](const int* at) { return CHAIN ? ld_acquire(at) : __ldca(at); };
+    auto lock_slot = [](int* at, int was) { return CHAIN ? cas_acquire(at, was, kLock) : atomicCAS(at, was, kLock); };
     const int nbody = p.nbody;
     const int root = p.nnodes - u;
     const float4 rc = p.node4[root];
@@ -211,7 +216,7 @@ __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts,
     // the cell was initialised can only show kNull, never a child index left by
     // the previous step's tree.  Reading through L1 keeps the descents off the L2
     // lines of the top cells.
-    int ch = __ldca(slot);
+    int ch = read_slot(slot);
     for (;;) {
         while (ch >= nbody) {                      // :77-89
             if (ch >= node || depth >= kMaxDepth) {  // children sit below parents
@@ -229,10 +234,10 @@ __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts,
             r = h;
             path = octant(cx, cy, cz, bp.x, bp.y, bp.z);
             slot = cell_child(p, node) + path;
-            ch = __ldca(slot);
+            ch = read_slot(slot);
         }
         int seen = kLock;
-        if (ch != kLock && (seen = atomicCAS(slot, ch, kLock)) == ch) {
+        if (ch != kLock && (seen = lock_slot(slot, ch)) == ch) {
             if (ch == kNull) {
                 // nothing but the index itself is published: no fence needed
                 st_relaxed(slot, b);
@@ -272,6 +277,10 @@ __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts,
                     p.arrive[cell - nbody] = 0;
                     p.count[cell - nbody] = -1;           // not summed yet (see link_kernel)
                     p.clevel[cell - nbody] = depth - 1;   // root = level 0
+                    if constexpr (CHAIN) {
+                        p.start[cell - nbody] = *chain;
+                        *chain = cell;
+                    }
                     if (zero_counts) {   // bucket counters of the sampled tree
                         int4* bc = reinterpret_cast<int4*>(p.kids4 + ((size_t)(cell - nbody) << 3));
                         bc[0] = make_int4(0, 0, 0, 0);
@@ -301,6 +310,7 @@ __device__ bool lock_insert(const StepParams& p, int b, int u, bool zero_counts,
         // until it holds the new subtree
         ch = bounded_wait_ne(slot, kLock, kWaitNs, p.st, kBackoffMinNs, &waits);
         if (ch == kLock) return false;
+        if constexpr (CHAIN) ch = ld_acquire(slot);
     }
     return true;
 }
@@ -1390,11 +1400,42 @@ __device__ __forceinline__ float4 sum_children(const StepParams& p, int c, const
     }
 }
 
+// Sums cell c, which has no cell children, and climbs for as long as this thread's arrival at the
+// parent is the last one.
+template <bool REF, bool PRECISE>
+__device__ __forceinline__ void sum_and_climb(const StepParams& p, int c) {
+    const int nbody = p.nbody;
+    const int first_root = p.nnodes - p.nuniv + 1;
+    for (;;) {
+        // Every cell child of c has been summed and no other thread touches c now, so
+        // its slots are stable until the compaction below.
+        int* ch8 = cell_child(p, c);
+        const int4 s0 = reinterpret_cast<const int4*>(ch8)[0];
+        const int4 s1 = reinterpret_cast<const int4*>(ch8)[1];
+        const int sl[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        // (precise mode: the roots in FP64, as a path of its own -- folded into the
+        // FP32 loop as a per-child branch, it ran the FP64 arithmetic for every cell)
+        const float4 com = (PRECISE && c >= first_root) ? sum_children<REF, true>(p, c, sl, ch8)
+                                                        : sum_children<REF, false>(p, c, sl, ch8);
+        p.node4[c] = com;
+        const int pc = p.parent[c];
+        if (pc < 0) break;          // a root
+        if (pc <= c) {              // parents always have higher indices
+            raise_error(p.st, NBH_ERR_STATE);
+            break;
+        }
+        // pc is summed only after all its cell children arrive, this one included, so
+        // its tag still holds link's value
+        const int kc = -1 - __ldcg(p.count + (pc - nbody));
+        if (arrive_acq_rel(p.arrive + (pc - nbody)) != kc - 1) break;   // another child is to come
+        c = pc;
+    }
+}
+
 template <bool REF, bool PRECISE>
 __global__ void __launch_bounds__(256) summarize_kernel(StepParams p) {
     if (load_status(p.st)) return;
     const int nbody = p.nbody;
-    const int first_root = p.nnodes - p.nuniv + 1;
     const int stride = gridDim.x * blockDim.x;
     int low;
     const int cells = cells_to_sum(p, low);
@@ -1403,31 +1444,7 @@ __global__ void __launch_bounds__(256) summarize_kernel(StepParams p) {
         // link's tag -1 - (cell children): only a cell without cell children starts here; the
         // others are summed by their last cell child (tag < -1), perhaps already (tag >= 0)
         if (p.count[c0 - nbody] != -1) continue;
-        int c = c0;
-        for (;;) {
-            // Every cell child of c has been summed and no other thread touches c now, so
-            // its slots are stable until the compaction below.
-            int* ch8 = cell_child(p, c);
-            const int4 s0 = reinterpret_cast<const int4*>(ch8)[0];
-            const int4 s1 = reinterpret_cast<const int4*>(ch8)[1];
-            const int sl[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-            // (precise mode: the roots in FP64, as a path of its own -- folded into the
-            // FP32 loop as a per-child branch, it ran the FP64 arithmetic for every cell)
-            const float4 com = (PRECISE && c >= first_root) ? sum_children<REF, true>(p, c, sl, ch8)
-                                                            : sum_children<REF, false>(p, c, sl, ch8);
-            p.node4[c] = com;
-            const int pc = p.parent[c];
-            if (pc < 0) break;          // a root
-            if (pc <= c) {              // parents always have higher indices
-                raise_error(p.st, NBH_ERR_STATE);
-                break;
-            }
-            // pc is summed only after all its cell children arrive, this one included, so
-            // its tag still holds link's value
-            const int kc = -1 - __ldcg(p.count + (pc - nbody));
-            if (arrive_acq_rel(p.arrive + (pc - nbody)) != kc - 1) break;   // another child is to come
-            c = pc;
-        }
+        sum_and_climb<REF, PRECISE>(p, c0);
     }
 }
 
@@ -1483,8 +1500,8 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 //
 // Per cell of the shared tree: 8 slots, level, centre of mass, body count, offset in its
 // parent's range, parent, and the list of the cells by level.  A universe whose tree does not fit (close pairs make chains of
-// single-child cells) or goes too deep is left to the last block to finish, which builds such
-// universes one after another in global memory, through the lock insertion.
+// single-child cells) or goes too deep is built by its block in global memory, through the lock
+// insertion.
 // Measured, us, one launch / the stages: one sphere of 300 bodies 38 / 124, 1,000 52 / 132,
 // 3,000 97 / 140, 5,000 134 / 158, 7,168 175 / 156; 8 of 7,168 184 / 197, 200 of 1,000
 // 134 / 227, 200 of 7,168 404 / 503: up to 7,168 bodies (what shared memory holds) from 8
@@ -1510,7 +1527,7 @@ static int small_tree_cells(int bodies) {
 static size_t small_tree_smem(int cells) { return (size_t)cells * kSmallCellBytes; }
 
 struct SmallShared {
-    int status, ncell, failed, depth_max, gbase, last;
+    int status, ncell, failed, depth_max, gbase;
     int level[kMaxDepth + 1];                        // first place of each level's cells in the list
     int tie, sum[32];
     float lo[3][32], hi[3][32];
@@ -1532,67 +1549,94 @@ __global__ void begin_step_kernel(StepParams p) {
     if (!load_status(p.st)) begin_step(p);
 }
 
-// One universe's tree in global memory, by the whole block: lock insertion, then link, summarize
-// and sort over its cells, which are the ones taken from the pool meanwhile.
+// The block's universe in global memory: lock insertion, then link, summarize and sort, each thread
+// over the cells that it made itself (a list through start[], which the sort fills last; thread 0
+// has the root too).  The cells come from the pool one by one while other blocks take theirs, and their
+// slots are not emptied beforehand (see lock_insert).  One SM moves at most two sectors a clock, and a
+// cell takes some 26 of them; many universes have an SM each.  Tree stages in us, this / the stages
+// (three phases): one sphere of 1,000 bodies with 300 close pairs 300 / 381, 5,000 with 300 494 / 287,
+// with 1,500 899 / 520; 16 of 7,000 with 300 724 / 416; 50 of 1,000 with 300 549 / 879, of 7,000 with 300
+// 843 / 798; 200 of 3,000 with 900 3785 / 4312.
 template <bool REF, bool PRECISE>
-__device__ void rescue_universe(const StepParams& p, int u, int* shared_bottom) {
+__device__ void rescue_universe(const StepParams& p, int u, int* shared_status) {
     const int nbody = p.nbody, root = p.nnodes - u;
-    if (threadIdx.x == 0) *shared_bottom = ld_relaxed(&p.st->bottom);
-    __syncthreads();
-    const int above = *shared_bottom;                  // cells of this universe: [below, above) and the root
-    __syncthreads();
-    // the slots of the free cells, which the insertion expects to be empty
-    for (long long i = 2 + threadIdx.x; i < 2ll * (above - nbody); i += blockDim.x)
-        reinterpret_cast<int4*>(p.child)[i] = make_int4(kNull, kNull, kNull, kNull);
     if (threadIdx.x < 8) cell_child(p, root)[threadIdx.x] = kNull;
-    __threadfence();
     __syncthreads();
-    int lm = 1, waits = 0, misses = 0;
+    int lm = 1, waits = 0, misses = 0, mine = kNull;
     for (int b = p.ubody[u] + (int)threadIdx.x; b < p.ubody[u + 1]; b += blockDim.x)
-        if (!lock_insert(p, b, u, false, lm, waits, misses)) break;
-    atomicMax(&p.st->max_depth, lm);
-    __threadfence();
+        if (!lock_insert<true>(p, b, u, false, lm, waits, misses, &mine)) break;
+    if (threadIdx.x == 0) {
+        p.start[root - nbody] = mine;
+        mine = root;
+    }
+    if (lm > ld_relaxed(&p.st->max_depth)) atomicMax(&p.st->max_depth, lm);
+    if (waits) atomicAdd(&p.st->lock_waits[blockIdx.x % kDiagSlots], waits);
+    if (misses) atomicAdd(&p.st->cas_misses[blockIdx.x % kDiagSlots], misses);
+    __syncthreads();                                   // the tree stands, or some thread has failed
+    if (threadIdx.x == 0) *shared_status = load_status(p.st);
     __syncthreads();
-    if (threadIdx.x == 0) *shared_bottom = load_status(p.st) ? -1 : ld_relaxed(&p.st->bottom);
-    __syncthreads();
-    const int below = *shared_bottom;
-    __syncthreads();
-    if (below < 0) return;
-    const int cells = above - below + 1;               // the root last
-    for (int i = threadIdx.x; i < cells; i += blockDim.x) {
-        const int c = i == cells - 1 ? root : below + i;
+    if (*shared_status) return;
+    // link; the thread's list is turned round, oldest cells (the upper ones of a chain) first
+    int oldest = kNull;
+    for (int c = mine; c != kNull;) {
+        const int next = p.start[c - nbody];
+        p.start[c - nbody] = oldest;
+        oldest = c;
+        const int4* const ch8 = reinterpret_cast<const int4*>(cell_child(p, c));
+        const int4 s0 = ch8[0], s1 = ch8[1];
+        const int sl[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        int kc = 0;
+#pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int ch = __ldcg(cell_child(p, c) + j);
-            if (ch >= 0) p.parent[ch] = c;
+            if (sl[j] >= 0) p.parent[sl[j]] = c;
+            kc += sl[j] >= nbody;
         }
+        p.count[c - nbody] = -1 - kc;
+        c = next;
     }
-    __threadfence();
     __syncthreads();
-    for (int level = kMaxDepth - 1; level >= 0; --level) {
-        for (int i = threadIdx.x; i < cells; i += blockDim.x) {
-            const int c = i == cells - 1 ? root : below + i;
-            if (__ldcg(p.clevel + (c - nbody)) != level) continue;
-            int sl[8];
-            int* ch8 = cell_child(p, c);
-            for (int j = 0; j < 8; ++j) sl[j] = __ldcg(ch8 + j);
-            p.node4[c] = (PRECISE && c == root) ? sum_children<REF, true>(p, c, sl, ch8)
-                                                : sum_children<REF, false>(p, c, sl, ch8);
+    // sums: the lanes look for their next cell without cell children, then climb side by side
+    for (int c = oldest;;) {
+        while (c != kNull && __ldcg(p.count + (c - nbody)) != -1) c = p.start[c - nbody];
+        if (!__any_sync(0xffffffffu, c != kNull)) break;
+        if (c != kNull) {
+            sum_and_climb<REF, PRECISE>(p, c);
+            c = p.start[c - nbody];
         }
-        __threadfence();
-        __syncthreads();
+        __syncwarp();
     }
-    for (int i = threadIdx.x; i < cells; i += blockDim.x) {
-        const int c = i == cells - 1 ? root : below + i;
-        int s = p.ubody[u];
-        for (int x = c; x != root; x = __ldcg(p.parent + x)) s += __ldcg(p.loff + (x - nbody));
-        p.start[c - nbody] = s;
+    __syncthreads();
+    // sort: a cell made after its parent by the same thread starts from the parent's place, the
+    // others walk up to the root (as in sort_kernel), side by side
+    int last = kNull, from = 0;                        // the thread's last cell and its first position
+    auto place = [&](int c) {
+        const int next = p.start[c - nbody];
+        p.start[c - nbody] = from;
+        const int4* const ch8 = reinterpret_cast<const int4*>(cell_child(p, c));
+        const int4 s0 = ch8[0], s1 = ch8[1];
+        const int sl[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        int at = from;
+#pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const int ch = __ldcg(cell_child(p, c) + j);
-            if (ch >= nbody) s += __ldcg(p.count + (ch - nbody));
-            else if (ch >= 0) p.sorted[s++] = ch;
+            if (sl[j] >= nbody) at += p.count[sl[j] - nbody];
+            else if (sl[j] >= 0) p.sorted[at++] = sl[j];
         }
+        last = c;
+        return next;
+    };
+    for (int c = oldest;;) {
+        while (c != kNull && last != kNull && p.parent[c] == last) {
+            from += p.loff[c - nbody];
+            c = place(c);
+        }
+        if (!__any_sync(0xffffffffu, c != kNull)) break;
+        if (c != kNull) {
+            from = p.ubody[u];
+            for (int x = c; x != root; x = p.parent[x]) from += p.loff[x - nbody];
+            c = place(c);
+        }
+        __syncwarp();
     }
-    __syncthreads();
 }
 
 template <bool REF, bool PRECISE>
@@ -1914,26 +1958,8 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
                 else p.sorted[s++] = first + v16;
             }
         }
-    } else if (tid == 0) {
-        p.start[root - nbody] = -1;                    // for the last block (a wait that gave up or an
-                                                       // empty pool have set the status)
-    }
-    // the last block to finish builds what did not fit
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) S.last = S.failed || p.nuniv > 1 ? atomicAdd(&p.st->bbox_ticket, 1) == p.nuniv - 1 : 0;
-    __syncthreads();
-    if (!S.last) return;
-    __threadfence();
-    if (tid == 0) p.st->bbox_ticket = 0;
-    for (int w = 0; w < p.nuniv; ++w) {
-        if (__ldcg(p.start + (p.nnodes - w - nbody)) != -1) continue;
-        if (tid == 0) S.status = load_status(p.st);
-        __syncthreads();
-        const int status = S.status;
-        __syncthreads();
-        if (status) return;
-        rescue_universe<REF, PRECISE>(p, w, &S.gbase);
+    } else if (S.failed == 1) {                        // (a wait that gave up or an empty pool: the status says so)
+        rescue_universe<REF, PRECISE>(p, u, &S.status);
     }
 }
 

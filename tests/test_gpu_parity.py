@@ -1029,3 +1029,40 @@ def test_shared_groups_whose_lists_end_empty(vote):
         again = g.read()
         for k in KEYS[6:]:
             np.testing.assert_array_equal(again[k], first[k])
+
+
+@pytest.mark.parametrize("mode", ["fma", "reference", "precise"])
+def test_one_launch_tree_of_many_that_do_not_fit(mode):
+    """More universes than SMs, two of three with chains that outgrow shared memory: their blocks build
+    them in global memory side by side, taking cells from the pool in turn, over slots that the
+    steps before have used."""
+    import nbh
+    kw = {"fma": {"theta": 0.5}, "reference": {"theta2": 1.5, "vote_width": 16, "arith": nbh.NBH_ARITH_REFERENCE},
+          "precise": {"theta": 0.5, "precise": True}}[mode]
+    parts = [plummer(40 + i, seed=200 + i) if i % 3 == 0 else _close_pairs(300 + 7 * i, 100 + i, 300 + i) for i in range(200)]
+    counts = [p[0].size for p in parts]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    load = lambda g: g.load_batch(counts, *cat)      # noqa: E731
+    kw["pool_factor"] = 16.0
+    _assert_same_steps(_steps(kw, load, 6), _steps({**kw, "build_phases": 1}, load, 6))
+
+
+@pytest.mark.parametrize("universes,n,pairs", [(20000, 16, 0), (100, 1000, 300)])
+def test_one_launch_tree_costs_no_more_than_the_staged_one(universes, n, pairs):
+    """Many tiny universes, and ones that do not fit shared memory: work that one block did for each of
+    them in turn took 5 to 200 times the stages.  (A step takes them side by side; 1.5 leaves room
+    for the clock and for launches.)"""
+    parts = [_close_pairs(n, pairs, 400 + i) for i in range(min(universes, 8))]
+    cat = [np.concatenate([parts[u % len(parts)][k] for u in range(universes)]) for k in range(7)]
+    ms = []
+    for kw in ({}, {"build_phases": 3}):
+        g = gpu_sim(theta=0.9, eps=0.05, dt=0.0, pool_factor=16.0, stage_timing=True, **kw)
+        g.load_batch([n] * universes, *cat)
+        t = []
+        for _ in range(9):
+            g.step()
+            st = g.stats()
+            t.append(st["ms_bbox"] + st["ms_build"] + st["ms_summarize"] + st["ms_sort"])
+        ms.append(np.median(t))
+        g.close()
+    assert ms[0] <= 1.5 * ms[1], ms
