@@ -56,6 +56,7 @@ struct nbh_sim {
     bool build_buckets = true;     // lock phases insert a sample, the rest is built per slot
     int max_bodies = 0;            // bodies of the largest universe
     bool small_tree = false;       // all tree stages in one launch, one block per universe
+    bool small_keep = false;       // ... by the tuner's choice
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
     int top_cells = 0;             // cells of each block's shared tree for these universes
@@ -669,6 +670,7 @@ int nbh_load_batch(nbh_sim* sim, int32_t nuniv, const int32_t* counts, const flo
     // one launch for small universes unless the configuration names a schedule
     sim->small_tree = sim->max_bodies <= small_tree_max_bodies(nuniv) && sim->cfg.build_phases == 0 &&
                       sim->cfg.build_buckets == 0 && sim->cfg.top_phase == 0;
+    sim->small_keep = false;
     sim->top_possible = max_chunks <= top_build_max_samples();
     sim->top_cells = top_build_cells(max_chunks);
     if (!sim->top_possible || sim->top_phase == 2) sim->top_split = 0;
@@ -789,6 +791,13 @@ int finish_steps(nbh_sim* sim, int32_t nsteps) {
                            : status == NBH_ERR_TIMEOUT ? "a device-side wait timed out"
                                                        : "device error";
         return fail(sim, status, what);
+    }
+    // close pairs that outgrow the one launch's shared memory stay for a while: the stages build the
+    // same tree
+    if (sim->small_tree && !sim->small_keep && sim->h_state->handed_over > 0 &&
+        hand_over_to_stages(sim->nuniv, sim->max_bodies, sim->sms)) {
+        sim->small_tree = false;
+        drop_graph(sim);
     }
     return NBH_OK;
 }
@@ -1484,7 +1493,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
     sim->build_phases = best_ph;
     sim->build_buckets = best_bk;
     sim->top_split = best_top;
-    sim->small_tree = best_small;
+    sim->small_tree = sim->small_keep = best_small;
     if ((e = set_geometry(sim))) return e;
     drop_graph(sim);
     out->force_threads = best_t;

@@ -61,6 +61,7 @@ struct DevState {
     int pool_low;        // lowest cell whose slots a build may have written since the last reset
     int sum_low;         // cells below were summed as they were built, but for the listed ones
     int nextra;          // cells below sum_low that were not, listed in start[]
+    int handed_over;     // one-launch trees of the last step that did not fit shared memory
     // Build contention meters, spread over kDiagSlots addresses so that counting does not
     // itself serialise: descents that found their slot locked, and lost lock races.
     int lock_waits[32];

@@ -21,6 +21,8 @@ void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int s
 // universe (max_bodies: bodies of the largest).
 void launch_small_tree(const StepParams& p, bool ref, int max_bodies, cudaStream_t s);
 int small_tree_max_bodies(int universes);
+// Universes whose tree did not fit shared memory in a step cost less in the stages from the next one on.
+bool hand_over_to_stages(int universes, int max_bodies, int sms);
 int top_build_max_samples();
 int top_build_cells(int max_chunks);
 cudaError_t prepare_tree_kernels();   // raises the dynamic shared-memory limit of the top builder

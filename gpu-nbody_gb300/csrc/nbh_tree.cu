@@ -1509,6 +1509,8 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 constexpr int kSmallBodies = 7168, kSmallBodiesFew = 5120;
 constexpr size_t kSmallCellBytes = 8 * sizeof(unsigned short) + sizeof(float4) + 4 * sizeof(unsigned short) + 1;
 int small_tree_max_bodies(int universes) { return universes >= 8 ? kSmallBodies : kSmallBodiesFew; }
+// (measured either side of 50 universes and of 1,000 bodies on 152 SMs: see rescue_universe)
+bool hand_over_to_stages(int universes, int max_bodies, int sms) { return 3 * universes < sms && max_bodies > 1024; }
 // Universes of at most kSortedBodies bodies, a body per thread, are built by sorting the bodies'
 // paths below the root: kSortedLevels octants and the body's index in 64 bits, kept in the
 // place of the centres of mass until the tree stands.
@@ -1542,6 +1544,7 @@ __device__ __forceinline__ void begin_step(const StepParams& p) {
     st->bbox_ticket = 0;
     st->step += 1;
     st->force_next = 0;
+    st->handed_over = 0;
     for (int j = 0; j < kDiagSlots; ++j) st->lock_waits[j] = st->cas_misses[j] = 0;
     st->interactions = 0ull;
 }
@@ -1556,7 +1559,8 @@ __global__ void begin_step_kernel(StepParams p) {
 // cell takes some 26 of them; many universes have an SM each.  Tree stages in us, this / the stages
 // (three phases): one sphere of 1,000 bodies with 300 close pairs 300 / 381, 5,000 with 300 494 / 287,
 // with 1,500 899 / 520; 16 of 7,000 with 300 724 / 416; 50 of 1,000 with 300 549 / 879, of 7,000 with 300
-// 843 / 798; 200 of 3,000 with 900 3785 / 4312.
+// 843 / 798; 200 of 3,000 with 900 3785 / 4312.  So few universes of more than 1,024 bodies go on with
+// the stages once one of them has not fit (hand_over_to_stages).
 template <bool REF, bool PRECISE>
 __device__ void rescue_universe(const StepParams& p, int u, int* shared_status) {
     const int nbody = p.nbody, root = p.nnodes - u;
@@ -1568,6 +1572,7 @@ __device__ void rescue_universe(const StepParams& p, int u, int* shared_status) 
     if (threadIdx.x == 0) {
         p.start[root - nbody] = mine;
         mine = root;
+        atomicAdd(&p.st->handed_over, 1);
     }
     if (lm > ld_relaxed(&p.st->max_depth)) atomicMax(&p.st->max_depth, lm);
     if (waits) atomicAdd(&p.st->lock_waits[blockIdx.x % kDiagSlots], waits);

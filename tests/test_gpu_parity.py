@@ -1047,7 +1047,7 @@ def test_one_launch_tree_of_many_that_do_not_fit(mode):
     _assert_same_steps(_steps(kw, load, 6), _steps({**kw, "build_phases": 1}, load, 6))
 
 
-@pytest.mark.parametrize("universes,n,pairs", [(20000, 16, 0), (100, 1000, 300)])
+@pytest.mark.parametrize("universes,n,pairs", [(20000, 16, 0), (1, 5000, 1500), (100, 1000, 300)])
 def test_one_launch_tree_costs_no_more_than_the_staged_one(universes, n, pairs):
     """Many tiny universes, and ones that do not fit shared memory: work that one block did for each of
     them in turn took 5 to 200 times the stages.  (A step takes them side by side; 1.5 leaves room
