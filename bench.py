@@ -60,14 +60,14 @@ def step_launches(counts, tune=None):
     """Kernels in one fixed-angle step graph of universes of `counts` bodies: the work-item order
     is part of the integrate launch; small universes build their tree in one launch, mid-size
     ones the whole 1/16 sample in the first phase (include/nbh.h, top_phase)."""
-    phases, buckets, top = ((3, 1, 1) if tune is None else
-                            (tune["build_phases"], tune["build_buckets"], tune["top_phase"]))
     largest, chunks = max(counts), sum((c + 255) // 256 for c in counts)
-    if (phases, buckets, top) == (3, 1, 1):
-        if largest <= (7168 if len(counts) >= 8 else 5120):
-            return 3 + (len(counts) > 1)      # (step counter of a batch,) tree, force, integrate
-        if largest <= (65536 if chunks >= 4096 else 32768):
-            return graph_launches(3, 1) - 1 - 4
+    small = 4 if largest <= (7168 if len(counts) >= 8 else 5120) else 1
+    phases, buckets, top = ((3, 1, small) if tune is None else
+                            (tune["build_phases"], tune["build_buckets"], tune["top_phase"]))
+    if top == 4:
+        return 3 + (len(counts) > 1)          # (step counter of a batch,) tree, force, integrate
+    if (phases, buckets, top) == (3, 1, 1) and largest <= (65536 if chunks >= 4096 else 32768):
+        return graph_launches(3, 1) - 1 - 4
     return graph_launches(phases, buckets) - 1
 
 

@@ -56,7 +56,7 @@ struct nbh_sim {
     bool build_buckets = true;     // lock phases insert a sample, the rest is built per slot
     int max_bodies = 0;            // bodies of the largest universe
     bool small_tree = false;       // all tree stages in one launch, one block per universe
-    bool small_keep = false;       // ... by the tuner's choice
+    bool small_keep = false;       // ... by the configuration or the tuner's choice
     int top_phase = 0;             // config: where the first phase may build in shared memory
     bool top_possible = false;     // the loaded universes are small enough for it
     int top_cells = 0;             // cells of each block's shared tree for these universes
@@ -558,7 +558,7 @@ int nbh_create(const nbh_config* cfg_in, nbh_sim** out) {
                                               "in [64, 256]");
     if (cfg.build_phases != 0 && cfg.build_phases != 1 && cfg.build_phases != 3 && cfg.build_phases != 5)
         return fail(nullptr, NBH_ERR_INVALID, "build_phases must be 1, 3 or 5");
-    if (cfg.top_phase < 0 || cfg.top_phase > 3) return fail(nullptr, NBH_ERR_INVALID, "top_phase must be 0 to 3");
+    if (cfg.top_phase < 0 || cfg.top_phase > 4) return fail(nullptr, NBH_ERR_INVALID, "top_phase must be 0 to 4");
     if (cfg.force_list < 0 || cfg.force_list > 2)
         return fail(nullptr, NBH_ERR_INVALID, "force_list must be 0 (default), 1 (on) or 2 (off)");
     if (cfg.build_buckets < 0 || cfg.build_buckets > 2)
@@ -667,10 +667,10 @@ int nbh_load_batch(nbh_sim* sim, int32_t nuniv, const int32_t* counts, const flo
     // disc, 16384 chunks: 11-15 % slower in shared memory)
     sim->max_bodies = 0;
     for (int u = 0; u < nuniv; ++u) sim->max_bodies = std::max(sim->max_bodies, (int)counts[u]);
-    // one launch for small universes unless the configuration names a schedule
-    sim->small_tree = sim->max_bodies <= small_tree_max_bodies(nuniv) && sim->cfg.build_phases == 0 &&
-                      sim->cfg.build_buckets == 0 && sim->cfg.top_phase == 0;
-    sim->small_keep = false;
+    // one launch for small universes unless the configuration names another schedule
+    const bool unnamed = sim->cfg.build_phases == 0 && sim->cfg.build_buckets == 0 && sim->cfg.top_phase == 0;
+    sim->small_keep = sim->cfg.top_phase == 4;
+    sim->small_tree = sim->max_bodies <= small_tree_max_bodies(nuniv) && (unnamed || sim->small_keep);
     sim->top_possible = max_chunks <= top_build_max_samples();
     sim->top_cells = top_build_cells(max_chunks);
     if (!sim->top_possible || sim->top_phase == 2) sim->top_split = 0;
@@ -1402,8 +1402,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
         bool in_place;   // the schedule in place before
     };
     std::vector<TreeCand> tcands;
-    // (fourth column: one launch for small universes, where that is in place; reported as the
-    // three-phase bucketed schedule with one block per universe, which it would be otherwise)
+    // (fourth column: one launch for small universes, where that is in place)
     const int tree_c[14][4] = {{1, 0, 0, 0}, {3, 0, 0, 0}, {5, 0, 0, 0}, {3, 1, 0, 0}, {5, 1, 0, 0},
                                {3, 0, 1, 0}, {5, 0, 1, 0}, {3, 1, 1, 0}, {5, 1, 1, 0},
                                {3, 0, 8, 0}, {5, 0, 8, 0}, {3, 1, 8, 0}, {5, 1, 8, 0}, {3, 1, 1, 1}};
@@ -1420,7 +1419,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
         float ms = 0.0f;
         err = timed([&] { enqueue_tree(sim, p); }, &ms);
         if (err != cudaSuccess) break;
-        add_trial(1, tc[0], tc[1], tc[2], ms);
+        add_trial(1, tc[0], tc[1], tc[3] ? -1 : tc[2], ms);
         const bool before = (tc[3] != 0) == small_before &&
                             (small_before || (tc[0] == phases_before &&
                                               (tc[1] != 0) == (buckets_before && phases_before != 1) &&
@@ -1501,7 +1500,7 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
     out->stack_cap = best_c;
     out->build_phases = best_ph;
     out->build_buckets = best_bk ? 1 : 2;
-    out->top_phase = best_top == 8 ? 3 : (best_top == 1 ? 1 : 2);
+    out->top_phase = best_small ? 4 : (best_top == 8 ? 3 : (best_top == 1 ? 1 : 2));
     out->ms_force = best_ms;
     out->ms_tree = best_tree;
     return NBH_OK;

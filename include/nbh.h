@@ -109,9 +109,14 @@ typedef struct nbh_config {
                               block per universe builds the whole 1/16 sample of the 3-phase
                               bucketed schedule where no universe has more than 128 * 256
                               bodies (256 * 256 in batches of 4096 * 256 and more).
-                              With build_phases, build_buckets and top_phase all 0, universes
-                              of at most 5120 bodies (7168 each from 8 universes on) take one
-                              launch for the whole tree, one block per universe */
+                              4: universes of at most 5120 bodies (7168 each from 8 universes
+                              on) take one launch for the whole tree, one block per universe;
+                              larger ones as with 0.  So do the defaults (build_phases,
+                              build_buckets and top_phase all 0), until a step finds a
+                              universe whose tree does not fit shared memory (many close
+                              pairs) among fewer universes than a third of the SMs, of more
+                              than 1024 bodies: from the next call on those take the launches
+                              of the stages, which are faster then */
     int32_t force_list;    /* the whole-warp walks (vote width 32, 64 or 128; FMA arithmetic;
                               fixed or per-body angle): 1 decides each tested child on its own
                               lane (the group's bounding box and its most central body settle
@@ -308,10 +313,12 @@ typedef struct nbh_tune {
     int32_t trial_b[NBH_TUNE_MAX_TRIALS];       /* stack capacity (force), or bucketed (tree) */
     int32_t trial_vote[NBH_TUNE_MAX_TRIALS];    /* vote width (force); blocks per universe of
                                                    the shared-memory first phase, 0 for the
-                                                   global locks (tree) */
+                                                   global locks, -1 for the one launch of
+                                                   small universes (tree) */
     float   trial_ms[NBH_TUNE_MAX_TRIALS];      /* mean of 3 timed launches after 1 warm-up */
     int32_t top_phase;             /* chosen first phase, as nbh_config.top_phase: 1 or 3
-                                      shared memory (one or eight blocks per universe), 2 global */
+                                      shared memory (one or eight blocks per universe), 2 global,
+                                      4 the whole tree in one launch */
 } nbh_tune;
 int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out);
 

@@ -169,3 +169,34 @@ def test_close_pairs_inside_the_sample_make_long_chains():
         np.testing.assert_array_equal(srt, ref[0], err_msg=str(key))
         for k in KEYS:
             np.testing.assert_array_equal(state[k], ref[1][k], err_msg="%s %s" % (key, k))
+
+
+@pytest.mark.parametrize("counts", [[1000], [300, 2000, 40], [900] * 9])
+def test_one_launch_tree_has_a_name_of_its_own(counts):
+    """The tuner tells the one launch for small universes from the staged schedules, and a sim that
+    is created with what it reports takes the schedule that it chose."""
+    parts = [plummer(c, seed=70 + i) for i, c in enumerate(counts)]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+
+    def stages(**kw):
+        g = gpu_sim(theta=0.5, eps=0.05, dt=0.01, stage_timing=True, **kw)
+        g.load_batch(counts, *cat)
+        g.step(3)
+        st = g.stats()
+        return g, st["ms_bbox"] > 0.004 and st["ms_summarize"] > 0.004
+
+    g, staged = stages()
+    assert not staged
+    t = g.autotune()
+    trees = [(tr["a"], tr["b"], tr["vote"]) for tr in t["trials"] if tr["kind"] == "tree"]
+    assert len(set(trees)) == len(trees) and (3, 1, -1) in trees
+    schedule = {k: t[k] for k in ("build_phases", "build_buckets", "top_phase")}
+    h, staged = stages(**schedule)
+    assert staged == (schedule["top_phase"] != 4)
+    for top in (1, 4):
+        h, staged = stages(**{**schedule, "build_phases": 3, "build_buckets": 1, "top_phase": top})
+        assert staged == (top != 4)
+    big = gpu_sim(top_phase=4)                       # too large for it: the default schedule
+    big.load(*plummer(6000, seed=69))
+    big.step(2)
+    assert big.stats()["status"] == 0

@@ -41,6 +41,18 @@ def test_graph_launch_count_follows_the_build_schedule():
     assert bench.graph_launches(1, 1) == 7 + 1                 # one pass has no bucketed completion
 
 
+def test_step_launch_count_follows_the_reported_schedule():
+    import bench
+    tune = dict(build_phases=3, build_buckets=1, top_phase=4)
+    staged = bench.graph_launches(3, 1) - 1                    # (the work-item order is part of integrate)
+    assert bench.step_launches([1000]) == bench.step_launches([1000], tune) == 3
+    assert bench.step_launches([1000, 50]) == bench.step_launches([1000, 50], tune) == 4
+    assert bench.step_launches([1000], {**tune, "top_phase": 1}) == staged - 4   # the tuner left the one launch
+    assert bench.step_launches([1000], {**tune, "top_phase": 2}) == staged
+    assert bench.step_launches([6000]) == staged - 4           # the whole 1/16 sample in the first phase
+    assert bench.step_launches([1 << 20], {**tune, "top_phase": 3}) == staged
+
+
 def test_workload_shapes():
     import argparse
     import bench
