@@ -992,6 +992,7 @@ int nbh_get_stats(nbh_sim* sim, nbh_stats* out) {
         out->lock_waits += d.lock_waits[j];
         out->cas_misses += d.cas_misses[j];
     }
+    out->force_restarts = d.restarts;
     out->ms_bbox = sim->stage_ms[0];
     out->ms_build = sim->stage_ms[1];
     out->ms_summarize = sim->stage_ms[2];
@@ -1282,8 +1283,9 @@ int nbh_autotune(nbh_sim* sim, int32_t flags, nbh_tune* out) {
             ++out->trials;
         }
     };
-    // force geometries: stacks from the smallest that walks this depth (+2 levels of
-    // headroom) on the fast path, to the largest; the geometry in place is always timed
+    // force geometries: stacks from about the smallest that holds a depth-first walk of this depth
+    // (+ 2 levels; seven waiting siblings a level, while a group whose stack does fill up restarts
+    // on the per-level walk), midway, and the largest; the geometry in place is always timed
     int cap_fit = 7 * (depth + 1) + 8;
     cap_fit = std::max(64, (cap_fit + 7) / 8 * 8);
     std::vector<std::pair<int, int>> geo;

@@ -62,6 +62,7 @@ struct DevState {
     int sum_low;         // cells below were summed as they were built, but for the listed ones
     int nextra;          // cells below sum_low that were not, listed in start[]
     int handed_over;     // one-launch trees of the last step that did not fit shared memory
+    int restarts;        // groups of the last force walk that went on with the per-level walk
     // Build contention meters, spread over kDiagSlots addresses so that counting does not
     // itself serialise: descents that found their slot locked, and lost lock races.
     int lock_waits[32];

@@ -358,7 +358,7 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
         if (item >= nitems) break;
         const int half = W < 32 ? item & 1 : 0;
         if (W < 32) item >>= 1;
-        if (p.item_order) item = p.item_order[item];   // costly items first (see item_order_kernel)
+        if (p.item_order) item = p.item_order[item];   // costly items first (see order_items)
         const int2 wi = items[item];
         const int u = wi.y;
         const int uend = p.ubody[u + 1];
@@ -882,7 +882,8 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                 __syncwarp();
             }
             if (!walked) {
-                // Deep trees: per-level (cell, next child) walk (calculateforce.cl:112-172).
+                // The stack was full: per-level (cell, next child) walk (calculateforce.cl:112-172).
+                if (lane == 0) atomicAdd(&p.st->restarts, 1);
                 int depth = 0;
                 int node = root;
                 int k8 = 0;

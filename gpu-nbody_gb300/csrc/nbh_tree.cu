@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(256) bbox_kernel(StepParams p) {
         st->bucket_next = 0;
         st->sum_low = 0;
         st->nextra = 0;
+        st->restarts = 0;
         for (int j = 0; j < kDiagSlots; ++j) st->lock_waits[j] = st->cas_misses[j] = 0;
         st->interactions = 0ull;
     }
@@ -1545,6 +1546,7 @@ __device__ __forceinline__ void begin_step(const StepParams& p) {
     st->step += 1;
     st->force_next = 0;
     st->handed_over = 0;
+    st->restarts = 0;
     for (int j = 0; j < kDiagSlots; ++j) st->lock_waits[j] = st->cas_misses[j] = 0;
     st->interactions = 0ull;
 }

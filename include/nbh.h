@@ -86,11 +86,12 @@ typedef struct nbh_config {
     int32_t use_graph;     /* 1: replay each step as one captured CUDA graph (default) */
     int32_t force_threads; /* force launch geometry: threads per block, 64 / 128 / 256
                               (0: 128); set by nbh_autotune */
-    int32_t stack_cap;     /* entries of each vote group's shared-memory stack, 64..256, a
-                              multiple of 8 (0: 256); trees deeper than (cap - 8) / 7 + 1
-                              levels take the per-level walk; in the list walk (force_list)
-                              the cells whose children are pending, and a group that would
-                              hold more restarts on the per-level walk */
+    int32_t stack_cap;     /* size of each vote group's shared-memory stack, 64..256, a
+                              multiple of 8 (0: 256): in the list walk (force_list) the cells
+                              whose children are still to be tested, in the ordered walk half
+                              as many nodes again that wait for their turn.  A group whose
+                              stack would overflow restarts on a walk with one entry per
+                              level: the same result, slower (nbh_stats.force_restarts) */
     int32_t build_phases;  /* octree insertion launches: 1 (one pass), 3 or 5 (0: 3) */
     int32_t build_buckets; /* 1 (or 0, the default): with 5 phases the lock phases insert a
                               1/16 sample of the bodies and every other body joins the
@@ -148,7 +149,9 @@ typedef struct nbh_stats {
     float   ms_bbox, ms_build, ms_summarize, ms_sort, ms_force, ms_integrate, ms_step;
     float   ms_theta;          /* learned opening angle: features + MLP inference of the last
                                   step (0 without a model; stage_timing = 1 only) */
-    float   reserved[7];
+    int32_t force_restarts;    /* groups of the last force walk whose stack overflowed and which
+                                  restarted on the per-level walk (stack_cap) */
+    float   reserved[6];
 } nbh_stats;
 
 typedef struct nbh_sim nbh_sim;

@@ -1066,3 +1066,75 @@ def test_one_launch_tree_costs_no_more_than_the_staged_one(universes, n, pairs):
         ms.append(np.median(t))
         g.close()
     assert ms[0] <= 1.5 * ms[1], ms
+
+
+def _nest(levels, seed):
+    """A body in each of seven octants of every level and the next level in octant 0: a depth-first
+    walk to the innermost bodies leaves seven nodes a level waiting."""
+    r = np.random.default_rng(seed)
+    pos = [np.zeros(3)]
+    for l in range(levels):
+        for o in range(1, 8):
+            upper = 0.7 if l == 0 else r.uniform(0.6, 0.68)
+            pos.append([(upper if (o >> a) & 1 else r.uniform(0.2, 0.3)) * 2.0 ** -l for a in range(3)])
+    pos = np.array(pos).astype(np.float32)
+    n = pos.shape[0]
+    zero = np.zeros(n, np.float32)
+    return (pos[:, 0].copy(), pos[:, 1].copy(), pos[:, 2].copy(), zero, zero, zero,
+            r.uniform(0.5, 1.5, n).astype(np.float32) / n)
+
+
+@pytest.mark.parametrize("kw", [{"precise": True}, {"force_list": 2, "vote_width": 128}, {"force_list": 2, "vote_width": 32},
+                                {"vote_width": 16}, {"vote_width": 16, "reference": True},
+                                {"vote_width": 32, "reference": True}],
+                         ids=["precise", "128", "32", "16", "16-reference", "32-reference"])
+def test_ordered_walk_restarts_on_the_per_level_walk(kw):
+    """Groups whose stack overflows restart (and are counted); the per-level walk gives the same sums,
+    the oracle's interactions, and the same error bounds."""
+    import nbh
+    from nbh import learned as LR
+    kw = dict(kw)
+    reference = kw.pop("reference", False)
+    if reference:
+        kw["arith"] = nbh.NBH_ARITH_REFERENCE
+    arrs = _nest(22, 7)
+    n = arrs[0].size
+    out = []
+    for cap in (256, 64):
+        g = gpu_sim(theta=0.5, eps=0.05, dt=0.0, stack_cap=cap, **kw)
+        g.load(*arrs)
+        g.step(2)
+        st = g.stats()
+        out.append((g.read(), st["interactions"], list(LR.probe(g, None))))
+        assert (st["force_restarts"] > 0) == (cap == 64)
+        assert (g.stats()["force_restarts"] > 0) == (cap == 64)          # of the probe
+        out[-1][2].extend(LR.probe(g, np.linspace(0.4, 0.6, n, dtype=np.float32)))   # an angle per body
+        assert (g.stats()["force_restarts"] > 0) == (cap == 64)
+    (state, inter, probe), (state1, inter1, probe1) = out
+    assert inter == inter1
+    for k in KEYS:
+        np.testing.assert_array_equal(state1[k], state[k], err_msg=k)
+    for a, b in zip(probe, probe1):
+        np.testing.assert_array_equal(a, b)
+    o = oracle_for(n, theta=0.5, eps=0.05, dt=0.0, vote=kw.get("vote_width", 64), fma=not reference)
+    o.load(*arrs)
+    assert o.step() == 0 and inter == o.interactions
+    if reference:
+        for k in KEYS:
+            np.testing.assert_array_equal(state1[k], o.state()[k], err_msg=k)
+
+
+@pytest.mark.parametrize("vote,n", [(64, 3000), (32, 20000), (128, 20000), (64, 300000)])
+def test_list_walk_restarts_are_counted(vote, n):
+    """Small angles overflow a 64-cell stack for some groups, shared among warps or not."""
+    arrs = plummer(n, seed=91)
+    inter = []
+    for cap in (256, 64):
+        g = gpu_sim(theta=0.15, eps=0.05, dt=0.0, vote_width=vote, stack_cap=cap)
+        g.load(*arrs)
+        g.step()
+        st = g.stats()
+        inter.append(st["interactions"])
+        if cap == 64:
+            assert st["force_restarts"] > 0
+    assert inter[0] == inter[1]
