@@ -236,3 +236,38 @@ def test_training_with_a_rate_that_falls_to_zero(n, lr):
     np.testing.assert_array_equal(p, p0)             # rates far below a parameter's last bit
     rl, _ = mlp_ref.grad(p0, X, T, 0.2)
     assert abs(loss.value - rl) <= 1e-5 * max(1.0, abs(rl))
+
+
+@pytest.mark.parametrize("n", [4097, 4160, 6145, 6200, 40000, 60001, 131073])
+def test_mlp_gradient_at_chunk_edges(n):
+    """Two to 64 chunks of samples, their edges inside a tile of 64 or on one: the samples within 1e-5
+    of a kink (a residual or a unit's input; FP32 errs by 1e-6 there) are left out, so that the
+    gradient is held to 1e-5 of its largest component.  An emulation of the FP32 sums is off by
+    half of that at most, one sample left out at a chunk's first place by 1.05e-5 (60,001) or more.
+    The last component, thousands of equal addends whose rounding errors do not average out (2e-5 at
+    6,200), equals its chain of FP32 additions."""
+    import mlp_ref
+    L, lib = _lib()
+    rng = np.random.default_rng(500 + n)
+    p = (rng.standard_normal(mlp_ref.NPARAMS) * 0.2).astype(np.float32)
+    m = n + n // 50 + 64
+    X = rng.standard_normal((m, 12)).astype(np.float32)
+    T = rng.standard_normal(m).astype(np.float32)
+    W1, b1, W2, b2, W3, b3 = mlp_ref.unpack(p)
+    z1 = X.astype(np.float64) @ W1.T + b1
+    z2 = np.maximum(z1, 0.0) @ W2.T + b2
+    r = T - (np.maximum(z2, 0.0) @ W3 + b3)
+    clear = np.minimum(np.minimum(np.abs(z1).min(1), np.abs(z2).min(1)), np.abs(r)) > 1e-5
+    X, T = np.ascontiguousarray(X[clear][:n]), np.ascontiguousarray(T[clear][:n])
+    assert T.size == n
+    g = np.empty(mlp_ref.NPARAMS, np.float32)
+    loss = C.c_float()
+    L.check(lib.nbh_mlp_grad(0, p.ctypes.data, X.ctypes.data, T.ctypes.data, n, 0.2, g.ctypes.data, C.byref(loss)))
+    rl, rg = mlp_ref.grad(p, X, T, 0.2)
+    assert abs(loss.value - rl) <= 1e-5 * max(1.0, abs(rl))
+    assert np.abs(g - rg)[:-1].max() <= 1e-5 * np.abs(rg).max()
+    dy = np.where(r[clear][:n] > 0, -np.float32(0.2), np.float32(1) - np.float32(0.2)) * (np.float32(1) / np.float32(n))
+    chunks = max(1, min(64, n // 2048))
+    size = (n + chunks - 1) // chunks
+    parts = [np.cumsum(dy[c * size:(c + 1) * size], dtype=np.float32)[-1] for c in range(chunks)]
+    assert g[-1] == np.cumsum(parts, dtype=np.float32 if chunks <= 16 else np.float64)[-1].astype(np.float32)
