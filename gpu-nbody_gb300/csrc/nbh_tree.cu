@@ -744,7 +744,10 @@ constexpr int kBucketWarps = 4;
 constexpr int kBucketStack = 232;
 constexpr int kSmallStack = 48;
 constexpr int kBucketBlocksPerSm = 7;     // all resident, at 72 registers (9 blocks: 1M sphere 324 for 310 us)
+constexpr int kPartLanes = 8;        // lanes that may hold a part: the eight octants of a large bucket, and
+                                     // the buckets that three bits of a key tell apart
 constexpr int kBucketChunk = 8;      // most buckets a warp takes per work-counter atomic
+static_assert(kBucketChunk <= kPartLanes, "a lane and a key for every bucket");
 
 // Stack position of each child cell among the nc cells pushed now: the largest deepest.
 __device__ __forceinline__ int deeper_rank(int mycnt, int lane) {
@@ -871,14 +874,14 @@ struct Part {
     float4 g;
 };
 
-// Parts that fit the lanes together: how many, from lane `first` on (at most kBucketChunk lanes hold
+// Parts that fit the lanes together: how many, from lane `first` on (at most kPartLanes lanes hold
 // one); incl: inclusive sum of their bodies.
 __device__ __forceinline__ int parts_that_fit(const Part& part, int first, int end, int& incl) {
     const int lane = threadIdx.x & 31;
     const bool mine = lane >= first && lane < end;
     incl = mine ? min(part.m, 64) : 0;
 #pragma unroll
-    for (int o = 1; o < kBucketChunk; o <<= 1) {
+    for (int o = 1; o < kPartLanes; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
     }
