@@ -566,9 +566,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     float qlb = 0.0f;
                     if (chk >= nbody) {
                         const float4 lo = gc[0], hi = gc[1];
-                        const float gx = fmaxf(fmaxf(__fsub_rn(q.x, hi.x), __fsub_rn(lo.x, q.x)), 0.0f);
-                        const float gy = fmaxf(fmaxf(__fsub_rn(q.y, hi.y), __fsub_rn(lo.y, q.y)), 0.0f);
-                        const float gz = fmaxf(fmaxf(__fsub_rn(q.z, hi.z), __fsub_rn(lo.z, q.z)), 0.0f);
+                        const float gx = gap_nan(__fsub_rn(q.x, hi.x), __fsub_rn(lo.x, q.x));
+                        const float gy = gap_nan(__fsub_rn(q.y, hi.y), __fsub_rn(lo.y, q.y));
+                        const float gz = gap_nan(__fsub_rn(q.z, hi.z), __fsub_rn(lo.z, q.z));
                         const float dlb = dist2<false>(gx, gy, gz, eps2);
                         qlb = PB ? __fmaf_rn(lo.w, sl, eps2) : __fadd_rn(__fmul_rn(lo.w, sl), eps2);
                         if (dlb >= qlb) {

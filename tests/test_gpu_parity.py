@@ -963,9 +963,10 @@ def test_sorted_paths_build_the_staged_tree(n):
 
 
 @pytest.mark.parametrize("kw", [{"vote_width": 16}, {"vote_width": 16, "reference": True}, {"vote_width": 32, "reference": True},
-                                {"vote_width": 32, "force_list": 2}, {"force_list": 2}, {"vote_width": 128, "force_list": 2}],
-                         ids=["16", "16-reference", "32-reference", "32", "64", "128"])
-def test_ordered_walk_opens_cells_of_massless_bodies(kw):
+                                {"vote_width": 32, "force_list": 2}, {"force_list": 2}, {"vote_width": 128, "force_list": 2},
+                                {"vote_width": 32}, {}, {"vote_width": 128}],
+                         ids=["16", "16-reference", "32-reference", "32", "64", "128", "list-32", "list-64", "list-128"])
+def test_walks_open_cells_of_massless_bodies(kw):
     """The centre of a cell of massless bodies is not a number (0 / 0): no body's distance test passes
     on it, so it is opened, however small it is beside the softening, and its bodies add nothing."""
     import nbh
