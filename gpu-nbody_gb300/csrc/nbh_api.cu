@@ -100,7 +100,10 @@ namespace {
 // 84 us, 4 x 30,000 141 -> 127, 256 x 16,384 724 -> 660.  Beyond, the one block's chain of lock
 // rounds takes longer than the pass it saves (40,000 bodies 119 -> 128 us, 8 x 60,000 204 -> 216),
 // unless the pass is that of many universes: from 1M bodies in all the limit is twice as high
-// (256 of 1K-64K bodies 668 -> 617 us, 32 x 60,000 414 -> 384).
+// (256 of 1K-64K bodies 668 -> 617 us, 32 x 60,000 414 -> 384).  All tree stages around the limits:
+// 33,000 + 8 x 16,000 218 -> 205, 40,000 + 20 x 5,000 203 -> 205, 32 x 65,536 549 -> 523, 32 x 80,000
+// 628 -> 607, 16 x 131,072 556 -> 588, 131,072 + 100 x 20,000 530 -> 590.  The largest universe decides
+// for all of a batch: its block is the one that the others would wait for.
 constexpr int kDirectSamples = 2048, kDirectManyChunks = 4096;
 
 thread_local std::string g_create_error;

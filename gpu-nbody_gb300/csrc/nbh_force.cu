@@ -38,7 +38,8 @@ struct SplitTeam {
 // SM (the walk's residency).  Force stage of Plummer spheres in groups of 64, us, shared / one
 // warp each: 1,000 bodies 51 / 84, 16,384 145 / 449, 65,536 262 / 674, 100,003 367 / 702,
 // 200,000 (two warps) 549 / 743; at 300,000 two warps lose, 881 / 786.  With kSplitFront 4 and
-// 12 in place of 8: 172 and 149 at 16,384, 262 and 306 at 65,536.
+// 12 in place of 8: 172 and 149 at 16,384, 262 and 306 at 65,536.  The number of warps decides the
+// order of a group's sum, so a universe's last bits depend on the batch it is in.
 static int force_split(int groups, int sms) {
     int s = 1;
     while (s < kSplitMax && groups * s < 24 * sms) s *= 2;
@@ -294,7 +295,7 @@ __device__ __forceinline__ void eval_ordered(const float4* lst, const float* lw,
 // cells per warp wait; then warp w keeps every S-th of them and walks on alone, and the sums are
 // added in the order of the warps at the end.  The records accepted on the way are dealt out
 // the same way.  S depends on the number of groups only (force_split), so that the launch
-// geometry does not change the order of the sums.
+// geometry does not change the order of the sums; the number of universes beside one does.
 template <int W, bool REF, bool PB, bool FEAT, bool LIST = false, bool SPLIT = false>
 __device__ __forceinline__ void force_walk(const StepParams& p) {
     static_assert(!LIST || (W >= 32 && !REF), "the list walk takes whole-warp groups and FMA arithmetic");
@@ -661,8 +662,9 @@ __device__ __forceinline__ void force_walk(const StepParams& p) {
                     ctop += on;
                     __syncwarp();          // list and stack written before they are read
                     if (lcnt >= 32) {
-                        // 32 records at a time (unrolled completely: 2.6 % of the force at two bodies
-                        // per lane against unrolled by 8); at most 31 wait behind them
+                        // 32 records at a time (two or more bodies per lane: unrolled completely, a 1M
+                        // step 2433 us against 2526 unrolled by 2, 256 universes 5796 against 5980);
+                        // at most 31 wait behind them
 #pragma unroll(BPL >= 2 ? 8 : 2)
                         for (int i = 0; i < 32; i += 4) eval4<BPL, FEAT>(lst + lbase, i, lb, eps22, ls);
                         accepted += 32;

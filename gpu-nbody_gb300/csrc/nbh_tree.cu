@@ -1503,13 +1503,13 @@ __global__ void __launch_bounds__(256) sort_kernel(StepParams p) {
 // The same arithmetic in the same order as the stages it replaces, so the same tree.
 //
 // Per cell of the shared tree: 8 slots, level, centre of mass, body count, offset in its
-// parent's range, parent, and the list of the cells by level.  A universe whose tree does not fit (close pairs make chains of
-// single-child cells) or goes too deep is built by its block in global memory, through the lock
-// insertion.
-// Measured, us, one launch / the stages: one sphere of 300 bodies 38 / 124, 1,000 52 / 132,
-// 3,000 97 / 140, 5,000 134 / 158, 7,168 175 / 156; 8 of 7,168 184 / 197, 200 of 1,000
-// 134 / 227, 200 of 7,168 404 / 503: up to 7,168 bodies (what shared memory holds) from 8
-// universes on, up to 5,120 for fewer.
+// parent's range, parent, and the list of the cells by level.  A universe whose tree does not fit
+// (close pairs make chains of single-child cells) or goes too deep is built by its block in global
+// memory, through the lock insertion.
+// Measured, us, one launch / the stages: one sphere of 100 bodies 24 / 71, 300 29 / 82, 1,000 40 / 94,
+// 3,000 82 / 97, 5,120 112 / 113, 6,000 124 / 116, 7,168 142 / 113; 8 of 7,168 147 / 139, 200 of 1,000
+// 73 / 171, 200 of 7,168 283 / 360, 20,000 of 16 188 / 858: up to 5,120 bodies, and up to 7,168
+// (what shared memory holds) from 8 universes on.
 constexpr int kSmallBodies = 7168, kSmallBodiesFew = 5120;
 constexpr size_t kSmallCellBytes = 8 * sizeof(unsigned short) + sizeof(float4) + 4 * sizeof(unsigned short) + 1;
 int small_tree_max_bodies(int universes) { return universes >= 8 ? kSmallBodies : kSmallBodiesFew; }
@@ -2013,7 +2013,7 @@ void launch_build(const StepParams& p, bool ref, int phases, bool buckets, int s
     buckets = buckets && phases != 1;
     if (buckets && phases == 3 && direct > 0) {
         // the whole 1/16 sample in shared memory, then every other body as bucket subtrees: five
-        // launches fewer than below for small universes
+        // launches in place of the nine below
         top_build_kernel<<<split * p.nuniv, kTopThreads, top_build_smem(direct), s>>>(p, BuildPhase{16, 0}, true, direct,
                                                                                     split);
         launch_bucket_pass(p, kBucketBodies, true, true, ref, sms, s);

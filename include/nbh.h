@@ -125,7 +125,12 @@ typedef struct nbh_config {
                               shared memory; 2 keeps the reference's order of accumulation
                               (depth-first, children in order).  The same interactions either
                               way; the sums may differ in the last bits.  0: the default, 1
-                              except in precise mode, which keeps the reference's order */
+                              except in precise mode, which keeps the reference's order.
+                              With 1 and fewer than 24 groups per SM, 2, 4 or 8 warps share
+                              each group: the number of groups of all universes loaded, and
+                              of SMs, then decides the order of the sums, so a universe's
+                              last bits differ between a run alone and one in a batch (with
+                              2 they do not) */
     int32_t reserved[2];
 } nbh_config;
 
@@ -144,8 +149,11 @@ typedef struct nbh_stats {
     int32_t pool_nodes;        /* NUMBER_OF_NODES of the shared pool */
     int32_t status;            /* device status word of the last step (NBH_OK or NBH_ERR_*) */
     int32_t lock_waits;        /* build of the last step: descents that found their slot locked */
-    int32_t cas_misses;        /* build of the last step: lock attempts that lost the race */
-    /* per-stage device milliseconds of the last step (stage_timing = 1 only) */
+    int32_t cas_misses;        /* build of the last step: lock attempts that lost the race (both of
+                                  locks in global memory, not in shared memory) */
+    /* per-stage device milliseconds of the last step (stage_timing = 1 only); the one launch of
+     * small universes (nbh_config.top_phase) counts as ms_build, and ms_bbox, ms_summarize and
+     * ms_sort read about zero then */
     float   ms_bbox, ms_build, ms_summarize, ms_sort, ms_force, ms_integrate, ms_step;
     float   ms_theta;          /* learned opening angle: features + MLP inference of the last
                                   step (0 without a model; stage_timing = 1 only) */

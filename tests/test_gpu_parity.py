@@ -1139,3 +1139,31 @@ def test_list_walk_restarts_are_counted(vote, n):
         if cap == 64:
             assert st["force_restarts"] > 0
     assert inter[0] == inter[1]
+
+
+def test_ordered_walk_does_not_depend_on_the_batch():
+    """A universe in the ordered walk: the same bits alone and beside others; in the list walk, whose
+    sums follow the number of groups loaded, the same interactions and sums within rounding."""
+    parts = [plummer(c, seed=500 + c) for c in (3000, 6000, 20000, 400)]
+    counts = [p[0].size for p in parts]
+    cat = [np.concatenate([p[k] for p in parts]) for k in range(7)]
+    for force_list in (2, 1):
+        batch = gpu_sim(theta=0.5, eps=0.05, dt=0.0, force_list=force_list)
+        batch.load_batch(counts, *cat)
+        batch.step()
+        together, total, off = batch.read(), 0, 0
+        for part, c in zip(parts, counts):
+            g = gpu_sim(theta=0.5, eps=0.05, dt=0.0, force_list=force_list)
+            g.load(*part)
+            g.step()
+            alone = g.read()
+            total += g.stats()["interactions"]
+            sub = {k: together[k][off:off + c] for k in KEYS}
+            if force_list == 2:
+                for k in KEYS:
+                    np.testing.assert_array_equal(sub[k], alone[k])
+            else:
+                rel, _ = acc_rel(sub, alone)
+                assert rel.max() <= FMA_ACC_REL_MAX and np.median(rel) <= FMA_ACC_REL_MEDIAN
+            off += c
+        assert batch.stats()["interactions"] == total
