@@ -1919,33 +1919,38 @@ __global__ void __launch_bounds__(kTopThreads) small_tree_kernel(StepParams p, i
                 slots[c * 8 + at] = v16;
                 cell_child(p, gc)[at] = g;
                 if (some) p.kids4[((size_t)k << 3) + at] = q;
-                float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
-                double dm = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const float x = __shfl_sync(gmask, q.x, t, 8), y = __shfl_sync(gmask, q.y, t, 8);
-                    const float z = __shfl_sync(gmask, q.z, t, 8), w = __shfl_sync(gmask, q.w, t, 8);
-                    if (!((have >> t) & 1u)) continue;
-                    if (PRECISE && c == 0) {
+                float4 centre;
+                if (PRECISE && level == 0) {
+                    // the root, in FP64 (a path of its own: as a branch of the FP32 sums it took
+                    // its time for every cell, tree of 5,120 bodies 347 us)
+                    double dm = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
+#pragma unroll 1
+                    for (int t = 0; t < 8; ++t) {
+                        const float x = __shfl_sync(gmask, q.x, t, 8), y = __shfl_sync(gmask, q.y, t, 8);
+                        const float z = __shfl_sync(gmask, q.z, t, 8), w = __shfl_sync(gmask, q.w, t, 8);
+                        if (!((have >> t) & 1u)) continue;
                         dm += (double)w;
                         dx += (double)x * (double)w;
                         dy += (double)y * (double)w;
                         dz += (double)z * (double)w;
-                    } else {
+                    }
+                    centre = make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
+                } else {
+                    float cm = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) {
+                        const float x = __shfl_sync(gmask, q.x, t, 8), y = __shfl_sync(gmask, q.y, t, 8);
+                        const float z = __shfl_sync(gmask, q.z, t, 8), w = __shfl_sync(gmask, q.w, t, 8);
+                        if (!((have >> t) & 1u)) continue;
                         cm = __fadd_rn(cm, w);
                         sx = madd<REF>(x, w, sx);
                         sy = madd<REF>(y, w, sy);
                         sz = madd<REF>(z, w, sz);
                     }
+                    const float inv = __fdiv_rn(1.0f, cm);
+                    centre = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
                 }
                 if (j == 0) {
-                    float4 centre;
-                    if (PRECISE && c == 0) {
-                        centre = make_float4((float)(dx / dm), (float)(dy / dm), (float)(dz / dm), (float)dm);
-                    } else {
-                        const float inv = __fdiv_rn(1.0f, cm);
-                        centre = make_float4(__fmul_rn(sx, inv), __fmul_rn(sy, inv), __fmul_rn(sz, inv), cm);
-                    }
                     com[c] = centre;
                     count[c] = (unsigned short)total;
                     p.node4[gc] = centre;

@@ -1048,16 +1048,17 @@ def test_one_launch_tree_of_many_that_do_not_fit(mode):
     _assert_same_steps(_steps(kw, load, 6), _steps({**kw, "build_phases": 1}, load, 6))
 
 
-@pytest.mark.parametrize("universes,n,pairs", [(20000, 16, 0), (1, 5000, 1500), (100, 1000, 300)])
-def test_one_launch_tree_costs_no_more_than_the_staged_one(universes, n, pairs):
+@pytest.mark.parametrize("universes,n,pairs,precise", [(20000, 16, 0, False), (1, 5000, 1500, False), (100, 1000, 300, False),
+                                                       (1, 5000, 0, True)])
+def test_one_launch_tree_costs_no_more_than_the_staged_one(universes, n, pairs, precise):
     """Many tiny universes, and ones that do not fit shared memory: work that one block did for each of
-    them in turn took 5 to 200 times the stages.  (A step takes them side by side; 1.5 leaves room
-    for the clock and for launches.)"""
+    them in turn took 5 to 200 times the stages; in precise mode FP64 sums of every cell three times.
+    (A step takes them side by side; 1.5 leaves room for the clock and for launches.)"""
     parts = [_close_pairs(n, pairs, 400 + i) for i in range(min(universes, 8))]
     cat = [np.concatenate([parts[u % len(parts)][k] for u in range(universes)]) for k in range(7)]
     ms = []
     for kw in ({}, {"build_phases": 3}):
-        g = gpu_sim(theta=0.9, eps=0.05, dt=0.0, pool_factor=16.0, stage_timing=True, **kw)
+        g = gpu_sim(theta=0.9, eps=0.05, dt=0.0, pool_factor=16.0, stage_timing=True, precise=precise, **kw)
         g.load_batch([n] * universes, *cat)
         t = []
         for _ in range(9):
