@@ -28,23 +28,22 @@ constexpr size_t force_list_smem_bytes(int threads, int cap) { return (size_t)(t
 // room for the breadth-first queue, and what the warps tell each other.
 constexpr int kSplitFront = 8;
 constexpr int kSplitQueue = 256;
-constexpr int kSplitMax = 8;
-constexpr int kSplitKeep = kSplitQueue / (2 * 32);   // entries per lane of a warp's share, at two warps
+constexpr int kSplitMin = 4, kSplitMax = 8;
+constexpr int kSplitKeep = kSplitQueue / (kSplitMin * 32);   // entries per lane of a warp's share, at most
 struct SplitTeam {
     int item, status;
     int accepted[kSplitMax], opened[kSplitMax];
 };
-// Warps per group for `groups` groups: doubled, up to 8, while there are fewer than 24 warps per
-// SM (the walk's residency).  Force stage of Plummer spheres in groups of 64, us, shared / one
-// warp each: 1,000 bodies 51 / 84, 16,384 145 / 449, 65,536 262 / 674, 100,003 367 / 702,
-// 200,000 (two warps) 549 / 743; at 300,000 two warps lose, 881 / 786.  With kSplitFront 4 and
-// 12 in place of 8: 172 and 149 at 16,384, 262 and 306 at 65,536.  The number of warps decides the
-// order of a group's sum, so a universe's last bits depend on the batch it is in.
-static int force_split(int groups, int sms) {
-    int s = 1;
-    while (s < kSplitMax && groups * s < 24 * sms) s *= 2;
-    return s;
-}
+// Warps per group for `groups` groups.  Force stage of Plummer spheres in groups of 64, us, by the number
+// of groups: 469 (30,000 bodies) 182 / 211 / 240 with 8 / 4 / 2 warps; 907 281 / 264 / 299; 1,250 383 /
+// 297 / 311; 1,813 545 / 403 / 430; with 2 / 1 warps 1,875 465 / 385, 2,500 463 / 479, 3,125 571 / 563,
+// 3,438 767 / 608: from 12 groups per SM on the warps' common first rounds cost more than idle schedulers
+// do, and two warps are the best choice nowhere (in groups of 32 likewise: 1,032 groups 186 / 162 /
+// 160, 1,782 291 / 217 / 283, 2 / 1 warps 1,875 315 / 225; of 128: 1,797 1208 / 848 / 913, 1,875 950 / 819,
+// 3,594 1669 / 1171).  With kSplitFront 4 and 12 in place of 8: 172 and 149 us at 16,384 bodies (145),
+// 262 and 306 at 65,536 (262).  The number of warps decides the order of a group's sum, so a
+// universe's last bits depend on the batch it is in.
+static int force_split(int groups, int sms) { return groups >= 12 * sms ? 1 : (groups >= 6 * sms ? 4 : 8); }
 static_assert(kStackCapMin * sizeof(int2) >= 2 * kMaxDepth * sizeof(int), "the per-level walk fits the cell stack");
 
 // The ordered walk: per group, a stack of pending nodes (24 bytes for each of the `cap` entries
@@ -288,7 +287,7 @@ __device__ __forceinline__ void eval_ordered(const float4* lst, const float* lw,
 // entries: 256 by default; the 64-body groups of the benchmarked spheres need at most 99 in the
 // list walk).
 //
-// SPLIT (with LIST): a block of S = 2, 4 or 8 warps shares one group.  A group's walk is one
+// SPLIT (with LIST): a block of S = 4 or 8 warps shares one group.  A group's walk is one
 // chain of rounds, and a universe with fewer groups than the GPU has room for warps leaves
 // most of it idle (16,384 bodies in groups of 32: 512 warps on 608 schedulers).  Every warp
 // expands the tree from the root breadth first, all of them the same way, until kSplitFront

@@ -126,7 +126,7 @@ typedef struct nbh_config {
                               (depth-first, children in order).  The same interactions either
                               way; the sums may differ in the last bits.  0: the default, 1
                               except in precise mode, which keeps the reference's order.
-                              With 1 and fewer than 24 groups per SM, 2, 4 or 8 warps share
+                              With 1 and fewer than 12 groups per SM, 4 or 8 warps share
                               each group: the number of groups of all universes loaded, and
                               of SMs, then decides the order of the sums, so a universe's
                               last bits differ between a run alone and one in a batch (with

@@ -1186,3 +1186,10 @@ def test_groups_are_spread_over_the_sms():
     there are groups, left SMs without any and took 0.98 of the time of 4,688 groups, with 1.27 times
     the interactions; spread evenly 0.82."""
     assert _force_ms(240000) <= 0.92 * _force_ms(300000)
+
+
+@pytest.mark.parametrize("vote,fewer,more", [(64, 230000, 240000), (128, 460000, 490000)])
+def test_sharing_groups_ends_where_it_costs_more(vote, fewer, more):
+    """24 groups per SM from either side: groups shared among two warps below took 1.26 and 1.4 times as
+    long as whole ones above."""
+    assert _force_ms(fewer, vote_width=vote) <= 1.1 * _force_ms(more, vote_width=vote)
