@@ -47,10 +47,15 @@ static int force_split(int groups, int sms) { return groups >= 12 * sms ? 1 : (g
 static_assert(kStackCapMin * sizeof(int2) >= 2 * kMaxDepth * sizeof(int), "the per-level walk fits the cell stack");
 
 // The ordered walk: per group, a stack of pending nodes (24 bytes for each of the `cap` entries
-// asked for, at 16 bytes each), with their widths^2 factors where error bounds are recorded,
+// asked for, at 16 bytes each; 160 entries at least: with 96, 73 % of the groups of a 3M disc
+// overflowed theirs, and walking them twice took 27115 us where the per-level walk alone takes
+// 17143; with 160 12718), with their widths^2 factors where error bounds are recorded,
 // the list of accepted records (each twice over where a lane has two or more bodies) with their
 // widths^2, the undecided cells of a round, and the group's box and representatives.
-__host__ __device__ constexpr int ordered_entries(int cap) { return cap + cap / 2; }
+constexpr int kOrderedMin = 160;
+__host__ __device__ constexpr int ordered_entries(int cap) {
+    return cap + cap / 2 > kOrderedMin ? cap + cap / 2 : kOrderedMin;
+}
 template <int W>
 constexpr size_t force_smem_bytes(int threads, int cap, bool feat) {
     return (size_t)(threads / 32) * ((size_t)ordered_entries(cap) * (sizeof(float4) + (feat ? sizeof(float) : 0)) +

@@ -89,9 +89,10 @@ typedef struct nbh_config {
     int32_t stack_cap;     /* size of each vote group's shared-memory stack, 64..256, a
                               multiple of 8 (0: 256): in the list walk (force_list) the cells
                               whose children are still to be tested, in the ordered walk half
-                              as many nodes again that wait for their turn.  A group whose
-                              stack would overflow restarts on a walk with one entry per
-                              level: the same result, slower (nbh_stats.force_restarts) */
+                              as many nodes again (160 at least) that wait for their turn.
+                              A group whose stack would overflow restarts on a walk with one
+                              entry per level: the same interactions, slower
+                              (nbh_stats.force_restarts) */
     int32_t build_phases;  /* octree insertion launches: 1 (one pass), 3 or 5 (0: 3) */
     int32_t build_buckets; /* 1 (or 0, the default): with 5 phases the lock phases insert a
                               1/16 sample of the bodies and every other body joins the
