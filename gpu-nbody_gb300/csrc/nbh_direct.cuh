@@ -10,7 +10,7 @@ struct Src64 {
     double x, y, z, m;
 };
 
-// Slices of the sources for `targets` blocks of target bodies: 32 blocks per SM in all (about 5
+// Slices of the sources for `targets` blocks of target bodies: 32 blocks per SM in all (four
 // are resident), so that the last wave is short.
 inline int direct_slices(int targets, int sms) {
     const int want = (32 * sms + targets - 1) / targets;
